@@ -144,6 +144,18 @@ int tct_farfield_tris_matvec(int kernel, int prec, void* out, const void* in,
                              const double* params, int accumulate,
                              void* workspace, size_t workspace_bytes, void* stream);
 
+/* The same product for a triangle set on itself (obs_tris == src_tris),
+ * elasticRH3 with a 3-, 4- or 7-point rule: each pair's geometry is formed
+ * once for both directions (the pair sums are symmetric).  Deterministic, as
+ * above.  The workspace query returns 0 for a kernel, precision, rule or size
+ * that only tct_farfield_tris_matvec serves (few triangles, or partial sums
+ * above 1 GiB). */
+size_t tct_farfield_self_workspace_bytes(int kernel, int prec, int64_t n, int n_q);
+int tct_farfield_self_matvec(int kernel, int prec, void* out, const void* in, const void* pts,
+                             const int32_t* tris, int64_t n, int n_q, const double* quad_pts,
+                             const double* quad_wts, const double* params, int accumulate,
+                             void* workspace, size_t workspace_bytes, void* stream);
+
 /* ------------------------------------------------------------------------ */
 /* Point-to-point farfield.                                                  */
 /* Replaces farfield_pts{K} (tectosaur/farfield_direct.cl:15-113) behind

@@ -50,6 +50,9 @@ _SIGS = {
     "tct_farfield_workspace_bytes": ([c_i, c_i, c_i64, c_i64, c_i], c_sz),
     "tct_farfield_tris_matvec": ([c_i, c_i, c_p, c_p, c_p, c_p, c_i64, c_p, c_i64, c_i, c_dp,
                                   c_dp, c_dp, c_i, c_p, c_sz, c_p], c_i),
+    "tct_farfield_self_workspace_bytes": ([c_i, c_i, c_i64, c_i], c_sz),
+    "tct_farfield_self_matvec": ([c_i, c_i, c_p, c_p, c_p, c_p, c_i64, c_i, c_dp, c_dp, c_dp, c_i,
+                                  c_p, c_sz, c_p], c_i),
     "tct_farfield_pts": ([c_i, c_i, c_p, c_p, c_p, c_i64, c_p, c_p, c_i64, c_p, c_dp, c_p], c_i),
     "tct_farfield_tris_dense": ([c_i, c_i, c_p, c_i, c_p, c_p, c_p, c_p, c_i64, c_p, c_i64, c_dp,
                                  c_p], c_i),

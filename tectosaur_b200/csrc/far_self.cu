@@ -1,0 +1,353 @@
+// elasticRH3 farfield of a triangle set on itself: the pair geometry is
+// formed once for both directions.
+//
+// The pair sums are symmetric (rh_sym.cuh).  The general kernel (far_main_rh2,
+// farfield.cu) forms them twice per unordered pair.  Here a CTA takes a group
+// of observation triangles and a chunk of sources after it, adds both
+// directions per pair: W of the group from the sources, V of the sources from
+// the group.  Chunks inside the group itself take the one-sided form
+// over the full square.
+//
+// What bounds it: the FMA pipe.  Per point pair 17 packed operations, per
+// triangle pair 36 for each direction, and about 22 scalar additions per
+// source and warp for the sum of V over the warp's observation triangles:
+// with the 3-point rule 237 pipe slots per unordered pair of (two packed
+// observation triangles, source) against 2 x 189.
+//
+// V is summed over the lanes by a transposing exchange of two sources' nine
+// sums (21 shuffles), written by the owning lanes to the warp's slots in
+// shared memory, added over warps after each tile and over the group's
+// strips in shared memory; group sums of V and chunk sums of W go to global
+// partials and a last kernel adds a triangle's partials in a fixed order in
+// double: no atomics, the same bits every run.
+#include <algorithm>
+
+#include "rh_sym.cuh"
+
+namespace tct {
+namespace {
+
+constexpr int SELF_TS = 64;  // sources per staged tile
+
+// How a self farfield of n triangles is cut: observation groups of `strips`
+// strips (128 H triangles each), source chunks of `chunk` (a divisor of the
+// group size), one CTA per (group, chunk at or after the group's first).
+struct SelfCut {
+    int strips, chunk;
+    int64_t groups, chunks, per_group;  // per_group: chunks of one group
+};
+
+__host__ __device__ inline int64_t self_tasks_before(int64_t g, int64_t chunks, int64_t per_group) {
+    return g * chunks - per_group * (g * (g - 1) / 2);
+}
+
+template <class V, int NQ>
+constexpr size_t self_smem(int chunk) {
+    return 8 * (size_t)RecSelf<NQ>::LEN * SELF_TS + sizeof(typename V::real) * 9 * (4 * SELF_TS + chunk);
+}
+
+// Resident CTAs an SM the registers are capped for.  FP32: 3 (168 registers)
+// ran 2.5 % faster than 2 with the 3-point rule at 20,001 and 59,858
+// triangles and 1 % with the 4-point rule, 4 (128 registers) 3 to 7 % slower;
+// with the 7-point rule 3 spills and runs 4 % slower than 2.  FP64: 3 ran 12 %
+// faster than 2 at 12,290 triangles, 4 4 % slower than 3.
+template <class V, int NQ>
+constexpr int self_ctas() { return V::H == 2 && NQ == 7 ? 2 : 3; }
+
+template <class V, int NQ, bool UNIFORM>
+__global__ void __launch_bounds__(128, self_ctas<V, NQ>())
+far_self_main(PairWeights<V, NQ> pw, const typename V::vec* __restrict__ rec, int64_t n,
+              int strips, int chunk, int64_t chunks, int64_t groups,
+              typename V::real* __restrict__ Wp, typename V::real* __restrict__ Vp) {
+    using R = typename V::real;
+    using vec = typename V::vec;
+    using L = RecSelf<NQ>;
+    constexpr int STRIP = 128 * V::H;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    vec* sm = reinterpret_cast<vec*>(smem_raw);                     // SELF_TS records
+    R* Vw = reinterpret_cast<R*>(sm + L::LEN * SELF_TS);            // 4 warps x SELF_TS x 9
+    R* Va = Vw + 4 * SELF_TS * 9;                                   // chunk x 9
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+
+    // task -> (group, chunk)
+    const int64_t per_group = (int64_t)strips * STRIP / chunk;
+    int64_t g = 0;
+    {
+        // the largest g with self_tasks_before(g) <= task, by bisection
+        int64_t lo = 0, hi = groups - 1;
+        while (lo < hi) {
+            const int64_t mid = (lo + hi + 1) / 2;
+            if (self_tasks_before(mid, chunks, per_group) <= (int64_t)blockIdx.x) lo = mid;
+            else hi = mid - 1;
+        }
+        g = lo;
+    }
+    const int64_t ck = g * per_group + ((int64_t)blockIdx.x - self_tasks_before(g, chunks, per_group));
+    const bool diag = ck < (g + 1) * per_group;
+    const int64_t c0 = ck * chunk, c1 = min(n, c0 + chunk);
+
+    for (int st = 0; st < strips; st++) {
+        const int64_t base = (g * strips + st) * STRIP;
+        if (base >= n) break;
+        const int64_t ia = base + tid, ib = ia + 128;
+        const bool va = ia < n, vb = V::H == 2 && ib < n;
+        const vec* ra = rec + (va ? ia : 0) * L::LEN;
+        const vec* rb = rec + (vb ? ib : 0) * L::LEN;
+        vec negx[NQ][3], S[18], W[9], tot[9];
+        {
+            // lanes past the end: points at the origin, zero input (no V)
+            const R* pa = reinterpret_cast<const R*>(ra);
+            const R* pb = reinterpret_cast<const R*>(rb);
+#pragma unroll
+            for (int q = 0; q < NQ; q++)
+#pragma unroll
+                for (int d = 0; d < 3; d++) {
+                    const int k = V::H * (L::Y + 3 * q + d);
+                    negx[q][d] = V::make(va ? -pa[k] : R(0), vb ? -pb[k] : R(0));
+                }
+#pragma unroll
+            for (int k = 0; k < 18; k++)
+                S[k] = V::make(va ? pa[V::H * (L::P + k)] : R(0), vb ? pb[V::H * (L::P + k)] : R(0));
+#pragma unroll
+            for (int k = 0; k < 9; k++) tot[k] = V::make(0, 0);
+        }
+        for (int64_t t0 = c0; t0 < c1; t0 += SELF_TS) {
+            const int nt = (int)min((int64_t)SELF_TS, c1 - t0);
+            __syncthreads();
+            {
+                const ulonglong2* srcv = reinterpret_cast<const ulonglong2*>(rec + t0 * L::LEN);
+                ulonglong2* dstv = reinterpret_cast<ulonglong2*>(sm);
+                for (int k = tid; k < nt * L::LEN / 2; k += 128) dstv[k] = __ldg(srcv + k);
+                // an odd last source is paired with one of zero points and input
+                if (nt & 1)
+                    for (int k = tid; k < L::LEN; k += 128) sm[nt * L::LEN + k] = V::make(0, 0);
+            }
+            __syncthreads();
+#pragma unroll
+            for (int k = 0; k < 9; k++) W[k] = V::make(0, 0);
+            if (diag) {
+#pragma unroll 1
+                for (int j = 0; j < nt; j++) {
+                    vec T[6], pm[18];
+                    self_tensor<V, NQ, UNIFORM>(sm + j * L::LEN, negx, pw, T);
+                    self_load_pm<V, NQ>(sm + j * L::LEN, pm);
+                    self_apply<V>(T, V::add(V::add(T[0], T[3]), T[5]), pm, W);
+                }
+            } else {
+#pragma unroll 1
+                for (int j = 0; j < nt; j += 2) {
+                    R s[2][9];
+#pragma unroll
+                    for (int u = 0; u < 2; u++) {
+                        vec T[6], pm[18], v[9];
+                        const vec* r = sm + (j + u) * L::LEN;
+                        self_tensor<V, NQ, UNIFORM>(r, negx, pw, T);
+                        const vec S0 = V::add(V::add(T[0], T[3]), T[5]);
+                        self_load_pm<V, NQ>(r, pm);
+                        self_apply<V>(T, S0, pm, W);
+#pragma unroll
+                        for (int k = 0; k < 9; k++) v[k] = V::make(0, 0);
+                        self_apply<V>(T, S0, S, v);
+#pragma unroll
+                        for (int k = 0; k < 9; k++) s[u][k] = V::hsum(v[k]);
+                    }
+                    R lo, hi;
+                    warp_sum2x9(s[0], s[1], lane, lo, hi);
+                    R* slot = Vw + (warp * SELF_TS + j + (lane >> 4)) * 9;
+                    if ((lane & 1) == 0) slot[(lane >> 1) & 7] = lo;
+                    if ((lane & 15) == 0) slot[8] = hi;
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < 9; k++) tot[k] = V::add(tot[k], W[k]);
+            if (!diag) {
+                __syncthreads();
+                for (int e = tid; e < nt * 9; e += 128) {
+                    const R v = (Vw[e] + Vw[SELF_TS * 9 + e]) +
+                                (Vw[2 * SELF_TS * 9 + e] + Vw[3 * SELF_TS * 9 + e]);
+                    const int a = (int)(t0 - c0) * 9 + e;
+                    Va[a] = st == 0 ? v : Va[a] + v;
+                }
+            }
+        }
+        R* wo = Wp + ck * n * 9;
+#pragma unroll
+        for (int k = 0; k < 9; k++) {
+            R o[V::H];
+            V::split(tot[k], o);
+            if (va) wo[ia * 9 + k] = o[0];
+            if (vb) wo[ib * 9 + k] = o[V::H - 1];
+        }
+    }
+    if (!diag) {
+        __syncthreads();
+        R* vo = Vp + (g * n + c0) * 9;
+        for (int e = tid; e < (int)(c1 - c0) * 9; e += 128) vo[e] = Va[e];
+    }
+}
+
+// A triangle's sums: W partials of the chunks from its group's first on and V
+// partials of the groups before its own, added in that order in double, then
+// out[b][d] (+)= J sum_j sc[b][j] W[d][j].  32 triangles a block, a thread
+// per sum; bound by the partials' reads (groups + chunks rows of 36 or 72
+// bytes a triangle over two).
+template <typename R>
+__global__ void __launch_bounds__(288)
+far_self_reduce(const R* __restrict__ pts, const int32_t* __restrict__ tris, int64_t n,
+                int64_t group_size, int64_t per_group, int64_t chunks,
+                const R* __restrict__ Wp, const R* __restrict__ Vp, R* __restrict__ out,
+                int accumulate) {
+    __shared__ R w[32 * 9];
+    __shared__ R geo[32][10];
+    const int64_t t0 = (int64_t)blockIdx.x * 32;
+    const int tid = threadIdx.x;
+    const int64_t i = t0 + tid / 9;
+    if (tid < 32 && t0 + tid < n) {
+        TriGeom<R> o;
+        load_tri(o, pts, tris, t0 + tid, 0, false, true);
+#pragma unroll
+        for (int b = 0; b < 3; b++)
+#pragma unroll
+            for (int j = 0; j < 3; j++) geo[tid][3 * b + j] = o.sc[b][j];
+        geo[tid][9] = o.J;
+    }
+    if (i < n) {
+        const int64_t e = t0 * 9 + tid, g = i / group_size;
+        double s = 0;
+#pragma unroll 8
+        for (int64_t c = g * per_group; c < chunks; c++) s += (double)Wp[c * n * 9 + e];
+#pragma unroll 8
+        for (int64_t k = 0; k < g; k++) s += (double)Vp[k * n * 9 + e];
+        w[tid] = (R)s;
+    }
+    __syncthreads();
+    if (i >= n) return;
+    const int l = tid / 9, b = (tid % 9) / 3, d = tid % 3;
+    const R v = geo[l][9] * (geo[l][3 * b] * w[l * 9 + 3 * d] + geo[l][3 * b + 1] * w[l * 9 + 3 * d + 1] +
+                             geo[l][3 * b + 2] * w[l * 9 + 3 * d + 2]);
+    R* op = out + t0 * 9 + tid;
+    *op = accumulate ? *op + v : v;
+}
+
+inline size_t al256(size_t b) { return (b + 255) / 256 * 256; }
+
+// The fewest triangles served: below, the general kernel's chunks keep more
+// of the chip busy (FP32, 3-point rule: 722 triangles 0.029 ms general, 0.045
+// here, 1,500 0.047 against 0.045; FP64: 300 triangles 0.044 against 0.041).
+constexpr int64_t SELF_MIN_F32 = 1500, SELF_MIN_F64 = 256;
+
+// Cut of n triangles: the largest groups and chunks (fewest partial sums) that
+// still give four CTAs for each of two per SM, so that the last wave is a
+// small part; the smallest cut where none does.
+SelfCut self_cut(int prec, int64_t n) {
+    const int64_t strip = prec == TCT_F32 ? 256 : 128;
+    static const int kStrips[] = {4, 2, 1, 1, 1};
+    static const int kDiv[] = {1, 1, 1, 2, 4};  // chunk = group / div
+    SelfCut c{0, 0, 0, 0, 0};
+    for (int k = 0; k < 5; k++) {
+        c.strips = kStrips[k];
+        const int64_t group = c.strips * strip;
+        c.per_group = kDiv[k];
+        c.chunk = (int)(group / kDiv[k]);
+        c.groups = (n + group - 1) / group;
+        c.chunks = (n + c.chunk - 1) / c.chunk;
+        if (self_tasks_before(c.groups, c.chunks, c.per_group) >= 148 * 2 * 4) return c;
+    }
+    return c;
+}
+
+// Bytes of the partials may not exceed this (n = 119,000 in FP32).
+constexpr size_t SELF_MAX_PARTIALS = size_t(1) << 30;
+
+size_t self_partials(int prec, int64_t n, const SelfCut& c) {
+    return (prec == TCT_F32 ? 4 : 8) * 9 * (size_t)n * (size_t)(c.groups + c.chunks);
+}
+
+template <class V, int NQ, bool UNIFORM>
+int run_self(const double* params, const double* qp, const double* qw, void* out, const void* in,
+             const void* pts, const int32_t* tris, int64_t n, int accumulate, unsigned char* ws,
+             const SelfCut& cut, cudaStream_t st) {
+    using R = typename V::real;
+    using vec = typename V::vec;
+    using L = RecSelf<NQ>;
+    const Consts<R> c = make_consts<R>(params);
+    Rule2D<R> rule;
+    PairWeights<V, NQ> pw;
+    self_rule<V, NQ>(qp, qw, rule, pw);
+    vec* rec = reinterpret_cast<vec*>(ws);
+    R* Wp = reinterpret_cast<R*>(ws + al256(8 * (size_t)L::LEN * n));
+    R* Vp = Wp + cut.chunks * n * 9;
+    far_self_prep<V, NQ, UNIFORM><<<(unsigned)((n + 127) / 128), 128, 0, st>>>(
+        c, rule, (const R*)pts, tris, n, (const R*)in, nullptr, rec);
+    int rc = launch_status("self farfield prep");
+    if (rc) return rc;
+    auto kfn = far_self_main<V, NQ, UNIFORM>;
+    const size_t smem = self_smem<V, NQ>(cut.chunk);
+    if (smem > 48 * 1024 &&
+        cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+            cudaSuccess)
+        return launch_status("self farfield shared memory");
+    const int64_t tasks = self_tasks_before(cut.groups, cut.chunks, cut.per_group);
+    kfn<<<(unsigned)tasks, 128, smem, st>>>(pw, rec, n, cut.strips, cut.chunk, cut.chunks,
+                                            cut.groups, Wp, Vp);
+    if ((rc = launch_status("self farfield main"))) return rc;
+    far_self_reduce<R><<<(unsigned)((n + 31) / 32), 288, 0, st>>>(
+        (const R*)pts, tris, n, (int64_t)cut.strips * 128 * V::H, cut.per_group, cut.chunks, Wp, Vp,
+        (R*)out, accumulate);
+    return launch_status("self farfield reduce");
+}
+
+}  // namespace
+}  // namespace tct
+
+extern "C" size_t tct_farfield_self_workspace_bytes(int kernel, int prec, int64_t n, int n_q) {
+    using namespace tct;
+    if (kernel != kRH || (prec != TCT_F32 && prec != TCT_F64) || self_rec_len(n_q) == 0 ||
+        n < (prec == TCT_F32 ? SELF_MIN_F32 : SELF_MIN_F64) || n >= (int64_t(1) << 31))
+        return 0;
+    const SelfCut c = self_cut(prec, n);
+    const size_t part = self_partials(prec, n, c);
+    if (part > SELF_MAX_PARTIALS) return 0;
+    return al256(8 * (size_t)self_rec_len(n_q) * n) + al256(part);
+}
+
+extern "C" int tct_farfield_self_matvec(int kernel, int prec, void* out, const void* in,
+                                        const void* pts, const int32_t* tris, int64_t n, int n_q,
+                                        const double* quad_pts, const double* quad_wts,
+                                        const double* params, int accumulate, void* workspace,
+                                        size_t workspace_bytes, void* stream) {
+    using namespace tct;
+    TCT_CHECK_ARG(n >= 0, "tct_farfield_self_matvec: negative size");
+    if (n == 0) return TCT_OK;
+    const size_t need = tct_farfield_self_workspace_bytes(kernel, prec, n, n_q);
+    TCT_CHECK_ARG(need > 0, "tct_farfield_self_matvec: kernel %d, precision %d, %d-point rule and "
+                  "%lld triangles are not served (tct_farfield_tris_matvec is)", kernel, prec, n_q,
+                  (long long)n);
+    TCT_CHECK_ARG(out && in && pts && tris && quad_pts && quad_wts && params,
+                  "tct_farfield_self_matvec: null pointer");
+    TCT_CHECK_ARG(workspace && aligned(workspace, 256),
+                  "tct_farfield_self_matvec: workspace not 256-byte aligned");
+    if (workspace_bytes < need) {
+        set_error("tct_farfield_self_matvec: workspace %zu bytes < required %zu", workspace_bytes,
+                  need);
+        return TCT_ERR_OOM;
+    }
+    const SelfCut cut = self_cut(prec, n);
+    unsigned char* ws = reinterpret_cast<unsigned char*>(workspace);
+    cudaStream_t st = as_stream(stream);
+    bool uniform = true;
+    for (int q = 1; q < n_q; q++) uniform = uniform && quad_wts[q] == quad_wts[0];
+#define TCT_SELF(V, NQ, UNI) \
+    return run_self<V, NQ, UNI>(params, quad_pts, quad_wts, out, in, pts, tris, n, accumulate, ws, cut, st)
+    if (prec == TCT_F32) {
+        if (n_q == 3 && uniform) TCT_SELF(VecF32, 3, true);
+        if (n_q == 3) TCT_SELF(VecF32, 3, false);
+        if (n_q == 4) TCT_SELF(VecF32, 4, false);
+        TCT_SELF(VecF32, 7, false);
+    }
+    if (n_q == 3 && uniform) TCT_SELF(VecF64, 3, true);
+    if (n_q == 3) TCT_SELF(VecF64, 3, false);
+    if (n_q == 4) TCT_SELF(VecF64, 4, false);
+    TCT_SELF(VecF64, 7, false);
+#undef TCT_SELF
+}

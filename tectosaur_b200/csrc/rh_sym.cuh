@@ -1,0 +1,274 @@
+// elasticRH3 triangle pairs with the geometry formed once for both directions:
+// shared by the self farfield (far_self.cu) and the FMM's P2P (fmm_p2p.cu).
+//
+// For RH the NQ x NQ point pairs of triangles (a, b) reduce to the symmetric
+// T = sum w_i w_j r^-3 D D^T and its trace (far_common.cuh), and T(a, b) =
+// T(b, a): per unordered pair
+//   W[a] += tr(T) P_b + T M_b,   V[b] += tr(T) P_a + T M_a,
+// P and M = -2 ssc carrying J CsRH0 of the triangle whose input they hold.
+#pragma once
+
+#include <cstring>
+
+#include "far_common.cuh"
+
+namespace tct {
+namespace {
+
+// Two observation triangles per lane (f32x2 halves) in FP32, one in FP64.
+struct VecF32 {
+    using real = float;
+    using vec = f2_t;
+    static constexpr int H = 2;
+    static constexpr float EPS = RH2_EPS;
+    static __device__ __forceinline__ vec make(float a, float b) { return pk(a, b); }
+    static __device__ __forceinline__ vec add(vec a, vec b) { return add2(a, b); }
+    static __device__ __forceinline__ vec mul(vec a, vec b) { return mul2(a, b); }
+    static __device__ __forceinline__ vec fma(vec a, vec b, vec c) { return fma2(a, b, c); }
+    static __device__ __forceinline__ vec rsqrt(vec a) {
+        float x, y;
+        upk(a, x, y);
+        return pk(rsqrtf(x), rsqrtf(y));
+    }
+    static __device__ __forceinline__ float hsum(vec a) {
+        float x, y;
+        upk(a, x, y);
+        return x + y;
+    }
+    static __device__ __forceinline__ void split(vec a, float (&o)[2]) { upk(a, o[0], o[1]); }
+};
+struct VecF64 {
+    using real = double;
+    using vec = double;
+    static constexpr int H = 1;
+    // r^-3 stays finite and D == 0 contributes nothing, as RH2_EPS in FP32
+    static constexpr double EPS = 1e-200;
+    static __device__ __forceinline__ vec make(double a, double) { return a; }
+    static __device__ __forceinline__ vec add(vec a, vec b) { return a + b; }
+    static __device__ __forceinline__ vec mul(vec a, vec b) { return a * b; }
+    static __device__ __forceinline__ vec fma(vec a, vec b, vec c) { return ::fma(a, b, c); }
+    static __device__ __forceinline__ vec rsqrt(vec a) { return ::rsqrt(a); }
+    static __device__ __forceinline__ double hsum(vec a) { return a; }
+    static __device__ __forceinline__ void split(vec a, double (&o)[1]) { o[0] = a; }
+};
+
+// Record of a triangle: its points (3 NQ), P (9), M (9), each one vec (an FP32
+// value twice, an FP64 value once: 8 bytes), padded to 16 bytes.
+template <int NQ>
+struct RecSelf {
+    static constexpr int Y = 0, P = 3 * NQ, M = 3 * NQ + 9, N = 3 * NQ + 18;
+    static constexpr int LEN = (N + 1) / 2 * 2;
+};
+
+// Products of rule weights by point pair, as kernel parameters (constant
+// bank operands).
+template <class V, int NQ>
+struct PairWeights {
+    typename V::vec w[NQ * NQ];
+};
+
+template <class V, int NQ, bool UNIFORM>
+__global__ void __launch_bounds__(128)
+far_self_prep(Consts<typename V::real> c, Rule2D<typename V::real> rule,
+              const typename V::real* __restrict__ pts, const int32_t* __restrict__ tris, int64_t n,
+              const typename V::real* __restrict__ in, const int64_t* __restrict__ orig,
+              typename V::vec* __restrict__ rec) {
+    using R = typename V::real;
+    using L = RecSelf<NQ>;
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    TriGeom<R> s;
+    load_tri(s, pts, tris, i, 0, false, true);
+    const int64_t ii = orig ? orig[i] : i;  // input row of tree-ordered triangles
+    R in9[9];
+#pragma unroll
+    for (int k = 0; k < 9; k++) in9[k] = in[ii * 9 + k];
+    typename V::vec* r = rec + i * L::LEN;
+#pragma unroll
+    for (int q = 0; q < NQ; q++) {
+        const R sx = rule.x[q], sy = rule.y[q];
+        const R sb[3] = {1 - sx - sy, sx, sy};
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            const R y = bary_point(s, sb, d);
+            r[L::Y + 3 * q + d] = V::make(y, y);
+        }
+    }
+    R ssc[3][3];
+#pragma unroll
+    for (int j = 0; j < 3; j++)
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            R a = 0;
+#pragma unroll
+            for (int b = 0; b < 3; b++) a += s.sc[b][j] * in9[b * 3 + d];
+            ssc[d][j] = a;
+        }
+    R scale = s.J * c.CsRH0;
+    if (UNIFORM) scale *= rule.w[0] * rule.w[0];
+    const R B = (ssc[0][0] + ssc[1][1] + ssc[2][2]) * c.CsRH1;
+#pragma unroll
+    for (int d = 0; d < 3; d++)
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            const R p = scale * ((d == j ? B : R(0)) + c.CsRH2 * ssc[j][d] - 2 * ssc[d][j]);
+            const R m = scale * (R(-2) * ssc[d][j]);
+            r[L::P + 3 * d + j] = V::make(p, p);
+            r[L::M + 3 * d + j] = V::make(m, m);
+        }
+#pragma unroll
+    for (int k = L::N; k < L::LEN; k++) r[k] = V::make(0, 0);
+}
+
+// T = sum over the point pairs of w_i w_j r^-3 D D^T (00 01 02 11 12 22) of a
+// staged record against this lane's observation triangles (negated points).
+template <class V, int NQ, bool UNIFORM>
+__device__ __forceinline__ void self_tensor(const typename V::vec* __restrict__ r,
+                                            const typename V::vec (&negx)[NQ][3],
+                                            const PairWeights<V, NQ>& pw,
+                                            typename V::vec (&T)[6]) {
+    using vec = typename V::vec;
+    constexpr int NY = 3 * NQ, NV = (NY + 1) / 2;
+    vec y[2 * NV];
+    const ulonglong2* r2 = reinterpret_cast<const ulonglong2*>(r);
+#pragma unroll
+    for (int k = 0; k < NV; k++) {
+        const ulonglong2 u = r2[k];
+        if constexpr (V::H == 2) {
+            y[2 * k] = u.x;
+            y[2 * k + 1] = u.y;
+        } else {
+            y[2 * k] = __longlong_as_double((long long)u.x);
+            y[2 * k + 1] = __longlong_as_double((long long)u.y);
+        }
+    }
+    const vec eps = V::make(V::EPS, V::EPS), zero = V::make(0, 0);
+#pragma unroll
+    for (int k = 0; k < 6; k++) T[k] = zero;
+#pragma unroll
+    for (int q2 = 0; q2 < NQ; q2++)
+#pragma unroll
+        for (int q1 = 0; q1 < NQ; q1++) {
+            const vec D0 = V::add(y[3 * q2 + 0], negx[q1][0]);
+            const vec D1 = V::add(y[3 * q2 + 1], negx[q1][1]);
+            const vec D2 = V::add(y[3 * q2 + 2], negx[q1][2]);
+            vec rr = V::fma(D0, D0, eps);
+            rr = V::fma(D1, D1, rr);
+            rr = V::fma(D2, D2, rr);
+            const vec invr = V::rsqrt(rr);
+            vec g = V::mul(V::mul(invr, invr), invr);
+            if (!UNIFORM) g = V::mul(g, pw.w[q1 * NQ + q2]);
+            const vec g0 = V::mul(g, D0), g1 = V::mul(g, D1), g2 = V::mul(g, D2);
+            T[0] = V::fma(g0, D0, T[0]);
+            T[1] = V::fma(g0, D1, T[1]);
+            T[2] = V::fma(g0, D2, T[2]);
+            T[3] = V::fma(g1, D1, T[3]);
+            T[4] = V::fma(g1, D2, T[4]);
+            T[5] = V::fma(g2, D2, T[5]);
+        }
+}
+
+// The 18 values P, M of a staged record.
+template <class V, int NQ>
+__device__ __forceinline__ void self_load_pm(const typename V::vec* __restrict__ r,
+                                             typename V::vec (&pm)[18]) {
+    using L = RecSelf<NQ>;
+    constexpr int K0 = L::P / 2, K1 = (L::N + 1) / 2, OFF = L::P % 2;
+    const ulonglong2* r2 = reinterpret_cast<const ulonglong2*>(r);
+    unsigned long long v[2 * (K1 - K0)];
+#pragma unroll
+    for (int k = K0; k < K1; k++) {
+        const ulonglong2 u = r2[k];
+        v[2 * (k - K0)] = u.x;
+        v[2 * (k - K0) + 1] = u.y;
+    }
+#pragma unroll
+    for (int k = 0; k < 18; k++) {
+        if constexpr (V::H == 2) pm[k] = v[OFF + k];
+        else pm[k] = __longlong_as_double((long long)v[OFF + k]);
+    }
+}
+
+// W[3 d + j] += tr(T) P[d][j] + sum_k T[d][k] M[k][j], P = pm[0..8], M = pm[9..17].
+template <class V>
+__device__ __forceinline__ void self_apply(const typename V::vec (&T)[6], typename V::vec S0,
+                                           const typename V::vec (&pm)[18],
+                                           typename V::vec (&W)[9]) {
+    constexpr int IDX[3][3] = {{0, 1, 2}, {1, 3, 4}, {2, 4, 5}};
+#pragma unroll
+    for (int d = 0; d < 3; d++)
+#pragma unroll
+        for (int j = 0; j < 3; j++) {
+            auto w = V::fma(S0, pm[3 * d + j], W[3 * d + j]);
+#pragma unroll
+            for (int k = 0; k < 3; k++) w = V::fma(T[IDX[d][k]], pm[9 + 3 * k + j], w);
+            W[3 * d + j] = w;
+        }
+}
+
+// Sums of nine values over the 16 lanes of a half-warp: value 4 b3 + 2 b2 + b1
+// of the lane's bits 3..1 in lo (both lanes of equal bits 4..1 hold it), value
+// 8 in hi.
+template <typename R>
+__device__ __forceinline__ void half_sum9(const R (&a)[9], int lane, R& lo, R& hi) {
+    const unsigned full = 0xffffffffu;
+    const bool b3 = lane & 8, b2 = lane & 4, b1 = lane & 2;
+    R c[4], e[2];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const R send = b3 ? a[k] : a[4 + k], keep = b3 ? a[4 + k] : a[k];
+        c[k] = keep + __shfl_xor_sync(full, send, 8);
+    }
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const R send = b2 ? c[k] : c[2 + k], keep = b2 ? c[2 + k] : c[k];
+        e[k] = keep + __shfl_xor_sync(full, send, 4);
+    }
+    const R send = b1 ? e[0] : e[1], keep = b1 ? e[1] : e[0];
+    R v = keep + __shfl_xor_sync(full, send, 2);
+    lo = v + __shfl_xor_sync(full, v, 1);
+    R h = a[8] + __shfl_xor_sync(full, a[8], 8);
+    h += __shfl_xor_sync(full, h, 4);
+    h += __shfl_xor_sync(full, h, 2);
+    hi = h + __shfl_xor_sync(full, h, 1);
+}
+
+// Sums over the warp of two sources' nine values: the lower half-warp ends with
+// source 0, the upper with source 1, spread over its lanes as in half_sum9.
+template <typename R>
+__device__ __forceinline__ void warp_sum2x9(const R (&s0)[9], const R (&s1)[9], int lane, R& lo,
+                                            R& hi) {
+    const bool b4 = lane & 16;
+    R a[9];
+#pragma unroll
+    for (int k = 0; k < 9; k++) {
+        const R send = b4 ? s0[k] : s1[k], keep = b4 ? s1[k] : s0[k];
+        a[k] = keep + __shfl_xor_sync(0xffffffffu, send, 16);
+    }
+    half_sum9<R>(a, lane, lo, hi);
+}
+
+// Rule and weight products in the kernels' precision.
+template <class V, int NQ>
+void self_rule(const double* qp, const double* qw, Rule2D<typename V::real>& rule,
+               PairWeights<V, NQ>& pw) {
+    using R = typename V::real;
+    for (int q = 0; q < MAXQ; q++) {
+        rule.x[q] = q < NQ ? (R)qp[2 * q] : R(0);
+        rule.y[q] = q < NQ ? (R)qp[2 * q + 1] : R(0);
+        rule.w[q] = q < NQ ? (R)qw[q] : R(0);
+    }
+    for (int a = 0; a < NQ; a++)
+        for (int b = 0; b < NQ; b++) {
+            const R w = rule.w[a] * rule.w[b];
+            const R h[2] = {w, w};
+            std::memcpy(&pw.w[a * NQ + b], h, sizeof(typename V::vec));
+        }
+}
+
+inline int self_rec_len(int nq) {
+    return nq == 3 ? RecSelf<3>::LEN : nq == 4 ? RecSelf<4>::LEN : nq == 7 ? RecSelf<7>::LEN : 0;
+}
+
+}  // namespace
+}  // namespace tct

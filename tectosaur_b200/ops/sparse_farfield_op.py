@@ -43,6 +43,14 @@ class TriToTriDirectFarfieldOp:
         if self.ws_bytes == 0 and self.n_src > 0:
             raise ValueError("farfield: unsupported kernel/rule (%s, %d points)" % (K_name, self.n_q))
         self.workspace = device.workspace(self.ws_bytes)
+        # one triangle set on both sides: the kernel that forms each pair's
+        # geometry once (0 bytes where it does not serve the configuration)
+        self.self_ws_bytes = 0
+        if np.array_equal(obs_subset, src_subset):
+            self.self_ws_bytes = int(_lib.lib.tct_farfield_self_workspace_bytes(
+                self.kid, self.prec, self.n_obs, self.n_q))
+            if self.self_ws_bytes:
+                self.self_workspace = device.workspace(self.self_ws_bytes)
         self._panel_ws = {}
 
     def autotune(self, x=None):
@@ -53,6 +61,14 @@ class TriToTriDirectFarfieldOp:
 
     def dot_device(self, x, y, accumulate=False, stream=None):
         """y (+)= Far x on device tensors of float_type."""
+        if self.self_ws_bytes:
+            _lib.check(_lib.lib.tct_farfield_self_matvec(
+                self.kid, self.prec, _lib.tptr(y), _lib.tptr(x), _lib.tptr(self.gpu_pts),
+                _lib.tptr(self.gpu_obs_tris), self.n_obs, self.n_q, _lib.dptr(self.qx),
+                _lib.dptr(self.qw), _lib.dptr(self.params), int(bool(accumulate)),
+                _lib.tptr(self.self_workspace), self.self_ws_bytes,
+                _lib.stream_ptr(stream)), "tct_farfield_self_matvec")
+            return y
         _lib.check(_lib.lib.tct_farfield_tris_matvec(
             self.kid, self.prec, _lib.tptr(y), _lib.tptr(x), _lib.tptr(self.gpu_pts),
             _lib.tptr(self.gpu_obs_tris), self.n_obs, _lib.tptr(self.gpu_src_tris), self.n_src,

@@ -1,0 +1,76 @@
+"""The self farfield (tct_farfield_self_matvec: each pair's geometry once for
+both directions) against the general entry point, which the oracle pins
+(test_gpu_kernels.py): group, strip, chunk and tile edges, odd counts, every
+rule, accumulation."""
+import numpy as np
+import pytest
+
+from tectosaur_b200 import _lib
+from tectosaur_b200.ops.sparse_farfield_op import TriToTriDirectFarfieldOp
+from tectosaur_b200.util import device
+
+from helpers import PARAMS, bumpy_mesh, rel
+
+pytestmark = pytest.mark.gpu
+
+# both sides are sums of n terms in tiles of at most 128 with compensated or
+# double totals: sqrt(128) roundings of the partial sums, times 2 sides
+TOL = {np.float32: 4 * np.sqrt(128) * 6e-8, np.float64: 4 * np.sqrt(128) * 1.2e-16}
+
+# the cuts of self_cut: chunks of 64 (32), 128 (64), 256 (128), groups of 512
+# (256) and 1,024 (512) triangles in FP32 (FP64)
+CASES = [(np.float32, 1, n) for n in (1500, 1537, 2303, 9001, 12545, 24833, 49409)]
+CASES += [(np.float32, 2, 1501), (np.float32, 2, 9217), (np.float32, 3, 2049)]
+CASES += [(np.float64, 1, n) for n in (256, 257, 700, 1153, 4481, 6401, 12417)]
+CASES += [(np.float64, 2, 511), (np.float64, 2, 4609), (np.float64, 3, 385)]
+
+
+def _op(ft, nq, n):
+    pts, tris = bumpy_mesh(int(np.ceil(np.sqrt(n / 2))) + 1, seed=n)
+    # a subset in shuffled order, the same on both sides
+    idx = np.random.default_rng(n).permutation(tris.shape[0])[:n]
+    return TriToTriDirectFarfieldOp(nq, "elasticRH3", PARAMS, pts, tris, ft, idx, idx)
+
+
+@pytest.mark.parametrize("ft,nq,n", CASES)
+def test_self_matches_general(cuda, ft, nq, n):
+    op = _op(ft, nq, n)
+    assert op.self_ws_bytes > 0
+    x = device.to_dev(np.random.default_rng(1).standard_normal(9 * n), ft)
+    y = op.dot(x)
+    y2 = op.dot_device(x, y.clone(), accumulate=True)
+    again = op.dot(x)
+    assert cuda.equal(y, again)  # deterministic
+    op.self_ws_bytes = 0
+    want = op.dot(x).cpu().numpy()
+    assert rel(y.cpu().numpy(), want) < TOL[ft]
+    assert rel(y2.cpu().numpy(), 2 * want) < TOL[ft]
+
+
+def test_self_only_for_one_set(cuda):
+    pts, tris = bumpy_mesh(30, seed=2)
+    idx = np.arange(tris.shape[0])
+    make = lambda K, ft, o, s: TriToTriDirectFarfieldOp(1, K, PARAMS, pts, tris, ft, o, s)  # noqa: E731
+    assert make("elasticRH3", np.float32, idx, idx.copy()).self_ws_bytes > 0
+    assert make("elasticRH3", np.float32, idx, idx[::-1]).self_ws_bytes == 0
+    assert make("elasticRH3", np.float32, idx[:-1], idx).self_ws_bytes == 0
+    assert make("elasticH3", np.float32, idx, idx).self_ws_bytes == 0
+
+
+def test_self_refuses(cuda):
+    op = _op(np.float64, 1, 300)
+    t = device.torch()
+    x = t.zeros(9 * 300, dtype=t.float64, device="cuda")
+    y = t.empty_like(x)
+
+    def call(kid, n, n_q, ws_bytes):
+        return _lib.lib.tct_farfield_self_matvec(
+            kid, op.prec, _lib.tptr(y), _lib.tptr(x), _lib.tptr(op.gpu_pts),
+            _lib.tptr(op.gpu_obs_tris), n, n_q, _lib.dptr(op.qx), _lib.dptr(op.qw),
+            _lib.dptr(op.params), 0, _lib.tptr(op.self_workspace), ws_bytes, _lib.stream_ptr())
+
+    assert call(3, 300, 3, op.self_ws_bytes) == _lib.TCT_ERR_ARG      # kernel
+    assert call(op.kid, 255, 3, op.self_ws_bytes) == _lib.TCT_ERR_ARG  # too few triangles
+    assert call(op.kid, 300, 13, op.self_ws_bytes) == _lib.TCT_ERR_ARG  # rule
+    assert call(op.kid, 300, 3, op.self_ws_bytes - 256) == _lib.TCT_ERR_OOM
+    assert call(op.kid, 0, 3, 0) == _lib.TCT_OK
