@@ -403,13 +403,12 @@ size_t tct_fmm_workspace_bytes(int kernel, int prec, int mode, int order, int n_
                                int64_t n_obs, int64_t n_src, int64_t n_obs_nodes,
                                int64_t n_src_nodes);
 
-/* Host-side check of the FMM M2L work plan (no GPU): for order p, nb local
- * terms per lane and `lanes` contraction lanes (a multiple of 32, at most
- * 224; the FP32 M2L uses 192 with two source nodes per pipeline stage, 224
- * with one), out[0] = valid (a, b) pairs covered, out[1] = pairs covered
+/* Host-side check of a lane plan over the full Cartesian terms (no GPU): for
+ * order p, nb local terms per lane and `lanes` lanes (a multiple of 32, at
+ * most 224), out[0] = valid (a, b) pairs covered, out[1] = pairs covered
  * twice (or lanes over their warp's step count), out[2] = the chunk length,
  * out[3] = lanes used, out[4] = summed warp step counts.  Returns 0, or 1
- * when the plan does not fit.  Test support for tct_fmm_matvec. */
+ * when the plan does not fit. */
 int tct_fmm_m2l_plan_stats(int order, int nb, int lanes, int64_t* out);
 
 /* Treecode / FMM farfield matvec for elasticU3, elasticRT3, elasticRA3 and
@@ -419,9 +418,9 @@ int tct_fmm_m2l_plan_stats(int order, int nb, int lanes, int64_t* out);
  *          height, P2P, M2P.
  *   mode 1 (FMM): far = the M2L list (traversal without treecode); P2M, M2M,
  *          M2L, L2L by depth, L2P, P2P.
- * Expansions are Cartesian multipoles / locals of order `order` on
- * monopole and dipole Laplace channels (the reference uses spherical
- * harmonics); which pairs are direct (P2P) is decided by the lists.
+ * Expansions are Cartesian multipoles / locals of order `order`, reduced to
+ * their harmonic terms, on monopole and dipole Laplace channels (the
+ * reference uses spherical harmonics); which pairs are direct (P2P) is decided by the lists.
  * quad_pts (n_q x 2) and quad_wts are the host 2-D rule (n_q in 3, 4, 7,
  * 13); obs_pts / src_pts Real (device); obs_tris / src_tris in tree order;
  * `in` (n_src x 9) and `out` (n_obs x 9) in original order; out (+)=

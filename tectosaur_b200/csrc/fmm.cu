@@ -10,35 +10,44 @@
 // Since D_k / r^3 = d/dx_k (1/r) and D_d = Y_d - X_d with Y = y - C,
 // X = x - C about an expansion centre C:
 //   F[d][j] = Phi[c_dj] + Phi_dip[Y_d m_.j] - X_d Phi_dip[m_.j] + Phi_dip[v_d.]
-// -- Laplace potentials of monopoles and dipoles only.
+// -- Laplace potentials of monopoles and dipoles only.  Charges with the same
+// transformation share one expansion channel: Z_dj carries c_dj, the dipoles
+// Y_d m_.j and (RT) v_d., so F[d][j] = Phi[Z_dj] - X_d Phi[m_.j] (RH: 12
+// channels, U and RT: 4; RA: 4 and the 9 of its obs-normal dipole field).
 //
-// Multipoles (Cartesian, scaled by the node radius s): N_a = sum q Yh^a for a
-// monopole q at Y (Yh = Y / s) and N_a += -(1/s) sum_k a_k w_k Yh^(a - e_k)
-// for a dipole w; the potential at X is
-//   Phi(X) = (1/s) sum_{|a| <= p} (-1)^|a| N_a D_a(X / s),  D_a = (1/a!) d^a (1/|X|),
-// with D from the recurrence
-//   n |X|^2 D_g = -(2n - 1) sum_i X_i D_(g - e_i) - (n - 1) sum_i D_(g - 2e_i).
-// M2M: N^P_a = sum_{b <= a} C(a, b) (s_C / s_P)^|b| (del / s_P)^(a - b) N^C_b,
-// del = C_C - C_P; the centre-dependent channels Y_d m gain del_d times the
-// shifted m channel.
+// Multipoles are Cartesian, scaled by the node radius s and divided by a!:
+// Nt_a = q Yh^a / a! for a monopole q at Y (Yh = Y / s), Nt_a = -(1/s) sum_k
+// w_k Yh^(a - e_k) / (a - e_k)! for a dipole w; the potential at X is
+//   Phi(X) = (1/s) sum_{|a| <= p} (-1)^|a| Nt_a Dc_a(X / s),  Dc_a = d^a (1/|X|).
+// 1/|X| is harmonic, so Dc_(a + 2 e_2) = -Dc_(a + 2 e_0) - Dc_(a + 2 e_1): every
+// order n is spanned by its 2n + 1 derivatives with a_2 <= 1, and moments
+// with a_2 >= 2 fold onto those of the same order exactly.  Only the (p + 1)^2
+// terms with a_2 <= 1 are kept (81 of 165 at p = 8, 121 of 286 at p = 10);
+// the truncation |a| + |b| <= p is by order, which the folding keeps, so the
+// sums are those of the full Cartesian expansion.  The folded monomials
+// H_a(xi) (xi^a / a! summed over what folds onto a) obey
+//   n H_a = xi_0 H_(a - e_0) + xi_1 H_(a - e_1) + xi_2 K_a,  d H_a / d xi_2 = K_a,
+//   K_a = H_(a - e_2) for a_2 = 1, -H_(a + e_2 - 2 e_0) - H_(a + e_2 - 2 e_1) for
+//   a_2 = 0, and d H_a / d xi_k = H_(a - e_k) for k = 0, 1;
+// the derivatives obey (unit-free, r = |X|)
+//   n r^2 Dc_c = -(2n - 1) sum_i c_i X_i Dc_(c - e_i)
+//                -(n - 1) sum_i c_i (c_i - 1) Dc_(c - 2 e_i),
+// closed on c_2 <= 1; c_2 = 2 follows from harmonicity.
+// M2M: Nt^P = fold of sum (s_C/s_P)^|b| Nt^C_b H_e(del / s_P) at b + e,
+// del = C_C - C_P, Z rows gaining del_d m first.
 //
 // Local expansions (FMM mode) about an obs node centre C_o, xi = x - C_o,
-// scaled by the obs node radius: Phi(x) = sum_b L_b (xi / s_o)^b with
-//   M2L: L_b = (1/rho) (s_o/rho)^|b| sum_a (-1)^|a| (s_s/rho)^|a| C(a+b, b)
-//              D_(a+b)(R0 / rho) N_a,   R0 = C_o - C_s, rho = |R0|, |a|+|b| <= p;
-//   L2L: L^C_b = (s_C/s_P)^|b| sum_{c >= b} C(c, b) (del / s_P)^(c - b) L^P_c;
-// the Y_d m channel becomes Yl = Phi[Y_d m] - R0_d Phi[m] (applied to each
-// pair's sums), so that at the target
-//   F[d][j] = L[c_dj](xi) + L[Yl_dj](xi) - xi_d L[m_.j](xi).
+// scaled by the obs node radius: Phi(x) = sum_b Lt_b H_b(xi / s_o), b_2 <= 1, with
+//   M2L: Lt_b = (1/rho) (s_o/rho)^|b| sum_a (-s_s/rho)^|a| Dc_(a+b)(R0 / rho) Nt_a,
+//              R0 = C_o - C_s, rho = |R0|, |a| + |b| <= p, Z rows less R0_d m;
+//   L2L: Lt^C_b = (s_C/s_P)^|b| sum_e H_e(del / s_P) Lt^P_(b+e), |b| + |e| <= p,
+//              Lt^P harmonic in its index as Dc is, Z rows less del_d m.
 //
-// Multi-indices a = (a0, a1, a2), |a| = n <= p, are stored graded:
-// idx(a) = n(n+1)(n+2)/6 + (n - a0)(n - a0 + 1)/2 + a2.
+// Kept terms a, |a| = n <= p, are stored by order: hidx(a) = n^2 + a_2 (n + 1) + a_1.
 //
 // P2P runs the direct farfield's triangle-level pair loop (far_common.cuh) on
 // the listed leaf pairs, from the same per-source records the P2M reads.
 #include <algorithm>
-#include <atomic>
-#include <cstring>
 #include <vector>
 
 #include "far_common.cuh"
@@ -47,32 +56,20 @@ namespace tct {
 namespace {
 
 constexpr int FMM_MAXP = 12;
-constexpr int FMM_LVL = (FMM_MAXP + 1) * (FMM_MAXP + 2) / 2;  // 91 terms in the top level
 
-__host__ __device__ constexpr int n_terms(int p) { return (p + 1) * (p + 2) * (p + 3) / 6; }
-// number of (a, b) pairs with |a| + |b| <= p: C(p + 6, 6)
-__host__ __device__ constexpr int n_terms6(int p) {
-    return (p + 1) * (p + 2) * (p + 3) * (p + 4) * (p + 5) * (p + 6) / 720;
-}
-__host__ __device__ __forceinline__ int midx(int a0, int a1, int a2) {
+// kept terms (a_2 <= 1) up to order p, and their storage index
+__host__ __device__ constexpr int n_harm(int p) { return (p + 1) * (p + 1); }
+__host__ __device__ __forceinline__ int hidx(int a0, int a1, int a2) {
     const int n = a0 + a1 + a2;
-    return n * (n + 1) * (n + 2) / 6 + (n - a0) * (n - a0 + 1) / 2 + a2;
+    return n * n + a2 * (n + 1) + a1;
 }
-// position of (a0, ., a2) within level n
-__device__ __forceinline__ int lidx(int n, int a0, int a2) { return (n - a0) * (n - a0 + 1) / 2 + a2; }
-
-__host__ __device__ __forceinline__ void decode(int g, int& a0, int& a1, int& a2) {
-    int n = 0;
-    while (n_terms(n) <= g) n++;
-    int rem = n > 0 ? g - n_terms(n - 1) : 0;
-    a0 = n;
-    int off = 0;
-    while (off + (n - a0 + 1) <= rem) {
-        off += n - a0 + 1;
-        a0--;
-    }
-    a2 = rem - off;
-    a1 = n - a0 - a2;
+__host__ __device__ __forceinline__ void hdecode(int g, int& n, int& a0, int& a1, int& a2) {
+    n = 0;
+    while ((n + 1) * (n + 1) <= g) n++;
+    const int w = g - n * n;
+    a2 = w > n ? 1 : 0;
+    a1 = w - a2 * (n + 1);
+    a0 = n - a1 - a2;
 }
 
 template <typename R>
@@ -82,19 +79,39 @@ __device__ __forceinline__ R ipow(R x, int n) {
     return v;
 }
 
-// binomial table C(n, k), n, k <= FMM_MAXP, built in shared memory
-template <typename R>
-__device__ __forceinline__ void fill_binom(R* bin) {
-    if (threadIdx.x <= FMM_MAXP) {
-        const int n = threadIdx.x;
-        R v = 1;
-        for (int k = 0; k <= FMM_MAXP; k++) {
-            bin[n * (FMM_MAXP + 1) + k] = (k <= n) ? v : R(0);
-            v = v * (R)(n - k) / (R)(k + 1);
-        }
+// H_(a - e_0), H_(a - e_1) and K_a of term (n, a1, a2), n >= 1, from the
+// level n - 1 terms prev(0 .. 2n - 2) (0 where an index would be negative).
+template <typename R, typename F>
+__device__ __forceinline__ void harm_below(int n, int a1, int a2, F&& prev, R& h0, R& h1, R& k) {
+    const int a0 = n - a1 - a2;
+    const int off = a2 * n + a1;  // (a0 - 1, a1, a2) of level n - 1
+    h0 = a0 >= 1 ? prev(off) : R(0);
+    h1 = a1 >= 1 ? prev(off - 1) : R(0);
+    if (a2) {
+        k = prev(a1);
+    } else {
+        k = R(0);
+        if (a0 >= 2) k -= prev(n + a1);
+        if (a1 >= 2) k -= prev(n + a1 - 2);
     }
 }
-#define BIN(n, k) bin[(n) * (FMM_MAXP + 1) + (k)]
+
+// H_a(xi), |a| <= p, by one warp into E (a lane per term of a level).
+template <typename R>
+__device__ __forceinline__ void harm_warp(R* E, int p, R x0, R x1, R x2, int lane) {
+    if (lane == 0) E[0] = R(1);
+    __syncwarp();
+    for (int n = 1; n <= p; n++) {
+        if (lane <= 2 * n) {
+            const int a2 = lane > n ? 1 : 0, a1 = lane - a2 * (n + 1);
+            const R* P = E + (n - 1) * (n - 1);
+            R h0, h1, k;
+            harm_below<R>(n, a1, a2, [&](int i) { return P[i]; }, h0, h1, k);
+            E[n * n + lane] = (x0 * h0 + x1 * h1 + x2 * k) / (R)n;
+        }
+        __syncwarp();
+    }
+}
 
 // Per-kernel channel layout.
 //   U, RT, RH: F[d][j] as above (NOU = 3J outputs per target point).
@@ -113,11 +130,10 @@ struct Chan {
     // then v(9) for RT or a'(3) for RA
     static constexpr int XT = 3 + NOU + 3 * J;
     static constexpr int REC = XT + (HAS_V ? 9 : 0) + (HAS_A ? 3 : 0);
-    static constexpr int NV = HAS_V ? 3 : (HAS_A ? 9 : 0);
-    // expansion channels: mono (NOU), Y (NOU), M (J), V / A dipoles (NV)
-    static constexpr int NCH = 2 * NOU + J + NV;
+    // expansion channels: Z (NOU), M (J), RA's dipoles (9)
+    static constexpr int NCH = NOU + J + (HAS_A ? 9 : 0);
     static constexpr int NCHP = (NCH + 3) / 4 * 4;  // padded row of one term
-    static constexpr int CH_MONO = 0, CH_Y = NOU, CH_M = 2 * NOU, CH_V = 2 * NOU + J;
+    static constexpr int CH_M = NOU, CH_V = NOU + J;
 };
 
 // Charges of source quadrature point q from the far_prep record r.
@@ -167,7 +183,7 @@ __device__ __forceinline__ void point_charges(const Consts<R>& c, const R* __res
 }
 
 // Combine the expansion channels at a target into F (the M2P/L2P epilogue).
-// X is the target relative to the centre the Y channel refers to.
+// X is the target relative to the expansion centre.
 template <typename R, int K>
 __device__ __forceinline__ void combine(const R (&phi)[Chan<K>::NCH], const R X[3], const R nrm[3],
                                         R (&acc)[Chan<K>::NO]) {
@@ -175,19 +191,52 @@ __device__ __forceinline__ void combine(const R (&phi)[Chan<K>::NCH], const R X[
 #pragma unroll
     for (int d = 0; d < 3; d++)
 #pragma unroll
-        for (int j = 0; j < C::J; j++) {
-            const int oc = d * C::J + j;
-            acc[oc] += phi[C::CH_MONO + oc] + phi[C::CH_Y + oc] - X[d] * phi[C::CH_M + j];
-        }
-    if (C::HAS_V) {
-#pragma unroll
-        for (int d = 0; d < 3; d++) acc[d] += phi[C::CH_V + d];
-    }
+        for (int j = 0; j < C::J; j++) acc[d * C::J + j] += phi[d * C::J + j] - X[d] * phi[C::CH_M + j];
     if (C::HAS_A) {
 #pragma unroll
         for (int d = 0; d < 3; d++)
             acc[C::NOU + d] -= nrm[0] * phi[C::CH_V + 3 * d] + nrm[1] * phi[C::CH_V + 3 * d + 1] +
                                nrm[2] * phi[C::CH_V + 3 * d + 2];
+    }
+}
+
+// Z rows of one term plus t_d times its M channels.
+template <typename R, int K>
+__device__ __forceinline__ void shift_z(R (&v)[Chan<K>::NCHP], R t0, R t1, R t2) {
+    using C = Chan<K>;
+#pragma unroll
+    for (int j = 0; j < C::J; j++) {
+        v[0 * C::J + j] += t0 * v[C::CH_M + j];
+        v[1 * C::J + j] += t1 * v[C::CH_M + j];
+        v[2 * C::J + j] += t2 * v[C::CH_M + j];
+    }
+}
+
+template <typename R, int N>
+__device__ __forceinline__ void load_row(R (&v)[N], const R* __restrict__ src) {
+    constexpr int PER = 16 / sizeof(R);
+    static_assert(N % 4 == 0, "rows are padded to four values");
+#pragma unroll
+    for (int k = 0; k < N / PER; k++) {
+        if constexpr (sizeof(R) == 4) {
+            const float4 q = reinterpret_cast<const float4*>(src)[k];
+            v[4 * k] = q.x; v[4 * k + 1] = q.y; v[4 * k + 2] = q.z; v[4 * k + 3] = q.w;
+        } else {
+            const double2 q = reinterpret_cast<const double2*>(src)[k];
+            v[2 * k] = q.x; v[2 * k + 1] = q.y;
+        }
+    }
+}
+template <typename R, int N>
+__device__ __forceinline__ void store_row(R* __restrict__ dst, const R (&v)[N]) {
+    constexpr int PER = 16 / sizeof(R);
+#pragma unroll
+    for (int k = 0; k < N / PER; k++) {
+        if constexpr (sizeof(R) == 4)
+            reinterpret_cast<float4*>(dst)[k] =
+                make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+        else
+            reinterpret_cast<double2*>(dst)[k] = make_double2(v[2 * k], v[2 * k + 1]);
     }
 }
 
@@ -214,133 +263,205 @@ __device__ __forceinline__ void target_point(const TriGeom<R>& o, const Rule2D<R
 }
 
 // ---- P2M -------------------------------------------------------------------
-// One block per source leaf; thread g owns term g of every channel.
+// One block per source leaf, a thread per kept term.  For 32 source points at
+// a time warp 0 tabulates H_a in shared memory (a lane per point) while warp 1
+// forms the points' charges; then every thread adds the points to its term.
+__host__ __device__ constexpr int p2m_threads(int p) {
+    return n_harm(p) <= 64 ? 64 : (n_harm(p) + 31) / 32 * 32;
+}
+template <int K>
+__host__ __device__ constexpr int p2m_reals(int p) {
+    return 33 * n_harm(p) + 32 * ((Chan<K>::REC + 1) | 1);
+}
+
 template <typename R, int K, int NQ>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(192)
 fmm_p2m(Consts<R> c, int p, const int64_t* __restrict__ leaves, const int64_t* __restrict__ nstart,
         const int64_t* __restrict__ nend, const R* __restrict__ ncent, const R* __restrict__ nrad,
         const R* __restrict__ rec, R* __restrict__ mom) {
     using C = Chan<K>;
     using L = Rec<K, NQ>;
-    const int NT = n_terms(p);
+    constexpr int CS = (C::REC + 1) | 1;  // odd stride of a point's charges
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    R* Hs = reinterpret_cast<R*>(smem_raw);  // NT x 33
+    const int NT = n_harm(p);
+    R* cs = Hs + 33 * NT;                    // 32 x CS
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t node = leaves[blockIdx.x];
     const R c0 = ncent[3 * node], c1 = ncent[3 * node + 1], c2 = ncent[3 * node + 2];
     const R inv_s = R(1) / nrad[node];
-    const int64_t t0 = nstart[node], t1 = nend[node];
-    R* M = mom + node * (int64_t)C::NCHP * NT;
-    for (int g = threadIdx.x; g < NT; g += blockDim.x) {
-        int a0, a1, a2;
-        decode(g, a0, a1, a2);
-        R acc[C::NCH];
+    const int64_t q0 = nstart[node] * NQ, q1 = nend[node] * NQ;
+    const int g = threadIdx.x;
+    // this thread's term: tables of the terms its H derivatives read (the
+    // constant term's row with factor 0 where there is none)
+    int i0 = 0, i1 = 0, ka = 0, kb = 0;
+    R f0 = 0, f1 = 0, fa = 0, fb = 0;
+    if (g > 0 && g < NT) {
+        int n, a0, a1, a2;
+        hdecode(g, n, a0, a1, a2);
+        const int base = (n - 1) * (n - 1);
+        if (a0 >= 1) { i0 = base + a2 * n + a1; f0 = 1; }
+        if (a1 >= 1) { i1 = base + a2 * n + a1 - 1; f1 = 1; }
+        if (a2) { ka = base + a1; fa = 1; }
+        else {
+            if (a0 >= 2) { ka = base + n + a1; fa = -1; }
+            if (a1 >= 2) { kb = base + n + a1 - 2; fb = -1; }
+        }
+    }
+    R acc[C::NCHP];
 #pragma unroll
-        for (int k = 0; k < C::NCH; k++) acc[k] = 0;
-        for (int64_t t = t0; t < t1; t++) {
-            for (int q = 0; q < NQ; q++) {
-                R ch[C::REC];
-                point_charges<R, K, NQ>(c, rec + t * L::LEN, q, ch);
-                const R Y[3] = {ch[0] - c0, ch[1] - c1, ch[2] - c2};
-                const R Yh[3] = {Y[0] * inv_s, Y[1] * inv_s, Y[2] * inv_s};
-                const R p0 = ipow(Yh[0], a0 > 0 ? a0 - 1 : 0);
-                const R p1 = ipow(Yh[1], a1 > 0 ? a1 - 1 : 0);
-                const R p2 = ipow(Yh[2], a2 > 0 ? a2 - 1 : 0);
-                const R f0 = a0 > 0 ? p0 * Yh[0] : R(1);
-                const R f1 = a1 > 0 ? p1 * Yh[1] : R(1);
-                const R f2 = a2 > 0 ? p2 * Yh[2] : R(1);
-                const R mono = f0 * f1 * f2;
-                // dipole factors: -(1/s) a_k Yh^(a - e_k)
-                const R e0 = a0 > 0 ? -inv_s * (R)a0 * p0 * f1 * f2 : R(0);
-                const R e1 = a1 > 0 ? -inv_s * (R)a1 * f0 * p1 * f2 : R(0);
-                const R e2 = a2 > 0 ? -inv_s * (R)a2 * f0 * f1 * p2 : R(0);
-#pragma unroll
-                for (int o = 0; o < C::NOU; o++) acc[C::CH_MONO + o] += ch[3 + o] * mono;
-#pragma unroll
-                for (int j = 0; j < C::J; j++) {
-                    const R mk0 = ch[3 + C::NOU + 0 * C::J + j], mk1 = ch[3 + C::NOU + 1 * C::J + j],
-                            mk2 = ch[3 + C::NOU + 2 * C::J + j];
-                    const R dm = e0 * mk0 + e1 * mk1 + e2 * mk2;
-                    acc[C::CH_M + j] += dm;
-#pragma unroll
-                    for (int d = 0; d < 3; d++) acc[C::CH_Y + d * C::J + j] += Y[d] * dm;
-                }
-                if (C::HAS_V) {
-#pragma unroll
-                    for (int d = 0; d < 3; d++)
-                        acc[C::CH_V + d] += e0 * ch[C::XT + 3 * d] + e1 * ch[C::XT + 3 * d + 1] +
-                                            e2 * ch[C::XT + 3 * d + 2];
-                }
-                if (C::HAS_A) {
-#pragma unroll
-                    for (int d = 0; d < 3; d++) {
-                        const R ad = ch[C::XT + d];
-                        acc[C::CH_V + 3 * d + 0] += e0 * ad;
-                        acc[C::CH_V + 3 * d + 1] += e1 * ad;
-                        acc[C::CH_V + 3 * d + 2] += e2 * ad;
+    for (int k = 0; k < C::NCHP; k++) acc[k] = 0;
+    for (int64_t qb = q0; qb < q1; qb += 32) {
+        const int np = (int)min((int64_t)32, q1 - qb);
+        __syncthreads();
+        if (warp < 2 && lane < np) {
+            const int64_t t = (qb + lane) / NQ;
+            const int q = (int)(qb + lane - t * NQ);
+            const R* r = rec + t * L::LEN;
+            const R Y[3] = {r[L::Y + 3 * q] - c0, r[L::Y + 3 * q + 1] - c1, r[L::Y + 3 * q + 2] - c2};
+            if (warp == 0) {
+                const R x0 = Y[0] * inv_s, x1 = Y[1] * inv_s, x2 = Y[2] * inv_s;
+                Hs[lane] = R(1);
+                for (int n = 1; n <= p; n++) {
+                    const R rn = R(1) / (R)n;
+                    const R* P = Hs + (n - 1) * (n - 1) * 33 + lane;
+                    for (int w = 0; w <= 2 * n; w++) {
+                        const int a2 = w > n ? 1 : 0, a1 = w - a2 * (n + 1);
+                        R h0, h1, k;
+                        harm_below<R>(n, a1, a2, [&](int i) { return P[33 * i]; }, h0, h1, k);
+                        Hs[(n * n + w) * 33 + lane] = (x0 * h0 + x1 * h1 + x2 * k) * rn;
                     }
+                }
+            } else {
+                R ch[C::REC];
+                point_charges<R, K, NQ>(c, r, q, ch);
+#pragma unroll
+                for (int d = 0; d < 3; d++) ch[d] = Y[d];
+#pragma unroll
+                for (int k = 0; k < C::REC; k++) cs[lane * CS + k] = ch[k];
+            }
+        }
+        __syncthreads();
+        if (g >= NT) continue;
+        for (int i = 0; i < np; i++) {
+            const R* ch = cs + i * CS;
+            const R h = Hs[g * 33 + i];
+            const R e0 = -inv_s * (f0 * Hs[i0 * 33 + i]);
+            const R e1 = -inv_s * (f1 * Hs[i1 * 33 + i]);
+            const R e2 = -inv_s * (fa * Hs[ka * 33 + i] + fb * Hs[kb * 33 + i]);
+#pragma unroll
+            for (int j = 0; j < C::J; j++) {
+                const R dm = e0 * ch[3 + C::NOU + j] + e1 * ch[3 + C::NOU + C::J + j] +
+                             e2 * ch[3 + C::NOU + 2 * C::J + j];
+                acc[C::CH_M + j] += dm;
+#pragma unroll
+                for (int d = 0; d < 3; d++)
+                    acc[d * C::J + j] += ch[3 + d * C::J + j] * h + ch[d] * dm;
+            }
+            if constexpr (C::HAS_V) {
+#pragma unroll
+                for (int d = 0; d < 3; d++)
+                    acc[d] += e0 * ch[C::XT + 3 * d] + e1 * ch[C::XT + 3 * d + 1] +
+                              e2 * ch[C::XT + 3 * d + 2];
+            }
+            if constexpr (C::HAS_A) {
+#pragma unroll
+                for (int d = 0; d < 3; d++) {
+                    const R ad = ch[C::XT + d];
+                    acc[C::CH_V + 3 * d + 0] += e0 * ad;
+                    acc[C::CH_V + 3 * d + 1] += e1 * ad;
+                    acc[C::CH_V + 3 * d + 2] += e2 * ad;
                 }
             }
         }
-#pragma unroll
-        for (int k = 0; k < C::NCHP; k++) M[g * C::NCHP + k] = k < C::NCH ? acc[k] : R(0);
     }
+    if (g < NT) store_row<R, C::NCHP>(mom + (node * (int64_t)NT + g) * C::NCHP, acc);
 }
 
 // ---- M2M -------------------------------------------------------------------
-// One block per parent node of one height; children are final.
+// One block per parent node of one height; children are final.  Warp c
+// tabulates H_e of child c; per child the rows (scaled, Z moved to the
+// parent's centre) are staged and a thread forms four channels of one term.
+template <int K>
+__host__ __device__ constexpr int m2m_reals(int p) {
+    return n_harm(p) * Chan<K>::NCHP + 8 * n_harm(p);
+}
+
 template <typename R, int K>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(256)
 fmm_m2m(int p, const int64_t* __restrict__ parents, const int64_t* __restrict__ children,
         const R* __restrict__ ncent, const R* __restrict__ nrad, R* __restrict__ mom) {
     using C = Chan<K>;
-    __shared__ R bin[(FMM_MAXP + 1) * (FMM_MAXP + 1)];
-    fill_binom(bin);
-    __syncthreads();
-    const int NT = n_terms(p);
+    constexpr int Q = C::NCHP / 4;
+    constexpr int MAXI = (n_harm(FMM_MAXP) * Q + 255) / 256;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int NT = n_harm(p);
+    R* rows = reinterpret_cast<R*>(smem_raw);  // NT x NCHP
+    R* E = rows + NT * C::NCHP;                // 8 x NT
     const int64_t P = parents[blockIdx.x];
     const R sP = nrad[P];
-    R* MP = mom + P * (int64_t)C::NCHP * NT;
-    for (int g = threadIdx.x; g < NT; g += blockDim.x) {
-        int a0, a1, a2;
-        decode(g, a0, a1, a2);
-        R acc[C::NCH];
+    {
+        const int64_t cn = children[8 * P + (threadIdx.x >> 5)];
+        harm_warp<R>(E + (threadIdx.x >> 5) * NT, p, (ncent[3 * cn] - ncent[3 * P]) / sP,
+                     (ncent[3 * cn + 1] - ncent[3 * P + 1]) / sP,
+                     (ncent[3 * cn + 2] - ncent[3 * P + 2]) / sP, threadIdx.x & 31);
+    }
+    R acc[MAXI][4];
 #pragma unroll
-        for (int k = 0; k < C::NCH; k++) acc[k] = 0;
-        for (int cidx = 0; cidx < 8; cidx++) {
-            const int64_t cn = children[8 * P + cidx];
-            const R* MC = mom + cn * (int64_t)C::NCHP * NT;
-            const R del[3] = {ncent[3 * cn] - ncent[3 * P], ncent[3 * cn + 1] - ncent[3 * P + 1],
-                              ncent[3 * cn + 2] - ncent[3 * P + 2]};
-            const R dh[3] = {del[0] / sP, del[1] / sP, del[2] / sP};
-            const R ratio = nrad[cn] / sP;
-            R sm[C::NCH];  // shifted child moments
+    for (int t = 0; t < MAXI; t++)
 #pragma unroll
-            for (int k = 0; k < C::NCH; k++) sm[k] = 0;
-            R q0 = 1;
-            for (int b0 = a0; b0 >= 0; b0--) {
-                R q1 = 1;
-                for (int b1 = a1; b1 >= 0; b1--) {
-                    R q2 = 1;
-                    for (int b2 = a2; b2 >= 0; b2--) {
-                        const R coef = BIN(a0, b0) * BIN(a1, b1) * BIN(a2, b2) * q0 * q1 * q2 *
-                                       ipow(ratio, b0 + b1 + b2);
-                        const R* nb = MC + midx(b0, b1, b2) * C::NCHP;
+        for (int k = 0; k < 4; k++) acc[t][k] = 0;
+    for (int ci = 0; ci < 8; ci++) {
+        const int64_t cn = children[8 * P + ci];
+        const R ratio = nrad[cn] / sP;
+        __syncthreads();
+        for (int g = threadIdx.x; g < NT; g += blockDim.x) {
+            int n, a0, a1, a2;
+            hdecode(g, n, a0, a1, a2);
+            R v[C::NCHP];
+            load_row<R, C::NCHP>(v, mom + (cn * (int64_t)NT + g) * C::NCHP);
+            shift_z<R, K>(v, ncent[3 * cn] - ncent[3 * P], ncent[3 * cn + 1] - ncent[3 * P + 1],
+                          ncent[3 * cn + 2] - ncent[3 * P + 2]);
+            const R f = ipow(ratio, n);
 #pragma unroll
-                        for (int k = 0; k < C::NCH; k++) sm[k] += coef * nb[k];
-                        q2 *= dh[2];
-                    }
-                    q1 *= dh[1];
-                }
-                q0 *= dh[0];
-            }
-#pragma unroll
-            for (int k = 0; k < C::NCH; k++) acc[k] += sm[k];
-            // Y_d m channel: + del_d times the shifted m channel
-#pragma unroll
-            for (int d = 0; d < 3; d++)
-#pragma unroll
-                for (int j = 0; j < C::J; j++) acc[C::CH_Y + d * C::J + j] += del[d] * sm[C::CH_M + j];
+            for (int k = 0; k < C::NCHP; k++) v[k] *= f;
+            store_row<R, C::NCHP>(rows + g * C::NCHP, v);
         }
+        __syncthreads();
+        const R* Ec = E + ci * NT;
 #pragma unroll
-        for (int k = 0; k < C::NCHP; k++) MP[g * C::NCHP + k] = k < C::NCH ? acc[k] : R(0);
+        for (int t = 0; t < MAXI; t++) {
+            const int it = threadIdx.x + t * 256;
+            if (it >= NT * Q) break;
+            const int g = it / Q, qd = it - g * Q;
+            int n, a0, a1, a2;
+            hdecode(g, n, a0, a1, a2);
+            // adds f * sum_{b0 <= A0, b1 <= A1} H_(A0 - b0, A1 - b1, e2) row_(b0, b1, b2)
+            auto conv = [&](int A0, int A1, int e2, int b2, R f) {
+                for (int b0 = 0; b0 <= A0; b0++)
+                    for (int b1 = 0; b1 <= A1; b1++) {
+                        const R e = f * Ec[hidx(A0 - b0, A1 - b1, e2)];
+                        R v[4];
+                        load_row<R, 4>(v, rows + hidx(b0, b1, b2) * C::NCHP + 4 * qd);
+#pragma unroll
+                        for (int k = 0; k < 4; k++) acc[t][k] += e * v[k];
+                    }
+            };
+            if (a2) {
+                conv(a0, a1, 1, 0, R(1));
+                conv(a0, a1, 0, 1, R(1));
+            } else {
+                conv(a0, a1, 0, 0, R(1));
+                if (a0 >= 2) conv(a0 - 2, a1, 1, 1, R(-1));
+                if (a1 >= 2) conv(a0, a1 - 2, 1, 1, R(-1));
+            }
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < MAXI; t++) {
+        const int it = threadIdx.x + t * 256;
+        if (it >= NT * Q) break;
+        store_row<R, 4>(mom + P * (int64_t)NT * C::NCHP + 4 * it, acc[t]);
     }
 }
 
@@ -351,7 +472,6 @@ __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc) {
                  : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait_group() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
@@ -660,8 +780,13 @@ fmm_p2p_rh2(Rule2D<float> rule, const float* __restrict__ pts,
 
 // ---- M2P (treecode) --------------------------------------------------------
 // One block per obs leaf with a non-empty M2P list; the moments of each listed
-// source node are staged in shared memory; a thread per target point; the D
-// recurrence keeps its last three levels in a per-thread ring.
+// source node are staged in shared memory; a lane per target point, Dc by
+// order through the warp's ring of the last three orders.
+template <int K>
+__host__ __device__ constexpr int m2p_reals(int p) {
+    return n_harm(p) * Chan<K>::NCHP + 4 * 3 * (2 * p + 1) * 32;
+}
+
 template <typename R, int K>
 __global__ void __launch_bounds__(128)
 fmm_m2p(int p, Rule2D<R> rule, int nq, const int64_t* __restrict__ obs_nodes,
@@ -672,10 +797,10 @@ fmm_m2p(int p, Rule2D<R> rule, int nq, const int64_t* __restrict__ obs_nodes,
     using C = Chan<K>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     R* sm = reinterpret_cast<R*>(smem_raw);
-    const int NT = n_terms(p);
+    const int NT = n_harm(p), LV = 2 * p + 1;
+    R* ring = sm + NT * C::NCHP + (threadIdx.x >> 5) * 3 * LV * 32 + (threadIdx.x & 31);
     const int64_t node = obs_nodes[blockIdx.x];
     const int64_t t0 = o_start[node] * nq, t1 = o_end[node] * nq;
-    R Dr[3][FMM_LVL];
     for (int64_t tb = t0; tb < t1; tb += blockDim.x) {
         const int64_t t = tb + threadIdx.x;
         const bool valid = t < t1;
@@ -701,34 +826,33 @@ fmm_m2p(int p, Rule2D<R> rule, int nq, const int64_t* __restrict__ obs_nodes,
             const R Xh[3] = {X[0] * inv_s, X[1] * inv_s, X[2] * inv_s};
             const R inv_r2 = R(1) / (Xh[0] * Xh[0] + Xh[1] * Xh[1] + Xh[2] * Xh[2]);
             R phi[C::NCH];
-            Dr[0][0] = sqrt(inv_r2);
+            const R d0 = sqrt(inv_r2);
+            ring[0] = d0;
 #pragma unroll
-            for (int k = 0; k < C::NCH; k++) phi[k] = sm[k] * Dr[0][0];
-            int g = 1;
+            for (int k = 0; k < C::NCH; k++) phi[k] = sm[k] * d0;
             for (int n = 1; n <= p; n++) {
                 const R cA = -(R)(2 * n - 1) / (R)n * inv_r2;
                 const R cB = -(R)(n - 1) / (R)n * inv_r2;
                 const R sgn = (n & 1) ? R(-1) : R(1);
-                R* cur = Dr[n % 3];
-                const R* prv = Dr[(n - 1) % 3];
-                const R* pp = Dr[(n + 1) % 3];  // level n - 2
-                for (int a0 = n; a0 >= 0; a0--)
-                    for (int a2 = 0; a2 <= n - a0; a2++, g++) {
-                        const int a1 = n - a0 - a2;
-                        R s1 = 0, s2 = 0;
-                        if (a0 > 0) s1 += Xh[0] * prv[lidx(n - 1, a0 - 1, a2)];
-                        if (a1 > 0) s1 += Xh[1] * prv[lidx(n - 1, a0, a2)];
-                        if (a2 > 0) s1 += Xh[2] * prv[lidx(n - 1, a0, a2 - 1)];
-                        if (a0 > 1) s2 += pp[lidx(n - 2, a0 - 2, a2)];
-                        if (a1 > 1) s2 += pp[lidx(n - 2, a0, a2)];
-                        if (a2 > 1) s2 += pp[lidx(n - 2, a0, a2 - 2)];
-                        const R Dg = cA * s1 + cB * s2;
-                        cur[lidx(n, a0, a2)] = Dg;
-                        const R sD = sgn * Dg;
-                        const R* nrow = sm + g * C::NCHP;
+                R* cur = ring + (n % 3) * LV * 32;
+                const R* p1 = ring + ((n + 2) % 3) * LV * 32;  // order n - 1
+                const R* p2 = ring + ((n + 1) % 3) * LV * 32;  // order n - 2
+                for (int w = 0; w <= 2 * n; w++) {
+                    const int a2 = w > n ? 1 : 0, a1 = w - a2 * (n + 1), a0 = n - a1 - a2;
+                    R s1 = 0, s2 = 0;
+                    if (a0 > 0) s1 += (R)a0 * Xh[0] * p1[32 * (a2 * n + a1)];
+                    if (a1 > 0) s1 += (R)a1 * Xh[1] * p1[32 * (a2 * n + a1 - 1)];
+                    if (a2 > 0) s1 += Xh[2] * p1[32 * a1];
+                    if (a0 > 1) s2 += (R)(a0 * (a0 - 1)) * p2[32 * (a2 * (n - 1) + a1)];
+                    if (a1 > 1) s2 += (R)(a1 * (a1 - 1)) * p2[32 * (a2 * (n - 1) + a1 - 2)];
+                    const R Dg = cA * s1 + cB * s2;
+                    cur[32 * w] = Dg;
+                    const R sD = sgn * Dg;
+                    R v[C::NCHP];
+                    load_row<R, C::NCHP>(v, sm + (n * n + w) * C::NCHP);
 #pragma unroll
-                        for (int k = 0; k < C::NCH; k++) phi[k] += nrow[k] * sD;
-                    }
+                    for (int k = 0; k < C::NCH; k++) phi[k] += v[k] * sD;
+                }
             }
 #pragma unroll
             for (int k = 0; k < C::NCH; k++) phi[k] *= inv_s;
@@ -742,868 +866,403 @@ fmm_m2p(int p, Rule2D<R> rule, int nq, const int64_t* __restrict__ obs_nodes,
     }
 }
 
-// ---- M2L (FMM) -------------------------------------------------------------
-// Written as L_b = (s_o/rho)^|b| / (rho b!) sum_a f_|a| Dc_(a+b) Nt_a with
-// Dc_c = c! D_c(R0 / rho), f_n = (-1)^n (s_s/rho)^n and Nt_a = N_a / a! (the
-// moments are divided by a! once, after M2M, by fmm_moment_factorials), so a
-// pair's source moments are used as stored; the Yl correction (- R0_d times
-// the m channel) is linear in the moments and applied to each source row.
-template <typename R>
-__global__ void __launch_bounds__(128)
-fmm_moment_factorials(int p, int nchp, int64_t n_nodes, R* __restrict__ mom) {
-    const int NT = n_terms(p);
-    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= n_nodes * NT * nchp) return;
-    int a0, a1, a2;
-    decode((int)((e / nchp) % NT), a0, a1, a2);
-    R f = 1;
-    for (int k = 2; k <= a0; k++) f *= (R)k;
-    for (int k = 2; k <= a1; k++) f *= (R)k;
-    for (int k = 2; k <= a2; k++) f *= (R)k;
-    mom[e] /= f;
-}
+// ---- M2L (FMM), one CTA per observation node --------------------------------
+// Lt_b = (s_o/rho)^|b| / rho sum_a (-s_s/rho)^|a| Dc_(a+b) Nt_a = sum_a
+// Dh_(a+b) S_|a| Nt_a with Dh_c = Dc_c (s_o/rho)^|c| / rho and S_n = (-s_s/s_o)^n.
+//
+// The four warps take equal slices of the node's list and work alone until
+// their sums are added at the end (in warp order: deterministic).  A warp
+//  * forms Dh for PB pairs at a time, 32 / PB lanes a pair, order by order,
+//    into the pairs' cubes: entry c at c_0 + S1 c_1 + S2 c_2, additive, so
+//    Dh_(a+b) is one load at lin(a) + lin(b);
+//  * per pair stages the source rows in shared memory, scaled by S_|a| and
+//    with R0_d m taken off the Z channels;
+//  * walks the terms a: all lanes take the same a (its row is one broadcast),
+//    lane l the local terms b = l, 32 + l, ... that |a| + |b| <= p allows;
+//    where at most 16 (4) terms b are left the half-warps (lane quads) take
+//    2 (8) terms a at once into sums of their own.  At p = 8 that is 60
+//    steps for 1,365 (a, b) pairs, 71 % of the lanes, each step NCH
+//    multiply-adds a lane against one gathered load.
+// Bound by the FMA pipe and, next, the shared-memory loads (60 gathers and 45
+// rows of 48 bytes a pair at p = 8).
+constexpr int M2L_WARPS = 4;
 
 template <typename R>
-__device__ __forceinline__ R mfact(int b0, int b1, int b2) {
-    R f = 1;
-    for (int k = 2; k <= b0; k++) f *= (R)k;
-    for (int k = 2; k <= b1; k++) f *= (R)k;
-    for (int k = 2; k <= b2; k++) f *= (R)k;
-    return f;
-}
-
-// ---- M2L, one CTA per observation node ------------------------------------
-// L_b = 1/b! sum over the node's M2L list of (s_o/rho)^|b| / rho *
-// sum_a f_|a| Dc_(a+b) (N_a with the Yl correction Y_dj - R0_d m_j), |a| + |b|
-// <= p (ts_kernels.cl's m2l restated as a contraction over the pair's Dc
-// tensor).  Organised for throughput:
-//  * warps 0 and 1 (warp 0 alone for one-pair stages) are producers: for
-//    the next stage's source nodes (one each) they compute rho, f_n,
-//    (s_o/rho)^n / rho and Dc level by level, and scatter Dc into a dense
-//    cube, so that Dc_(a+b) = cube[lin(a) + lin(b)] is one indexed load;
-//    every thread copies its share of the next stage's moments into the
-//    second row buffers with cp.async while the current stage is
-//    contracted (the recurrence is latency-bound: one producer warp per
-//    pair keeps it off the critical path);
-//  * each contraction lane (192 with two-pair stages, 224 with one-pair
-//    stages) owns a fixed tuple of NB consecutive
-//    local terms b (all channels, accumulated in registers across the whole
-//    list) and a contiguous chunk of source terms a, the same chunk for the
-//    tuples that share it, so lanes of a warp mostly read the same source
-//    row (shared-memory broadcasts); pairs with |a| + |b| > p are masked;
-//  * at the end the lanes' partial sums go through shared memory in rounds
-//    and each b sums its chunks in a fixed lane order and scales by 1 / b!.
-// The plan (tuples, chunk length, lane tables) depends only on p and NB.
-constexpr int M2L3_THREADS = 256;
-// producer warps: one per pair of a two-pair stage, one for a one-pair stage
-// (at the large orders that need one-pair stages the contraction dominates)
-__host__ __device__ constexpr int m2l3_nprod(int B) { return B == 2 ? 2 : 1; }
-__host__ __device__ constexpr int m2l3_lanes(int B) { return M2L3_THREADS - 32 * m2l3_nprod(B); }
-constexpr int M2L3_LANES = M2L3_THREADS - 32;  // table capacity (the most lanes)
-constexpr int FMM_NTMAX = (FMM_MAXP + 1) * (FMM_MAXP + 2) * (FMM_MAXP + 3) / 6;
-constexpr int M2L3_PLAN_TAG = 0x4d324c33;  // "M2L3": the plan below is complete
-struct M2LPlan3 {
-    int tag;  // M2L3_PLAN_TAG once built (written last)
-    int p, nb, lanes, L, n_lanes, n_k;
-    int lane_k[M2L3_LANES];    // tuple of the lane (b = k NB + j), -1 for none
-    int lane_a0[M2L3_LANES];   // first source term (graded) and chunk length
-    int lane_cnt[M2L3_LANES];
-    int warp_steps[M2L3_LANES / 32];
-    int kstart[FMM_NTMAX + 1];  // lanes of tuple k: klane[kstart[k] .. kstart[k + 1])
-    int klane[M2L3_LANES];
-    int ainfo[FMM_NTMAX];      // lin(a) | |a| << 16
-    // Dc recurrence per graded c (level n): the graded indices of c - e_0,
-    // c - e_1, c - e_2 and lin(c); of c - 2 e_0, c - 2 e_1, c - 2 e_2 and 0;
-    // then as float bits cA c_d (3) and 0, cB c_d (c_d - 1) (3) and 0, with
-    // cA = -(2n - 1) / n, cB = -(n - 1) / n (absent neighbours: index 0,
-    // coefficient 0)
-    alignas(16) int rec[FMM_NTMAX][16];
+struct alignas(16) M2LTerm {  // recurrence of one kept term (fields: position in the cube, order)
+    int lin, n;
+    R k0, k1, k2, e0, e1;
 };
 
-// Cube index of a multi-index: lin(c) = c0 S0 + c1 S1 + c2, additive and
-// injective on |c| <= p (S1 > p, S0 > p S1 + p); the strides are padded past
-// the minimum so that the lanes of a warp, reading Dh[lin(a) + lin(b)] for
-// their different b, spread over the shared-memory banks (p = 8: 10 and 91
-// instead of 9 and 81 cut a warp step's wavefronts from ~30 to ~24).
-__host__ __device__ inline int cube_s1(int p) { return p + 2; }
-__host__ __device__ inline int cube_s0(int p) { return p * cube_s1(p) + p + 3; }
-__host__ __device__ inline int cube_lin(int p, int a0, int a1, int a2) {
-    return a0 * cube_s0(p) + a1 * cube_s1(p) + a2;
-}
-// cube entries read: lin(a) + lin(b) for |a|, |b| <= p (masked pairs included)
-__host__ __device__ inline int cube_size(int p) {
-    return 2 * p * (cube_s0(p) + cube_s1(p) + 1) + 1;
-}
-
-// Builds the plan; returns 0, or 1 when the tuples do not fit the lanes.
-// Tuples k = 0 .. ceil(NT / nb) - 1 take the b's k nb .. k nb + nb - 1; tuple
-// k's source range is [0, A_k), A_k = n_terms(p - |k nb|) (its lowest b), cut
-// into chunks of L terms, L the smallest length whose chunks fit the lanes;
-// lanes are dealt chunk-major (every tuple's first chunk, then every second
-// chunk, ...), so the lanes of one chunk index are adjacent.
-__host__ __device__ inline int m2l3_make_plan(int p, int nb, int lanes, M2LPlan3* plan) {
-    const int NT = n_terms(p);
-    const int nk = (NT + nb - 1) / nb;
-    if (lanes < 32 || lanes > M2L3_LANES || lanes % 32) return 1;
-    plan->p = p;
-    plan->nb = nb;
-    plan->lanes = lanes;
-    plan->n_k = nk;
-    auto A = [&](int k) {
-        int b0, b1, b2;
-        decode(k * nb, b0, b1, b2);
-        return n_terms(p - (b0 + b1 + b2));
-    };
-    int total = 0;
-    for (int k = 0; k < nk; k++) total += A(k);
-    int L = (total + lanes - 1) / lanes;
-    if (L < 1) L = 1;
-    for (;; L++) {
-        int cnt = 0;
-        for (int k = 0; k < nk; k++) cnt += (A(k) + L - 1) / L;
-        if (cnt <= lanes) break;
-        if (L > NT) return 1;
-    }
-    plan->L = L;
-    int lane = 0;
-    for (int c = 0;; c++) {
-        bool any = false;
-        for (int k = 0; k < nk; k++) {
-            const int ak = A(k);
-            if (c * L >= ak) continue;
-            plan->lane_k[lane] = k;
-            plan->lane_a0[lane] = c * L;
-            plan->lane_cnt[lane] = (ak - c * L < L) ? ak - c * L : L;
-            lane++;
-            any = true;
-        }
-        if (!any) break;
-    }
-    plan->n_lanes = lane;
-    for (int l = lane; l < M2L3_LANES; l++) {
-        plan->lane_k[l] = -1;
-        plan->lane_a0[l] = 0;
-        plan->lane_cnt[l] = 0;
-    }
-    for (int w = 0; w < lanes / 32; w++) {
-        int m = 0;
-        for (int l = 32 * w; l < 32 * w + 32; l++) m = plan->lane_cnt[l] > m ? plan->lane_cnt[l] : m;
-        plan->warp_steps[w] = m;
-    }
-    int pos = 0;
-    for (int k = 0; k < nk; k++) {
-        plan->kstart[k] = pos;
-        for (int l = 0; l < lane; l++)
-            if (plan->lane_k[l] == k) plan->klane[pos++] = l;
-    }
-    plan->kstart[nk] = pos;
-    for (int g = 0; g < NT; g++) {
-        int a0, a1, a2;
-        decode(g, a0, a1, a2);
-        plan->ainfo[g] = cube_lin(p, a0, a1, a2) | ((a0 + a1 + a2) << 16);
-        const int n = a0 + a1 + a2;
-        const float cA = n > 0 ? -(float)(2 * n - 1) / (float)n : 0.f;
-        const float cB = n > 0 ? -(float)(n - 1) / (float)n : 0.f;
-        int* r = plan->rec[g];
-        r[0] = a0 > 0 ? midx(a0 - 1, a1, a2) : 0;
-        r[1] = a1 > 0 ? midx(a0, a1 - 1, a2) : 0;
-        r[2] = a2 > 0 ? midx(a0, a1, a2 - 1) : 0;
-        r[3] = cube_lin(p, a0, a1, a2);
-        r[4] = a0 > 1 ? midx(a0 - 2, a1, a2) : 0;
-        r[5] = a1 > 1 ? midx(a0, a1 - 2, a2) : 0;
-        r[6] = a2 > 1 ? midx(a0, a1, a2 - 2) : 0;
-        r[7] = 0;
-        const float cf[8] = {cA * (float)a0, cA * (float)a1, cA * (float)a2, 0.f,
-                             cB * (float)(a0 * (a0 - 1)), cB * (float)(a1 * (a1 - 1)),
-                             cB * (float)(a2 * (a2 - 1)), 0.f};
-        for (int t = 0; t < 8; t++) {
-            float f = cf[t];
-            int bits;
-            memcpy(&bits, &f, sizeof(int));
-            r[8 + t] = bits;
-        }
-    }
-    return 0;
-}
-
-// Builds the plan in the operator's workspace once: a plan tagged complete
-// for this (p, nb) -- it depends on nothing else -- is reused.
-__global__ void __launch_bounds__(32) fmm_m2l3_plan(int p, int nb, int lanes,
-                                                    M2LPlan3* __restrict__ plan, int* err) {
-    if (threadIdx.x != 0) return;
-    volatile int* tag = &plan->tag;
-    if (*tag == M2L3_PLAN_TAG && plan->p == p && plan->nb == nb && plan->lanes == lanes) return;
-    *tag = 0;
-    if (m2l3_make_plan(p, nb, lanes, plan)) {
-        *err = 1;
-        return;
-    }
-    __threadfence();
-    *tag = M2L3_PLAN_TAG;
-}
-
-// Terms b per lane (FP32): the accumulators (NB x NCH values) stay near 64
-// registers.
-template <int K>
-struct M2L3Cfg {
-    static constexpr int NCH = Chan<K>::NCH;
-    static constexpr int NB = K == kRH ? 3 : 64 / NCH;
+struct M2LShape {
+    int NT, S1, S2, DS, rowsz, warp_reals;
 };
-
-// Shared-memory layout (floats), B pairs per pipeline stage: row buffers
-// 2 B x NT x NCHP, cubes 2 B x CUBEP (CUBEP >= cube_size(p), so lin(a) +
-// lin(b) needs no clamp; these two regions double as the reduction area, at least
-// 32 lanes' slots), graded Dc scratch B x NTP, 2 B x 40 scalars, 4 x
-// M2L3_CAP pair geometry, then ainfo (NTP ints), M2L3_CAP source node ids and
-// the recurrence table (NT x 16 ints).
-constexpr int M2L3_CAP = 512;  // pairs whose source node and geometry are staged
-struct M2L3Smem {
-    int NT, NTP, CUBEP, area, dg, sb, pg, ai, total_bytes;
-};
-template <int K>
-__host__ __device__ inline M2L3Smem m2l3_smem(int p, int B) {
-    using C = Chan<K>;
-    M2L3Smem m;
-    m.NT = n_terms(p);
-    m.NTP = (m.NT + 3) / 4 * 4;
-    m.CUBEP = (cube_size(p) + 3) / 4 * 4;
-    const int need = 2 * B * (m.NT * C::NCHP + m.CUBEP);
-    const int slots32 = 32 * M2L3Cfg<K>::NB * C::NCH;
-    m.area = need > slots32 ? need : (slots32 + 3) / 4 * 4;
-    m.dg = m.area;
-    m.sb = m.dg + B * m.NTP;
-    m.pg = m.sb + 2 * B * 40;
-    m.ai = m.pg + 4 * M2L3_CAP;
-    m.total_bytes = (int)(sizeof(float) * m.ai + sizeof(int) * (m.NTP + M2L3_CAP) +
-                          sizeof(int) * 16 * m.NT);
-    return m;
-}
-
-template <int K, int B>
-__global__ void __launch_bounds__(M2L3_THREADS, 2)
-fmm_m2l3(int p, const int64_t* __restrict__ obs_nodes, int64_t n_obs_nodes,
-         const int64_t* __restrict__ starts, const int64_t* __restrict__ srcs,
-         const float* __restrict__ ocent, const float* __restrict__ orad,
-         const float* __restrict__ scent, const float* __restrict__ srad,
-         const float* __restrict__ mom, const M2LPlan3* __restrict__ plan,
-         float* __restrict__ loc) {
-    using C = Chan<K>;
-    constexpr int NB = M2L3Cfg<K>::NB;
-    constexpr int NCH = C::NCH;
-    constexpr int NP = (NCH + 1) / 2;  // channel pairs (f32x2)
-    constexpr int NPROD = m2l3_nprod(B), LANES = m2l3_lanes(B);
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const M2L3Smem sm = m2l3_smem<K>(p, B);
-    const int NT = sm.NT;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int64_t oi = blockIdx.x;
-    if (oi >= n_obs_nodes) return;
-    const int rowsz = NT * C::NCHP;
-    float* base = reinterpret_cast<float*>(smem_raw);
-    float* Nb = base;                     // 2 B x NT x NCHP source rows
-    float* Cb = base + 2 * B * rowsz;     // 2 B x CUBEP scaled Dc cubes
-    float* Dg = base + sm.dg;             // B x NTP graded Dc (producer scratch)
-    float* Sb = base + sm.sb;             // 2 B x 40: (-s_s/s_o)^n [0, 16), R0 [32, 35)
-    float* pgeo = base + sm.pg;           // first M2L3_CAP pairs: source center and radius
-    int* ainfo = reinterpret_cast<int*>(base + sm.ai);
-    int* psrc = ainfo + sm.NTP;           // first M2L3_CAP pairs: source node
-    int* rtab = psrc + M2L3_CAP;          // recurrence table
-    for (int g = tid; g < NT; g += M2L3_THREADS) ainfo[g] = plan->ainfo[g];
-    for (int e = tid; e < NT * 4; e += M2L3_THREADS)
-        reinterpret_cast<int4*>(rtab)[e] = reinterpret_cast<const int4*>(plan->rec)[e];
-
-    const int64_t node = obs_nodes[oi];
-    const float co[3] = {ocent[3 * node], ocent[3 * node + 1], ocent[3 * node + 2]};
-    const float so = orad[node];
-    const float inv_so = 1.f / so;  // node radii are positive
-    const int64_t l0 = starts[oi], l1 = starts[oi + 1];
-    const int64_t npair = l1 - l0;
-    // the list's source nodes and geometry, staged once (the pipeline below
-    // would otherwise wait on dependent global loads every pair)
-    for (int64_t i = tid; i < npair && i < M2L3_CAP; i += M2L3_THREADS) {
-        const int64_t sn = srcs[l0 + i];
-        psrc[i] = (int)sn;
-        pgeo[4 * i] = scent[3 * sn];
-        pgeo[4 * i + 1] = scent[3 * sn + 1];
-        pgeo[4 * i + 2] = scent[3 * sn + 2];
-        pgeo[4 * i + 3] = srad[sn];
-    }
-    __syncthreads();
-
-    // pairs [k0, k0 + B) of the list (those below npair) into stage st
-    auto issue_copy = [&](int64_t k0, int st) {
-#pragma unroll
-        for (int u = 0; u < B; u++) {
-            const int64_t k = k0 + u;
-            if (k >= npair) break;
-            const int64_t sn = k < M2L3_CAP ? (int64_t)psrc[k] : srcs[l0 + k];
-            const float* src = mom + sn * (int64_t)rowsz;
-            float* dst = Nb + (st * B + u) * rowsz;
-            for (int e = tid; e < rowsz / 4; e += M2L3_THREADS) cp_async16(dst + e * 4, src + e * 4);
-        }
-        cp_async_commit();
-    };
-    // coef(a, b) = f_|a| (s_o/rho)^|b| / rho Dc_(a+b) = S_|a| Dh_(a+b) with
-    // Dh_c = Dc_c (s_o/rho)^|c| / rho (the cube) and S_n = (-s_s/s_o)^n; the
-    // B pairs' recurrences run interleaved (independent chains)
-    // producer warp w handles the stage's pairs u0 .. u0 + PB - 1
-    constexpr int PB = B / NPROD;
-    auto produce = [&](int64_t k0, int st) {  // warps 0 .. NPROD - 1
-        const int u0 = warp * PB;
-        float Rh[B][3], q[B], pwn[B];
-        bool on[B];
-#pragma unroll
-        for (int uu = 0; uu < PB; uu++) {
-            const int u = u0 + uu;
-            const int64_t k = k0 + u;
-            on[u] = k < npair;
-            float cs[3] = {co[0] + 1.f, co[1], co[2]}, rs = 0.f;  // any distinct point if off
-            if (on[u] && k < M2L3_CAP) {
-                const float* g = pgeo + 4 * k;
-                cs[0] = g[0]; cs[1] = g[1]; cs[2] = g[2]; rs = g[3];
-            } else if (on[u]) {
-                const int64_t sn = srcs[l0 + k];
-                cs[0] = scent[3 * sn]; cs[1] = scent[3 * sn + 1]; cs[2] = scent[3 * sn + 2];
-                rs = srad[sn];
-            }
-            const float R0[3] = {co[0] - cs[0], co[1] - cs[1], co[2] - cs[2]};
-            const float rho = sqrtf(R0[0] * R0[0] + R0[1] * R0[1] + R0[2] * R0[2]);
-            const float inv_rho = 1.f / rho;
-            Rh[u][0] = R0[0] * inv_rho; Rh[u][1] = R0[1] * inv_rho; Rh[u][2] = R0[2] * inv_rho;
-            q[u] = so * inv_rho;  // pw_n = q^n / rho
-            pwn[u] = inv_rho;
-            float* S = Sb + (st * B + u) * 40;
-            if (lane <= p) S[lane] = ipow(-rs * inv_so, lane);
-            if (lane < 3) S[32 + lane] = R0[lane];
-            if (lane == 0) {
-                Dg[u * sm.NTP] = 1.f;
-                Cb[(st * B + u) * sm.CUBEP] = inv_rho;
-            }
-        }
-        __syncwarp();
-        // level n from levels n - 1 and n - 2; a lane takes entries lane and
-        // lane + 32 of the level for each pair, loads first so the chains overlap
-        for (int n = 1; n <= p; n++) {
-            const int lsz = (n + 1) * (n + 2) / 2, b0 = n_terms(n - 1);
-            float v[B][2];
-            int dst[2], cl[2];
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int w = lane + 32 * h;
-                dst[h] = -1;
-                cl[h] = 0;
-                if (w >= lsz) continue;
-                const int4* rt = reinterpret_cast<const int4*>(rtab + 16 * (b0 + w));
-                const int4 i0 = rt[0], i1 = rt[1], f0 = rt[2], f1 = rt[3];
-#pragma unroll
-                for (int uu = 0; uu < PB; uu++) {
-                    const int u = u0 + uu;
-                    const float* D = Dg + u * sm.NTP;
-                    v[u][h] = __int_as_float(f0.x) * Rh[u][0] * D[i0.x] +
-                              __int_as_float(f0.y) * Rh[u][1] * D[i0.y] +
-                              __int_as_float(f0.z) * Rh[u][2] * D[i0.z] +
-                              __int_as_float(f1.x) * D[i1.x] + __int_as_float(f1.y) * D[i1.y] +
-                              __int_as_float(f1.z) * D[i1.z];
-                }
-                dst[h] = b0 + w;
-                cl[h] = i0.w;
-            }
-#pragma unroll
-            for (int uu = 0; uu < PB; uu++) {
-                const int u = u0 + uu;
-                pwn[u] *= q[u];
-#pragma unroll
-                for (int h = 0; h < 2; h++)
-                    if (dst[h] >= 0) {
-                        Dg[u * sm.NTP + dst[h]] = v[u][h];
-                        Cb[(st * B + u) * sm.CUBEP + cl[h]] = v[u][h] * pwn[u];
-                    }
-            }
-            __syncwarp();
-        }
-    };
-
-    // this lane's tuple and source chunk
-    const int ct = tid - 32 * NPROD;
-    int kk = -1, a_first = 0, cnt = 0, wsteps = 0;
-    int blin[NB], thr[NB];
-    if (warp >= NPROD) {
-        kk = plan->lane_k[ct];
-        a_first = plan->lane_a0[ct];
-        cnt = plan->lane_cnt[ct];
-        wsteps = plan->warp_steps[warp - NPROD];
-    }
-#pragma unroll
-    for (int j = 0; j < NB; j++) {
-        const int b = kk * NB + j;
-        if (kk >= 0 && b < NT) {
-            int b0, b1, b2;
-            decode(b, b0, b1, b2);
-            blin[j] = cube_lin(p, b0, b1, b2);
-            thr[j] = p - (b0 + b1 + b2);  // a valid while |a| <= thr
-        } else {
-            blin[j] = 0;
-            thr[j] = -1;  // never valid
-        }
-    }
-    f2_t acc[NB][NP];
-#pragma unroll
-    for (int j = 0; j < NB; j++)
-#pragma unroll
-        for (int i = 0; i < NP; i++) acc[j][i] = 0ull;
-
-    const int64_t nst = (npair + B - 1) / B;  // pipeline stages of B pairs
-    if (nst > 0) {
-        issue_copy(0, 0);
-        if (warp < NPROD) produce(0, 0);
-    }
-    for (int64_t st = 0; st < nst; st++) {
-        const int buf = (int)(st & 1);
-        cp_async_wait_all();
-        __syncthreads();  // stage st's rows, cubes and scalars are complete; st - 1 is done
-        if (st + 1 < nst) {
-            issue_copy((st + 1) * B, buf ^ 1);
-            if (warp < NPROD) produce((st + 1) * B, buf ^ 1);
-        }
-        if (warp < NPROD) continue;
-#pragma unroll 1
-        for (int u = 0; u < B; u++) {
-            if (st * B + u >= npair) break;
-            const float* S = Sb + (buf * B + u) * 40;
-            const float* Dc = Cb + (buf * B + u) * sm.CUBEP;
-            const float* N = Nb + (buf * B + u) * rowsz;
-            const float R0[3] = {S[32], S[33], S[34]};
-#pragma unroll 1
-            for (int s = 0; s < wsteps; s++) {
-                const bool on = s < cnt;
-                const int a = a_first + (on ? s : 0);
-                const int e = ainfo[a];
-                const int alin = e & 0xffff, la = e >> 16;
-                const float fa = on ? S[la] : 0.f;
-                f2_t cf[NB];
-#pragma unroll
-                for (int j = 0; j < NB; j++) {
-                    const float c = la <= thr[j] ? Dc[alin + blin[j]] * fa : 0.f;
-                    cf[j] = pk(c, c);
-                }
-                const float4* row = reinterpret_cast<const float4*>(N + a * C::NCHP);
-                float v[C::NCHP];
-#pragma unroll
-                for (int k4 = 0; k4 < C::NCHP / 4; k4++) {
-                    const float4 q4 = row[k4];
-                    v[4 * k4] = q4.x; v[4 * k4 + 1] = q4.y; v[4 * k4 + 2] = q4.z;
-                    v[4 * k4 + 3] = q4.w;
-                }
-#pragma unroll
-                for (int d = 0; d < 3; d++)
-#pragma unroll
-                    for (int j = 0; j < C::J; j++)
-                        v[C::CH_Y + d * C::J + j] -= R0[d] * v[C::CH_M + j];
-#pragma unroll
-                for (int i = 0; i < NP; i++) {
-                    const f2_t vi = pk(v[2 * i], v[2 * i + 1]);
-#pragma unroll
-                    for (int j = 0; j < NB; j++) acc[j][i] = fma2(cf[j], vi, acc[j][i]);
-                }
-            }
-        }
-    }
-    cp_async_wait_all();
-    __syncthreads();
-
-    // reduction in rounds through the row/cube area
-    constexpr int PER = NB * NCH;
-    const int lpr = sm.area / PER;
-    float* Lg = loc + node * (int64_t)rowsz;
-    for (int lo = 0; lo < LANES; lo += lpr) {
-        const int hi = lo + lpr < LANES ? lo + lpr : LANES;
-        if (warp >= NPROD && ct >= lo && ct < hi) {
-            float* sl = base + (ct - lo) * PER;
-#pragma unroll
-            for (int j = 0; j < NB; j++)
-#pragma unroll
-                for (int i = 0; i < NP; i++) {
-                    float x, y;
-                    upk(acc[j][i], x, y);
-                    sl[j * NCH + 2 * i] = x;
-                    if (2 * i + 1 < NCH) sl[j * NCH + 2 * i + 1] = y;
-                }
-        }
-        __syncthreads();
-        for (int b = tid; b < NT; b += M2L3_THREADS) {
-            const int k = b / NB, j = b - k * NB;
-            float sum[NCH];
-#pragma unroll
-            for (int c = 0; c < NCH; c++) sum[c] = 0.f;
-            for (int i = plan->kstart[k]; i < plan->kstart[k + 1]; i++) {
-                const int l = plan->klane[i];
-                if (l < lo || l >= hi) continue;
-                const float* sl = base + (l - lo) * PER + j * NCH;
-#pragma unroll
-                for (int c = 0; c < NCH; c++) sum[c] += sl[c];
-            }
-            int b0, b1, b2;
-            decode(b, b0, b1, b2);
-            const float inv = 1.f / mfact<float>(b0, b1, b2);
-            float* out = Lg + b * C::NCHP;
-            if (lo == 0) {
-#pragma unroll
-                for (int c = 0; c < C::NCHP; c++) out[c] = c < NCH ? sum[c] * inv : 0.f;
-            } else {
-#pragma unroll
-                for (int c = 0; c < NCH; c++) out[c] += sum[c] * inv;
-            }
-        }
-        __syncthreads();
-    }
-}
-
-
-// ---- M2L, item form (FP64, and FP32 when the lane plan does not fit) -------
-// The same L_b as fmm_m2l3 above.  Warp 0 is the producer:
-// for source node k + 1 it computes rho, f_n, (s_o/rho)^n / rho and Dc level
-// by level into the second of two shared-memory buffers, while the other
-// seven warps contract source node k; every thread copies its share of node
-// k + 1's moments into the second moment buffer with cp.async.  A
-// contraction thread owns up to M2L2_MAXIT work items (local term b, a range
-// of source terms a in graded order), the same items for every pair; per
-// pair an item's sum (coef = (s_o/rho)^|b| / rho * f_|a| * Dc_(a+b) times
-// the source row with the Yl correction folded in, Y_dj - R0_d m_j) is
-// accumulated in registers and added to the item's slot in shared memory,
-// which only that thread touches.  At the end the slots of each b are summed
-// in a fixed order and scaled by 1 / b!.  One barrier per pair; registers
-// stay under 80 so that three CTAs share an SM.
-constexpr int M2L2_THREADS = 256;
-constexpr int M2L2_TC = M2L2_THREADS - 32;  // contraction threads
-constexpr int M2L2_MAXIT = 3;
-constexpr int M2L2_MAXITEMS = M2L2_TC * M2L2_MAXIT;
-struct M2LPlan2 {
-    int n_items;
-    int item[M2L2_MAXITEMS][8];   // b, g0, g1, a0, a2, |a| at g0, b0, b2
-    int bstart[FMM_NTMAX + 1];    // items of term b: [bstart[b], bstart[b + 1])
-    int tcnt[M2L2_TC];
-    int titem[M2L2_TC][M2L2_MAXIT];
-    int rec[FMM_NTMAX][8];        // Dc recurrence: a0, a1, a2 and the 5 used indices
-};
-
-// The plan: items cut term b's n_terms(p - |b|) source terms into near-equal
-// chunks of at most CH = ceil(total / M2L2_TC) terms; the items, largest
-// first, are dealt to the contraction threads in snake order.  One thread,
-// written to the workspace each call.
-__global__ void __launch_bounds__(32) fmm_m2l2_plan(int p, M2LPlan2* __restrict__ plan, int* err) {
-    if (threadIdx.x != 0) return;
-    const int NT = n_terms(p);
-    const int total = n_terms6(p);
-    const int CH = (total + M2L2_TC - 1) / M2L2_TC;
-    int n = 0;
-    for (int b = 0; b < NT; b++) {
-        int b0, b1, b2;
-        decode(b, b0, b1, b2);
-        const int t = n_terms(p - (b0 + b1 + b2));
-        const int nch = (t + CH - 1) / CH;
-        plan->bstart[b] = n;
-        for (int c = 0; c < nch; c++) {
-            if (n >= M2L2_MAXITEMS) {
-                *err = 1;
-                return;
-            }
-            const int g0 = (int)((int64_t)t * c / nch), g1 = (int)((int64_t)t * (c + 1) / nch);
-            int a0, a1, a2;
-            decode(g0, a0, a1, a2);
-            int* it = plan->item[n];
-            it[0] = b; it[1] = g0; it[2] = g1; it[3] = a0; it[4] = a2; it[5] = a0 + a1 + a2;
-            it[6] = b0; it[7] = b2;
-            n++;
-        }
-    }
-    plan->bstart[NT] = n;
-    plan->n_items = n;
-    // deal items by size, largest first (counting sort on sizes 1..CH), snake order
-    for (int t = 0; t < M2L2_TC; t++) plan->tcnt[t] = 0;
-    int dealt = 0;
-    for (int sz = CH; sz >= 1; sz--)
-        for (int i = 0; i < n; i++) {
-            if (plan->item[i][2] - plan->item[i][1] != sz) continue;
-            const int round = dealt / M2L2_TC, pos = dealt % M2L2_TC;
-            const int th = (round & 1) ? M2L2_TC - 1 - pos : pos;
-            if (plan->tcnt[th] >= M2L2_MAXIT) {
-                *err = 1;
-                return;
-            }
-            plan->titem[th][plan->tcnt[th]++] = i;
-            dealt++;
-        }
-    // the Dc recurrence table
-    for (int g = 0; g < NT; g++) {
-        int a0, a1, a2;
-        decode(g, a0, a1, a2);
-        int* r = plan->rec[g];
-        r[0] = a0; r[1] = a1; r[2] = a2;
-        r[3] = a0 > 0 ? midx(a0 - 1, a1, a2) : 0;
-        r[4] = a1 > 0 ? midx(a0, a1 - 1, a2) : 0;
-        r[5] = a2 > 0 ? midx(a0, a1, a2 - 1) : 0;
-        r[6] = a0 > 1 ? midx(a0 - 2, a1, a2) : 0;
-        r[7] = 0;  // the a1 - 2 and a2 - 2 indices are recomputed (rare)
-    }
-}
-
-// Number of plan items for order p (host mirror of fmm_m2l2_plan's cut).
-inline int m2l2_items(int p) {
-    const int total = n_terms6(p), CH = (total + M2L2_TC - 1) / M2L2_TC;
-    int n = 0;
-    for (int m = 0; m <= p; m++) {
-        const int t = n_terms(p - m), cnt = (m + 1) * (m + 2) / 2;
-        n += cnt * ((t + CH - 1) / CH);
-    }
-    return n;
-}
-
+// pairs per batch: 8 in FP32, 4 in FP64 (shared memory)
+template <typename R>
+constexpr int m2l_pb() { return sizeof(R) == 4 ? 8 : 4; }
 
 template <typename R, int K>
-__global__ void __launch_bounds__(M2L2_THREADS, 3)
-fmm_m2l2(int p, const int64_t* __restrict__ obs_nodes, int64_t n_obs_nodes,
-         const int64_t* __restrict__ starts, const int64_t* __restrict__ srcs,
-         const R* __restrict__ ocent, const R* __restrict__ orad, const R* __restrict__ scent,
-         const R* __restrict__ srad, const R* __restrict__ mom, const M2LPlan2* __restrict__ plan,
-         R* __restrict__ loc) {
-    using C = Chan<K>;
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int NT = n_terms(p);
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int64_t oi = blockIdx.x;
-    if (oi >= n_obs_nodes) return;
-    const int rowsz = NT * C::NCHP;
-    R* Nb = reinterpret_cast<R*>(smem_raw);  // 2 x NT x NCHP moments
-    R* Db = Nb + 2 * rowsz;                  // 2 x NT Dc
-    R* Sb = Db + 2 * ((NT + 3) / 4 * 4);     // 2 x 40: f_n [0, 16), pw_n [16, 32), R0 [32, 35)
-    R* slots = Sb + 80;                      // n_items x NCHP item sums
-    const int64_t node = obs_nodes[oi];
-    const R co[3] = {ocent[3 * node], ocent[3 * node + 1], ocent[3 * node + 2]};
-    const R so = orad[node];
-    const int64_t l0 = starts[oi], l1 = starts[oi + 1];
-    const int64_t npair = l1 - l0;
-
-    auto issue_copy = [&](int64_t l, int buf) {
-        const R* src = mom + srcs[l] * (int64_t)rowsz;
-        R* dst = Nb + buf * rowsz;
-        constexpr int PER = 16 / sizeof(R);
-        for (int k = tid; k < rowsz / PER; k += M2L2_THREADS)
-            cp_async16(dst + k * PER, src + k * PER);
-        cp_async_commit();
-    };
-    auto produce = [&](int64_t l, int buf) {  // warp 0
-        const int64_t sn = srcs[l];
-        const R R0[3] = {co[0] - scent[3 * sn], co[1] - scent[3 * sn + 1],
-                         co[2] - scent[3 * sn + 2]};
-        const R rho = sqrt(R0[0] * R0[0] + R0[1] * R0[1] + R0[2] * R0[2]);
-        const R inv_rho = R(1) / rho;
-        const R Rh[3] = {R0[0] * inv_rho, R0[1] * inv_rho, R0[2] * inv_rho};
-        R* S = Sb + buf * 40;
-        R* D = Db + buf * ((NT + 3) / 4 * 4);
-        if (lane <= p) {
-            S[lane] = ((lane & 1) ? R(-1) : R(1)) * ipow(srad[sn] * inv_rho, lane);
-            S[16 + lane] = ipow(so * inv_rho, lane) * inv_rho;
-        }
-        if (lane < 3) S[32 + lane] = R0[lane];
-        if (lane == 0) D[0] = 1;
-        __syncwarp();
-        for (int n = 1; n <= p; n++) {
-            const int lsz = (n + 1) * (n + 2) / 2, base = n_terms(n - 1);
-            const R cA = -(R)(2 * n - 1) / (R)n, cB = -(R)(n - 1) / (R)n;
-            for (int w = lane; w < lsz; w += 32) {
-                const int* rr = plan->rec[base + w];
-                const int a0 = rr[0], a1 = rr[1], a2 = rr[2];
-                R s1 = 0, s2 = 0;
-                if (a0 > 0) s1 += Rh[0] * (R)a0 * D[rr[3]];
-                if (a1 > 0) s1 += Rh[1] * (R)a1 * D[rr[4]];
-                if (a2 > 0) s1 += Rh[2] * (R)a2 * D[rr[5]];
-                if (a0 > 1) s2 += (R)(a0 * (a0 - 1)) * D[rr[6]];
-                if (a1 > 1) s2 += (R)(a1 * (a1 - 1)) * D[midx(a0, a1 - 2, a2)];
-                if (a2 > 1) s2 += (R)(a2 * (a2 - 1)) * D[midx(a0, a1, a2 - 2)];
-                D[base + w] = cA * s1 + cB * s2;
-            }
-            __syncwarp();
-        }
-    };
-
-    // this thread's work items
-    const int ct = tid - 32;
-    int my_n = 0;
-    int itid[M2L2_MAXIT], itg0[M2L2_MAXIT], itg1[M2L2_MAXIT], ita0[M2L2_MAXIT],
-        ita2[M2L2_MAXIT], itna[M2L2_MAXIT], itb0[M2L2_MAXIT], itb2[M2L2_MAXIT],
-        itnb[M2L2_MAXIT];
-    if (warp > 0) {
-        my_n = plan->tcnt[ct];
-#pragma unroll
-        for (int i = 0; i < M2L2_MAXIT; i++) {
-            itid[i] = i < my_n ? plan->titem[ct][i] : 0;
-            const int* it = plan->item[itid[i]];
-            itg0[i] = it[1]; itg1[i] = it[2]; ita0[i] = it[3];
-            ita2[i] = it[4]; itna[i] = it[5]; itb0[i] = it[6]; itb2[i] = it[7];
-            int b0, b1, b2;
-            decode(it[0], b0, b1, b2);
-            itnb[i] = b0 + b1 + b2;
-        }
-    }
-    const int n_items = plan->n_items;
-    for (int e = tid; e < n_items * C::NCHP; e += M2L2_THREADS) slots[e] = 0;
-
-    if (npair > 0) {
-        issue_copy(l0, 0);
-        if (warp == 0) produce(l0, 0);
-    }
-    for (int64_t k = 0; k < npair; k++) {
-        const int buf = (int)(k & 1);
-        cp_async_wait_all();
-        __syncthreads();  // pair k's moments and Dc are complete; pair k - 1 is done
-        if (k + 1 < npair) {
-            issue_copy(l0 + k + 1, buf ^ 1);
-            if (warp == 0) produce(l0 + k + 1, buf ^ 1);
-        }
-        if (warp == 0) continue;
-        const R* S = Sb + buf * 40;
-        const R* D = Db + buf * ((NT + 3) / 4 * 4);
-        const R* N = Nb + buf * rowsz;
-        const R R0[3] = {S[32], S[33], S[34]};
-#pragma unroll 1
-        for (int i = 0; i < M2L2_MAXIT; i++) {
-            if (i >= my_n) break;
-            R acc[C::NCH];
-#pragma unroll
-            for (int c = 0; c < C::NCH; c++) acc[c] = 0;
-            const R sb = S[16 + itnb[i]];
-            const int b0 = itb0[i], b2 = itb2[i];
-            int a0 = ita0[i], a2 = ita2[i], na = itna[i];
-            int nn = na + itnb[i];
-            int rowbase = n_terms(nn - 1) + (nn - a0 - b0) * (nn - a0 - b0 + 1) / 2 + b2;
-            R f = sb * S[na];
-            for (int g = itg0[i]; g < itg1[i]; g++) {
-                const R coef = f * D[rowbase + a2];
-                const R* row = N + g * C::NCHP;
-                R v[C::NCHP];
-                if (sizeof(R) == 4) {
-#pragma unroll
-                    for (int k4 = 0; k4 < C::NCHP / 4; k4++) {
-                        const float4 q = reinterpret_cast<const float4*>(row)[k4];
-                        v[4 * k4] = (R)q.x; v[4 * k4 + 1] = (R)q.y;
-                        v[4 * k4 + 2] = (R)q.z; v[4 * k4 + 3] = (R)q.w;
-                    }
-                } else {
-#pragma unroll
-                    for (int k2 = 0; k2 < C::NCHP / 2; k2++) {
-                        const double2 q = reinterpret_cast<const double2*>(row)[k2];
-                        v[2 * k2] = (R)q.x; v[2 * k2 + 1] = (R)q.y;
-                    }
-                }
-#pragma unroll
-                for (int d = 0; d < 3; d++)
-#pragma unroll
-                    for (int j = 0; j < C::J; j++)
-                        v[C::CH_Y + d * C::J + j] -= R0[d] * v[C::CH_M + j];
-#pragma unroll
-                for (int c = 0; c < C::NCH; c++) acc[c] += coef * v[c];
-                // next source term in graded order
-                a2++;
-                if (a2 > na - a0) {
-                    a2 = 0;
-                    a0--;
-                    if (a0 < 0) {
-                        na++;
-                        a0 = na;
-                        nn++;
-                        f = sb * S[na];
-                    }
-                    rowbase = n_terms(nn - 1) + (nn - a0 - b0) * (nn - a0 - b0 + 1) / 2 + b2;
-                }
-            }
-            R* sl = slots + itid[i] * C::NCHP;
-#pragma unroll
-            for (int c = 0; c < C::NCH; c++) sl[c] += acc[c];
-        }
-    }
-    cp_async_wait_all();
-    __syncthreads();
-    R* Lg = loc + node * (int64_t)rowsz;
-    for (int b = tid; b < NT; b += M2L2_THREADS) {
-        int b0, b1, b2;
-        decode(b, b0, b1, b2);
-        const R inv = R(1) / mfact<R>(b0, b1, b2);
-        R sum[C::NCH];
-#pragma unroll
-        for (int c = 0; c < C::NCH; c++) sum[c] = 0;
-        for (int it = plan->bstart[b]; it < plan->bstart[b + 1]; it++)
-#pragma unroll
-            for (int c = 0; c < C::NCH; c++) sum[c] += slots[it * C::NCHP + c];
-#pragma unroll
-        for (int c = 0; c < C::NCHP; c++) Lg[b * C::NCHP + c] = c < C::NCH ? sum[c] * inv : R(0);
-    }
+__host__ __device__ inline M2LShape m2l_shape(int p) {
+    M2LShape s;
+    s.NT = n_harm(p);
+    s.S1 = p + 2;           // odd steps between the terms of an order: few bank conflicts
+    s.S2 = (p + 2) * p + 1;
+    s.DS = (2 * s.S2 + s.S1 * (p > 2 ? p - 2 : 0) + 1) | 1;
+    s.rowsz = s.NT * Chan<K>::NCHP;
+    // rows, cubes, S (16 a pair), R0 (4 a pair)
+    s.warp_reals = (s.rowsz + m2l_pb<R>() * (s.DS + 20) + 3) / 4 * 4;
+    return s;
+}
+template <typename R, int K>
+__host__ __device__ inline size_t m2l_smem(int p) {
+    const M2LShape s = m2l_shape<R, K>(p);
+    return sizeof(M2LTerm<R>) * (size_t)((s.NT + 1) / 2 * 2) +
+           sizeof(R) * (size_t)M2L_WARPS * s.warp_reals;
 }
 
+// A lane's sums for one local term: NCH channels, packed two by two in FP32.
+template <typename R, int N>
+struct M2LAcc {
+    R a[N];
+    __device__ __forceinline__ void zero() {
+#pragma unroll
+        for (int k = 0; k < N; k++) a[k] = 0;
+    }
+    __device__ __forceinline__ void get(R (&o)[N]) const {
+#pragma unroll
+        for (int k = 0; k < N; k++) o[k] = a[k];
+    }
+};
+template <int N>
+struct M2LAcc<float, N> {
+    f2_t a[(N + 1) / 2];
+    __device__ __forceinline__ void zero() {
+#pragma unroll
+        for (int k = 0; k < (N + 1) / 2; k++) a[k] = 0ull;
+    }
+    __device__ __forceinline__ void get(float (&o)[N]) const {
+#pragma unroll
+        for (int k = 0; k < (N + 1) / 2; k++) {
+            float x, y;
+            upk(a[k], x, y);
+            o[2 * k] = x;
+            if (2 * k + 1 < N) o[2 * k + 1] = y;
+        }
+    }
+};
+template <typename R, int N, int NP>
+struct M2LRow {
+    R v[NP];
+    __device__ __forceinline__ void load(const R* src) { load_row<R, NP>(v, src); }
+    __device__ __forceinline__ void add(M2LAcc<R, N>& acc, R c) const {
+#pragma unroll
+        for (int k = 0; k < N; k++) acc.a[k] += c * v[k];
+    }
+};
+template <int N, int NP>
+struct M2LRow<float, N, NP> {
+    f2_t v[NP / 2];
+    __device__ __forceinline__ void load(const float* src) {
+#pragma unroll
+        for (int k = 0; k < NP / 4; k++) {
+            const ulonglong2 u = reinterpret_cast<const ulonglong2*>(src)[k];
+            v[2 * k] = u.x;
+            v[2 * k + 1] = u.y;
+        }
+    }
+    __device__ __forceinline__ void add(M2LAcc<float, N>& acc, float c) const {
+        const f2_t c2 = pk(c, c);
+#pragma unroll
+        for (int k = 0; k < (N + 1) / 2; k++) acc.a[k] = fma2(c2, v[k], acc.a[k]);
+    }
+};
+
+// NS = ceil((p + 1)^2 / 32) or more: sums per lane for single terms a.
+template <typename R, int K, int NS>
+__global__ void __launch_bounds__(32 * M2L_WARPS, sizeof(R) == 4 && NS <= 4 ? 4 : 2)
+fmm_m2l(int p, const int64_t* __restrict__ obs_nodes, const int64_t* __restrict__ starts,
+        const int64_t* __restrict__ srcs, const R* __restrict__ ocent, const R* __restrict__ orad,
+        const R* __restrict__ scent, const R* __restrict__ srad, const R* __restrict__ mom,
+        R* __restrict__ loc) {
+    using C = Chan<K>;
+    constexpr int PB = m2l_pb<R>(), LPP = 32 / PB;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const M2LShape sh = m2l_shape<R, K>(p);
+    const int NT = sh.NT, S1 = sh.S1, S2 = sh.S2;
+    M2LTerm<R>* term = reinterpret_cast<M2LTerm<R>*>(smem_raw);
+    R* area = reinterpret_cast<R*>(term + (NT + 1) / 2 * 2);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    R* rows = area + warp * sh.warp_reals;  // NT x NCHP
+    R* Dw = rows + sh.rowsz;                // PB cubes
+    R* Sw = Dw + PB * sh.DS;                // PB x 16: S_n
+    R* Rw = Sw + PB * 16;                   // PB x 4: R0
+    for (int g = tid; g < NT; g += blockDim.x) {
+        int n, a0, a1, a2;
+        hdecode(g, n, a0, a1, a2);
+        M2LTerm<R> t;
+        t.lin = a0 + S1 * a1 + S2 * a2;
+        t.n = n;
+        const R cA = n > 0 ? -(R)(2 * n - 1) / (R)n : R(0);
+        const R cB = n > 0 ? -(R)(n - 1) / (R)n : R(0);
+        t.k0 = cA * (R)a0;
+        t.k1 = cA * (R)a1;
+        t.k2 = cA * (R)a2;
+        t.e0 = cB * (R)(a0 * (a0 - 1));
+        t.e1 = cB * (R)(a1 * (a1 - 1));
+        term[g] = t;
+    }
+    __syncthreads();
+
+    const int64_t node = obs_nodes[blockIdx.x];
+    const R co[3] = {ocent[3 * node], ocent[3 * node + 1], ocent[3 * node + 2]};
+    const R so = orad[node];
+    const int64_t l0 = starts[blockIdx.x], npair = starts[blockIdx.x + 1] - l0;
+    const int64_t kb = npair * warp / M2L_WARPS, ke = npair * (warp + 1) / M2L_WARPS;
+
+    // cube positions of this lane's terms b: 32 j + lane, lane & 15, lane & 3
+    int bl[NS + 2];
+#pragma unroll
+    for (int j = 0; j < NS + 2; j++) {
+        const int b = j < NS ? 32 * j + lane : (j == NS ? lane & 15 : lane & 3);
+        bl[j] = b < NT ? term[b].lin : 0;
+    }
+    M2LAcc<R, C::NCH> acc[NS + 2];
+#pragma unroll
+    for (int j = 0; j < NS + 2; j++) acc[j].zero();
+
+    for (int64_t k0 = kb; k0 < ke; k0 += PB) {
+        const int np = (int)min((int64_t)PB, ke - k0);
+        __syncwarp();
+        {   // Dh of the batch, LPP lanes a pair (idle pairs: any distinct point)
+            const int u = lane / LPP, h = lane % LPP;
+            const int64_t sn = u < np ? srcs[l0 + k0 + u] : -1;
+            const R r0 = sn >= 0 ? co[0] - scent[3 * sn] : R(1);
+            const R r1 = sn >= 0 ? co[1] - scent[3 * sn + 1] : R(0);
+            const R r2 = sn >= 0 ? co[2] - scent[3 * sn + 2] : R(0);
+            const R ss = sn >= 0 ? srad[sn] : R(0);
+            const R rho = sqrt(r0 * r0 + r1 * r1 + r2 * r2);
+            const R inv = R(1) / rho, q = so * inv, qq = q * q;
+            const R x0 = r0 * inv * q, x1 = r1 * inv * q, x2 = r2 * inv * q;
+            R* D = Dw + u * sh.DS;
+            for (int n = h; n <= p; n += LPP) Sw[u * 16 + n] = ipow(-ss / so, n);
+            if (h == 0) {
+                Rw[u * 4] = r0;
+                Rw[u * 4 + 1] = r1;
+                Rw[u * 4 + 2] = r2;
+                D[0] = inv;
+            }
+            __syncwarp();
+            for (int n = 1; n <= p; n++) {
+                for (int w = h; w <= 2 * n; w += LPP) {
+                    const M2LTerm<R> t = term[n * n + w];
+                    // absent neighbours: factor 0 at position 0
+                    R v = t.k0 * x0 * D[t.k0 != R(0) ? t.lin - 1 : 0] +
+                          t.k1 * x1 * D[t.k1 != R(0) ? t.lin - S1 : 0] +
+                          t.k2 * x2 * D[t.k2 != R(0) ? t.lin - S2 : 0];
+                    v += qq * (t.e0 * D[t.e0 != R(0) ? t.lin - 2 : 0] +
+                               t.e1 * D[t.e1 != R(0) ? t.lin - 2 * S1 : 0]);
+                    D[t.lin] = v;
+                }
+                __syncwarp();
+            }
+            // c_2 = 2 from c_2 = 0
+            for (int m = 0; m <= p - 2; m++)
+                for (int c1 = h; c1 <= m; c1 += LPP) {
+                    const int at = (m - c1) + S1 * c1;
+                    D[at + 2 * S2] = -D[at + 2] - D[at + 2 * S1];
+                }
+        }
+        for (int u = 0; u < np; u++) {
+            const int64_t sn = srcs[l0 + k0 + u];
+            const R* src = mom + sn * (int64_t)sh.rowsz;
+            __syncwarp();  // the batch's cubes; the last pair's rows are read
+            {
+                const R t0 = -Rw[u * 4], t1 = -Rw[u * 4 + 1], t2 = -Rw[u * 4 + 2];
+#pragma unroll 2
+                for (int g = lane; g < NT; g += 32) {
+                    R v[C::NCHP];
+                    load_row<R, C::NCHP>(v, src + g * C::NCHP);
+                    shift_z<R, K>(v, t0, t1, t2);
+                    const R f = Sw[u * 16 + term[g].n];
+#pragma unroll
+                    for (int k = 0; k < C::NCHP; k++) v[k] *= f;
+                    store_row<R, C::NCHP>(rows + g * C::NCHP, v);
+                }
+            }
+            __syncwarp();
+            const R* D = Dw + u * sh.DS;
+            M2LRow<R, C::NCH, C::NCHP> row;
+            for (int n = 0; n <= p; n++) {
+                const int nb = (p + 1 - n) * (p + 1 - n), cnt = 2 * n + 1;
+                const R* rn = rows + n * n * C::NCHP;
+                if (nb > 16) {
+                    int alin = n;
+                    for (int w = 0; w < cnt; w++) {
+                        if (w == n + 1) alin = n - 1 + S2;
+                        row.load(rn + w * C::NCHP);
+#pragma unroll
+                        for (int j = 0; j < NS; j++) {
+                            if (32 * j >= nb) break;
+                            const bool on = 32 * j + lane < nb;
+                            const R c = D[alin + (on ? bl[j] : 0)];
+                            row.add(acc[j], on ? c : R(0));
+                        }
+                        alin += S1 - 1;
+                    }
+                } else if (nb > 4) {
+                    const bool onb = (lane & 15) < nb;
+                    for (int i = 0; i < cnt; i += 2) {
+                        const int w = i + (lane >> 4);
+                        const bool on = onb && w < cnt;
+                        const int ww = w < cnt ? w : cnt - 1;
+                        const int a2 = ww > n ? 1 : 0, a1 = ww - a2 * (n + 1);
+                        row.load(rn + ww * C::NCHP);
+                        const R c = D[(n - a2 - a1) + S1 * a1 + S2 * a2 + (on ? bl[NS] : 0)];
+                        row.add(acc[NS], on ? c : R(0));
+                    }
+                } else {
+                    const bool onb = (lane & 3) < nb;
+                    for (int i = 0; i < cnt; i += 8) {
+                        const int w = i + (lane >> 2);
+                        const bool on = onb && w < cnt;
+                        const int ww = w < cnt ? w : cnt - 1;
+                        const int a2 = ww > n ? 1 : 0, a1 = ww - a2 * (n + 1);
+                        row.load(rn + ww * C::NCHP);
+                        const R c = D[(n - a2 - a1) + S1 * a1 + S2 * a2 + (on ? bl[NS + 1] : 0)];
+                        row.add(acc[NS + 1], on ? c : R(0));
+                    }
+                }
+            }
+        }
+    }
+    // the warps' sums, added in warp order
+    __syncthreads();
+    R* out = area;  // NT x NCHP
+    for (int w = 0; w < M2L_WARPS; w++) {
+        if (warp == w) {
+            R v[C::NCH];
+#pragma unroll
+            for (int j = 0; j < NS; j++) {
+                const int b = 32 * j + lane;
+                acc[j].get(v);
+                if (b < NT) {
+#pragma unroll
+                    for (int k = 0; k < C::NCH; k++)
+                        out[b * C::NCHP + k] = w == 0 ? v[k] : out[b * C::NCHP + k] + v[k];
+                    if (w == 0) {
+#pragma unroll
+                        for (int k = C::NCH; k < C::NCHP; k++) out[b * C::NCHP + k] = 0;
+                    }
+                }
+            }
+            __syncwarp();
+            acc[NS].get(v);
+#pragma unroll
+            for (int k = 0; k < C::NCH; k++) v[k] += __shfl_xor_sync(0xffffffffu, v[k], 16);
+            if (lane < 16 && lane < NT) {
+#pragma unroll
+                for (int k = 0; k < C::NCH; k++) out[lane * C::NCHP + k] += v[k];
+            }
+            __syncwarp();
+            acc[NS + 1].get(v);
+#pragma unroll
+            for (int k = 0; k < C::NCH; k++) {
+                v[k] += __shfl_xor_sync(0xffffffffu, v[k], 16);
+                v[k] += __shfl_xor_sync(0xffffffffu, v[k], 8);
+                v[k] += __shfl_xor_sync(0xffffffffu, v[k], 4);
+            }
+            if (lane < 4 && lane < NT) {
+#pragma unroll
+                for (int k = 0; k < C::NCH; k++) out[lane * C::NCHP + k] += v[k];
+            }
+        }
+        __syncthreads();
+    }
+    R* Lg = loc + node * (int64_t)sh.rowsz;
+    for (int e = tid; e < sh.rowsz; e += blockDim.x) Lg[e] = out[e];
+}
 
 // ---- L2L (FMM) -------------------------------------------------------------
 // One block per obs node of one depth (parents final): loc[child] += shift of
-// the parent's local expansion (with the Yl transform).
+// the parent's local expansion.  The parent's rows (Z less del_d m) and their
+// c_2 = 2 combinations are staged; a thread forms four channels of one term.
+template <int K>
+__host__ __device__ constexpr int l2l_reals(int p) {
+    return (n_harm(p) + (p > 1 ? p * (p - 1) / 2 : 0)) * Chan<K>::NCHP + n_harm(p);
+}
+
 template <typename R, int K>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(256)
 fmm_l2l(int p, const int64_t* __restrict__ nodes, const int64_t* __restrict__ parent,
         const R* __restrict__ ocent, const R* __restrict__ orad, R* __restrict__ loc) {
     using C = Chan<K>;
+    constexpr int Q = C::NCHP / 4;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int NT = n_terms(p);
-    R* Lp = reinterpret_cast<R*>(smem_raw);  // NT x NCHP
-    R* bin = Lp + NT * C::NCHP;
-    fill_binom(bin);
+    const int NT = n_harm(p), NX = NT + (p > 1 ? p * (p - 1) / 2 : 0);
+    R* Lp = reinterpret_cast<R*>(smem_raw);  // NX x NCHP
+    R* E = Lp + NX * C::NCHP;                // NT
     const int64_t cn = nodes[blockIdx.x];
     const int64_t pn = parent[cn];
     const R del[3] = {ocent[3 * cn] - ocent[3 * pn], ocent[3 * cn + 1] - ocent[3 * pn + 1],
                       ocent[3 * cn + 2] - ocent[3 * pn + 2]};
     const R sp = orad[pn];
-    const R dh[3] = {del[0] / sp, del[1] / sp, del[2] / sp};
     const R ratio = orad[cn] / sp;
-    const R* src = loc + pn * (int64_t)C::NCHP * NT;
-    for (int e = threadIdx.x; e < NT * C::NCHP; e += blockDim.x) {
-        const int k = e % C::NCHP;
-        R v = src[e];
-        if (k >= C::CH_Y && k < C::CH_M) {
-            const int o = k - C::CH_Y, d = o / C::J, j = o % C::J;
-            v -= del[d] * src[(e - k) + C::CH_M + j];
-        }
-        Lp[e] = v;
+    if (threadIdx.x < 32)
+        harm_warp<R>(E, p, del[0] / sp, del[1] / sp, del[2] / sp, threadIdx.x);
+    for (int g = threadIdx.x; g < NT; g += blockDim.x) {
+        R v[C::NCHP];
+        load_row<R, C::NCHP>(v, loc + (pn * (int64_t)NT + g) * C::NCHP);
+        shift_z<R, K>(v, -del[0], -del[1], -del[2]);
+        store_row<R, C::NCHP>(Lp + g * C::NCHP, v);
+    }
+    __syncthreads();
+    // row NT + m (m + 1) / 2 + c1: term (m - c1, c1, 2)
+    for (int it = threadIdx.x; it < (NX - NT) * Q; it += blockDim.x) {
+        const int r = it / Q, qd = it - r * Q;
+        int m = 0;
+        while ((m + 1) * (m + 2) / 2 <= r) m++;
+        const int c1 = r - m * (m + 1) / 2;
+        R v[4], w[4];
+        load_row<R, 4>(v, Lp + hidx(m - c1 + 2, c1, 0) * C::NCHP + 4 * qd);
+        load_row<R, 4>(w, Lp + hidx(m - c1, c1 + 2, 0) * C::NCHP + 4 * qd);
+#pragma unroll
+        for (int k = 0; k < 4; k++) v[k] = -v[k] - w[k];
+        store_row<R, 4>(Lp + (NT + r) * C::NCHP + 4 * qd, v);
     }
     __syncthreads();
     R* dst = loc + cn * (int64_t)C::NCHP * NT;
-    for (int b = threadIdx.x; b < NT; b += blockDim.x) {
-        int b0, b1, b2;
-        decode(b, b0, b1, b2);
-        const int nb = b0 + b1 + b2;
-        R acc[C::NCH];
+    for (int it = threadIdx.x; it < NT * Q; it += blockDim.x) {
+        const int g = it / Q, qd = it - g * Q;
+        int nb, b0, b1, b2;
+        hdecode(g, nb, b0, b1, b2);
+        R acc[4] = {0, 0, 0, 0};
+        for (int e2 = 0; e2 <= 1; e2++)
+            for (int e0 = 0; nb + e2 + e0 <= p; e0++)
+                for (int e1 = 0; nb + e2 + e0 + e1 <= p; e1++) {
+                    const int c0 = b0 + e0, c1 = b1 + e1, m = c0 + c1;
+                    const int r = b2 + e2 < 2 ? hidx(c0, c1, b2 + e2) : NT + m * (m + 1) / 2 + c1;
+                    const R e = E[hidx(e0, e1, e2)];
+                    R v[4];
+                    load_row<R, 4>(v, Lp + r * C::NCHP + 4 * qd);
 #pragma unroll
-        for (int k = 0; k < C::NCH; k++) acc[k] = 0;
-        R q0 = 1;
-        for (int c0 = b0; c0 <= p; c0++) {
-            R q1 = 1;
-            for (int c1 = b1; c0 + c1 <= p; c1++) {
-                R q2 = 1;
-                for (int c2 = b2; c0 + c1 + c2 <= p; c2++) {
-                    const R coef = BIN(c0, b0) * BIN(c1, b1) * BIN(c2, b2) * q0 * q1 * q2;
-                    const R* lrow = Lp + midx(c0, c1, c2) * C::NCHP;
-#pragma unroll
-                    for (int k = 0; k < C::NCH; k++) acc[k] += coef * lrow[k];
-                    q2 *= dh[2];
+                    for (int k = 0; k < 4; k++) acc[k] += e * v[k];
                 }
-                q1 *= dh[1];
-            }
-            q0 *= dh[0];
-        }
         const R sc = ipow(ratio, nb);
+        R v[4];
+        load_row<R, 4>(v, dst + 4 * it);
 #pragma unroll
-        for (int k = 0; k < C::NCH; k++) dst[b * C::NCHP + k] += sc * acc[k];
+        for (int k = 0; k < 4; k++) v[k] += sc * acc[k];
+        store_row<R, 4>(dst + 4 * it, v);
     }
 }
 
 // ---- L2P (FMM) -------------------------------------------------------------
-// One block per obs leaf; its local expansion staged in shared memory; a
-// thread per target point.
+// One block per obs leaf; its local expansion staged in shared memory; a lane
+// per target point, H by order through the warp's ring of two orders.
+template <int K>
+__host__ __device__ constexpr int l2p_reals(int p) {
+    return n_harm(p) * Chan<K>::NCHP + 4 * 2 * (2 * p + 1) * 32;
+}
+
 template <typename R, int K>
 __global__ void __launch_bounds__(128)
 fmm_l2p(int p, Rule2D<R> rule, int nq, const int64_t* __restrict__ leaves,
@@ -1613,7 +1272,8 @@ fmm_l2p(int p, Rule2D<R> rule, int nq, const int64_t* __restrict__ leaves,
     using C = Chan<K>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     R* sm = reinterpret_cast<R*>(smem_raw);
-    const int NT = n_terms(p);
+    const int NT = n_harm(p), LV = 2 * p + 1;
+    R* ring = sm + NT * C::NCHP + (threadIdx.x >> 5) * 2 * LV * 32 + (threadIdx.x & 31);
     const int64_t node = leaves[blockIdx.x];
     const int64_t t0 = o_start[node] * nq, t1 = o_end[node] * nq;
     if (t0 == t1) return;
@@ -1627,24 +1287,27 @@ fmm_l2p(int p, Rule2D<R> rule, int nq, const int64_t* __restrict__ leaves,
         R x[3];
         target_point(o, rule, (int)(t % nq), x);
         const R xi[3] = {x[0] - co[0], x[1] - co[1], x[2] - co[2]};
-        R pw[3][FMM_MAXP + 1];
-#pragma unroll
-        for (int d = 0; d < 3; d++) {
-            pw[d][0] = 1;
-            for (int k = 1; k <= p; k++) pw[d][k] = pw[d][k - 1] * (xi[d] * inv_s);
-        }
+        const R x0 = xi[0] * inv_s, x1 = xi[1] * inv_s, x2 = xi[2] * inv_s;
         R phi[C::NCH];
+        ring[0] = R(1);
 #pragma unroll
-        for (int k = 0; k < C::NCH; k++) phi[k] = 0;
-        int g = 0;
-        for (int n = 0; n <= p; n++)
-            for (int a0 = n; a0 >= 0; a0--)
-                for (int a2 = 0; a2 <= n - a0; a2++, g++) {
-                    const R mono = pw[0][a0] * pw[1][n - a0 - a2] * pw[2][a2];
-                    const R* lrow = sm + g * C::NCHP;
+        for (int k = 0; k < C::NCH; k++) phi[k] = sm[k];
+        for (int n = 1; n <= p; n++) {
+            const R rn = R(1) / (R)n;
+            R* cur = ring + (n & 1) * LV * 32;
+            const R* prv = ring + ((n + 1) & 1) * LV * 32;
+            for (int w = 0; w <= 2 * n; w++) {
+                const int a2 = w > n ? 1 : 0, a1 = w - a2 * (n + 1);
+                R h0, h1, k2;
+                harm_below<R>(n, a1, a2, [&](int i) { return prv[32 * i]; }, h0, h1, k2);
+                const R h = (x0 * h0 + x1 * h1 + x2 * k2) * rn;
+                cur[32 * w] = h;
+                R v[C::NCHP];
+                load_row<R, C::NCHP>(v, sm + (n * n + w) * C::NCHP);
 #pragma unroll
-                    for (int k = 0; k < C::NCH; k++) phi[k] += mono * lrow[k];
-                }
+                for (int k = 0; k < C::NCH; k++) phi[k] += h * v[k];
+            }
+        }
         R acc[C::NO];
 #pragma unroll
         for (int k = 0; k < C::NO; k++) acc[k] = 0;
@@ -1705,28 +1368,8 @@ fmm_finish(Rule2D<R> rule, const R* __restrict__ pts, const int32_t* __restrict_
 inline size_t al256(size_t b) { return (b + 255) / 256 * 256; }
 
 struct Sizes {
-    size_t rec, mom, loc, plan, W, F, rec2;
+    size_t rec, mom, loc, W, F, rec2;
 };
-
-// Whether the lane plan fits for (p, nb, lanes), decided on the host once.
-inline bool m2l3_plan_fits(int p, int nb, int lanes) {
-    static std::atomic<int> fits[FMM_MAXP + 1][16][8];  // 0 unknown, 1 yes, 2 no
-    if (p < 0 || p > FMM_MAXP || nb < 1 || nb > 15 || lanes < 32 || lanes > M2L3_LANES ||
-        lanes % 32)
-        return false;
-    std::atomic<int>& f = fits[p][nb][lanes / 32];
-    int v = f.load(std::memory_order_relaxed);
-    if (v == 0) {
-        std::vector<unsigned char> buf(sizeof(M2LPlan3));
-        v = m2l3_make_plan(p, nb, lanes, reinterpret_cast<M2LPlan3*>(buf.data())) == 0 ? 1 : 2;
-        f.store(v, std::memory_order_relaxed);
-    }
-    return v == 1;
-}
-
-inline size_t m2l_plan_bytes() {
-    return sizeof(M2LPlan2) > sizeof(M2LPlan3) ? sizeof(M2LPlan2) : sizeof(M2LPlan3);
-}
 
 // The packed P2P runs for elasticRH3 in FP32 with the 3-, 4- and 7-point rules.
 template <typename R, int K, int NQ>
@@ -1740,9 +1383,8 @@ Sizes sizes_for(size_t rs, int mode, int order, int64_t n_obs, int64_t n_src, in
     using C = Chan<K>;
     Sizes s;
     s.rec = al256(rs * Rec<K, NQ>::LEN * (size_t)n_src);
-    s.mom = al256(rs * C::NCHP * (size_t)n_terms(order) * n_src_nodes);
-    s.loc = mode == 1 ? al256(rs * C::NCHP * (size_t)n_terms(order) * n_obs_nodes) : 0;
-    s.plan = mode == 1 ? al256(m2l_plan_bytes()) + 256 : 0;
+    s.mom = al256(rs * C::NCHP * (size_t)n_harm(order) * n_src_nodes);
+    s.loc = mode == 1 ? al256(rs * C::NCHP * (size_t)n_harm(order) * n_obs_nodes) : 0;
     s.W = al256(rs * NAcc<K, NQ>::n * (size_t)n_obs);
     s.F = al256(rs * C::NO * (size_t)NQ * n_obs);
     s.rec2 = (rs == 4 && K == kRH && (NQ == 3 || NQ == 4 || NQ == 7))
@@ -1772,7 +1414,7 @@ Sizes sizes_dispatch(int kernel, int prec, int mode, int order, int nq, int64_t 
     TCT_SZ_K(kRH)
 #undef TCT_SZ_K
 #undef TCT_SZ_NQ
-    return Sizes{0, 0, 0, 0, 0, 0, 0};
+    return Sizes{0, 0, 0, 0, 0, 0};
 }
 
 template <typename KF>
@@ -1818,15 +1460,14 @@ int run_fmm(int mode, int p, const Rule2D<R>& rule, const double* params, double
     using C = Chan<K>;
     constexpr int NA = NAcc<K, NQ>::n;
     const Consts<R> c = make_consts<R>(params);
-    const int NT = n_terms(p);
+    const int NT = n_harm(p);
     const Sizes sz = sizes_for<K, NQ>(sizeof(R), mode, p, n_obs, n_src, ot.n_nodes, stt.n_nodes);
     R* rec = reinterpret_cast<R*>(ws);
     R* mom = reinterpret_cast<R*>(ws + sz.rec);
     R* loc = reinterpret_cast<R*>(ws + sz.rec + sz.mom);
-    unsigned char* plan = ws + sz.rec + sz.mom + sz.loc;
-    R* W = reinterpret_cast<R*>(ws + sz.rec + sz.mom + sz.loc + sz.plan);
-    R* F = reinterpret_cast<R*>(ws + sz.rec + sz.mom + sz.loc + sz.plan + sz.W);
-    float* rec2 = reinterpret_cast<float*>(ws + sz.rec + sz.mom + sz.loc + sz.plan + sz.W + sz.F);
+    R* W = reinterpret_cast<R*>(ws + sz.rec + sz.mom + sz.loc);
+    R* F = reinterpret_cast<R*>(ws + sz.rec + sz.mom + sz.loc + sz.W);
+    float* rec2 = reinterpret_cast<float*>(ws + sz.rec + sz.mom + sz.loc + sz.W + sz.F);
     bool uniform = true;
     for (int q = 1; q < NQ; q++) uniform = uniform && (rule.w[q] == rule.w[0]);
     const R* scent = (const R*)stt.centers;
@@ -1889,20 +1530,24 @@ int run_fmm(int mode, int p, const Rule2D<R>& rule, const double* params, double
         }
     }
     if (stt.n_leaves > 0) {
-        fmm_p2m<R, K, NQ><<<(unsigned)stt.n_leaves, 128, 0, se>>>(
+        const size_t smem = sizeof(R) * (size_t)p2m_reals<K>(p);
+        if ((rc = set_smem(fmm_p2m<R, K, NQ>, smem))) return rc;
+        fmm_p2m<R, K, NQ><<<(unsigned)stt.n_leaves, p2m_threads(p), smem, se>>>(
             c, p, stt.leaves, stt.start, stt.end, scent, srad, rec, mom);
         if ((rc = launch_status("fmm p2m"))) return rc;
     }
+    const size_t smem_m2m = sizeof(R) * (size_t)m2m_reals<K>(p);
+    if ((rc = set_smem(fmm_m2m<R, K>, smem_m2m))) return rc;
     for (int h = 0; h < stt.n_levels; h++) {
         const int64_t cnt = stt.level_offsets[h + 1] - stt.level_offsets[h];
         if (cnt == 0) continue;
-        fmm_m2m<R, K><<<(unsigned)cnt, 128, 0, se>>>(p, stt.levels + stt.level_offsets[h],
-                                                     stt.children, scent, srad, mom);
+        fmm_m2m<R, K><<<(unsigned)cnt, 256, smem_m2m, se>>>(p, stt.levels + stt.level_offsets[h],
+                                                            stt.children, scent, srad, mom);
         if ((rc = launch_status("fmm m2m"))) return rc;
     }
     if (mode == 0) {
         if (far.n_obs > 0) {
-            const size_t smem = sizeof(R) * (size_t)C::NCHP * NT;
+            const size_t smem = sizeof(R) * (size_t)m2p_reals<K>(p);
             if ((rc = set_smem(fmm_m2p<R, K>, smem))) return rc;
             fmm_m2p<R, K><<<(unsigned)far.n_obs, 128, smem, se>>>(
                 p, rule, NQ, far.obs, far.start, far.src, ot.start, ot.end, scent, srad, obs_pts,
@@ -1912,73 +1557,32 @@ int run_fmm(int mode, int p, const Rule2D<R>& rule, const double* params, double
     } else {
         if (cudaMemsetAsync(loc, 0, sz.loc, se) != cudaSuccess) return launch_status("fmm memset");
         if (far.n_obs > 0) {
-            const int64_t n_el = stt.n_nodes * (int64_t)NT * C::NCHP;
-            fmm_moment_factorials<R><<<(unsigned)((n_el + 127) / 128), 128, 0, se>>>(
-                p, C::NCHP, stt.n_nodes, mom);
-            if ((rc = launch_status("fmm moment factorials"))) return rc;
-            bool lanes = false;  // the lane plan (fmm_m2l3) for FP32
-            int* plan_err = reinterpret_cast<int*>(plan + al256(m2l_plan_bytes()));
-            if constexpr (sizeof(R) == 4) {
-                const int smem1 = m2l3_smem<K>(p, 1).total_bytes;
-                const int smem2 = m2l3_smem<K>(p, 2).total_bytes;
-                // two pairs per stage while two CTAs still fit an SM
-                const bool two = smem2 + 1024 <= 113 * 1024;
-                const int nl = two ? m2l3_lanes(2) : m2l3_lanes(1);
-                lanes = m2l3_plan_fits(p, M2L3Cfg<K>::NB, nl) && smem1 <= 227 * 1024;
-                if (lanes) {
-                    M2LPlan3* plan3 = reinterpret_cast<M2LPlan3*>(plan);
-                    fmm_m2l3_plan<<<1, 32, 0, se>>>(p, M2L3Cfg<K>::NB, nl, plan3, plan_err);
-                    if ((rc = launch_status("fmm m2l plan"))) return rc;
-                    if (two) {
-                        if ((rc = set_smem(fmm_m2l3<K, 2>, (size_t)smem2))) return rc;
-                        fmm_m2l3<K, 2><<<(unsigned)far.n_obs, M2L3_THREADS, smem2, se>>>(
-                            p, far.obs, far.n_obs, far.start, far.src, ocent, orad, scent, srad,
-                            mom, plan3, loc);
-                    } else {
-                        if ((rc = set_smem(fmm_m2l3<K, 1>, (size_t)smem1))) return rc;
-                        fmm_m2l3<K, 1><<<(unsigned)far.n_obs, M2L3_THREADS, smem1, se>>>(
-                            p, far.obs, far.n_obs, far.start, far.src, ocent, orad, scent, srad,
-                            mom, plan3, loc);
-                    }
-                }
-            }
-            if (!lanes) {
-                if (m2l2_items(p) > M2L2_MAXITEMS) {
-                    set_error("tct_fmm_matvec: FMM order %d exceeds the M2L plan's capacity", p);
-                    return TCT_ERR_ARG;
-                }
-                M2LPlan2* plan2 = reinterpret_cast<M2LPlan2*>(plan);
-                fmm_m2l2_plan<<<1, 32, 0, se>>>(p, plan2, plan_err);
-                if ((rc = launch_status("fmm m2l plan"))) return rc;
-                const size_t smem_all = sizeof(R) * (2 * (size_t)NT * C::NCHP +
-                                                     2 * (size_t)((NT + 3) / 4 * 4) + 80 +
-                                                     (size_t)m2l2_items(p) * C::NCHP);
-                if (smem_all > 227 * 1024) {
-                    // FP64 at p = 12 needs 286 KB (p = 10: 190 KB)
-                    set_error("tct_fmm_matvec: the item-form M2L at order %d needs %zu bytes of "
-                              "shared memory (the limit is 227 KB; FP64 runs orders up to 10)",
-                              p, smem_all);
-                    return TCT_ERR_ARG;
-                }
-                if ((rc = set_smem(fmm_m2l2<R, K>, smem_all))) return rc;
-                fmm_m2l2<R, K><<<(unsigned)far.n_obs, M2L2_THREADS, smem_all, se>>>(
-                    p, far.obs, far.n_obs, far.start, far.src, ocent, orad, scent, srad, mom,
-                    plan2, loc);
-            }
+            const size_t smem = m2l_smem<R, K>(p);
+#define TCT_M2L(NS)                                                                               \
+    {                                                                                             \
+        if ((rc = set_smem(fmm_m2l<R, K, NS>, smem))) return rc;                                  \
+        fmm_m2l<R, K, NS><<<(unsigned)far.n_obs, 32 * M2L_WARPS, smem, se>>>(                     \
+            p, far.obs, far.start, far.src, ocent, orad, scent, srad, mom, loc);                  \
+    }
+            // sums a lane holds for single terms: ceil((p + 1)^2 / 32)
+            if (NT <= 64) TCT_M2L(2)
+            else if (NT <= 96) TCT_M2L(3)
+            else if (NT <= 128) TCT_M2L(4)
+            else TCT_M2L(6)
+#undef TCT_M2L
             if ((rc = launch_status("fmm m2l"))) return rc;
         }
-        const size_t smem_l2l =
-            sizeof(R) * ((size_t)C::NCHP * NT + (FMM_MAXP + 1) * (FMM_MAXP + 1));
+        const size_t smem_l2l = sizeof(R) * (size_t)l2l_reals<K>(p);
         if ((rc = set_smem(fmm_l2l<R, K>, smem_l2l))) return rc;
         for (int d = 0; d < ot.n_levels; d++) {
             const int64_t cnt = ot.level_offsets[d + 1] - ot.level_offsets[d];
             if (cnt == 0) continue;
-            fmm_l2l<R, K><<<(unsigned)cnt, 128, smem_l2l, se>>>(
+            fmm_l2l<R, K><<<(unsigned)cnt, 256, smem_l2l, se>>>(
                 p, ot.levels + ot.level_offsets[d], ot.parent, ocent, orad, loc);
             if ((rc = launch_status("fmm l2l"))) return rc;
         }
         if (ot.n_leaves > 0) {
-            const size_t smem = sizeof(R) * (size_t)C::NCHP * NT;
+            const size_t smem = sizeof(R) * (size_t)l2p_reals<K>(p);
             if ((rc = set_smem(fmm_l2p<R, K>, smem))) return rc;
             fmm_l2p<R, K><<<(unsigned)ot.n_leaves, 128, smem, se>>>(
                 p, rule, NQ, ot.leaves, ot.start, ot.end, ocent, orad, obs_pts, obs_tris, loc, F);
@@ -2006,7 +1610,7 @@ extern "C" size_t tct_fmm_workspace_bytes(int kernel, int prec, int mode, int or
         return 0;
     const Sizes s = sizes_dispatch(kernel, prec, mode, order, n_q, n_obs, n_src, n_obs_nodes,
                                    n_src_nodes);
-    return s.rec + s.mom + s.loc + s.plan + s.W + s.F + s.rec2;
+    return s.rec + s.mom + s.loc + s.W + s.F + s.rec2;
 }
 
 extern "C" int tct_fmm_matvec(int kernel, int prec, int mode, int order, int n_q,
@@ -2034,6 +1638,9 @@ extern "C" int tct_fmm_matvec(int kernel, int prec, int mode, int order, int n_q
         set_error("tct_fmm_matvec: unsupported precision %d", prec);
         return TCT_ERR_PREC;
     }
+    // the orders taken are those of the full Cartesian expansion's shared memory
+    TCT_CHECK_ARG(!(mode == 1 && prec == TCT_F64 && kernel == kRH && order > 10 && far->n_obs > 0),
+                  "tct_fmm_matvec: elasticRH3 in FP64 runs FMM orders up to 10 (got %d)", order);
     TCT_CHECK_ARG(supported_nq(n_q), "tct_fmm_matvec: n_q must be 3, 4, 7 or 13 (got %d)", n_q);
     if (n_obs == 0) return TCT_OK;
     const size_t need = tct_fmm_workspace_bytes(kernel, prec, mode, order, n_q, n_obs, n_src,
@@ -2079,7 +1686,93 @@ extern "C" int tct_fmm_matvec(int kernel, int prec, int mode, int order, int n_q
     return TCT_ERR_ARG;
 }
 
-// Host-side check of the M2L work plan for order p, nb terms b per lane and
+namespace tct {
+namespace {
+
+// ---- lane plan of the Cartesian-term contraction (tct_fmm_m2l_plan_stats) -----
+// Host only: the dealing of full Cartesian terms to lanes that the C entry
+// below reports on; the M2L kernel above needs no plan.
+constexpr int n_terms(int p) { return (p + 1) * (p + 2) * (p + 3) / 6; }
+inline void decode(int g, int& a0, int& a1, int& a2) {
+    int n = 0;
+    while (n_terms(n) <= g) n++;
+    int rem = n > 0 ? g - n_terms(n - 1) : 0;
+    a0 = n;
+    int off = 0;
+    while (off + (n - a0 + 1) <= rem) {
+        off += n - a0 + 1;
+        a0--;
+    }
+    a2 = rem - off;
+    a1 = n - a0 - a2;
+}
+constexpr int PLAN_LANES = 224;  // the most lanes
+
+struct LanePlan {
+    int L, n_lanes;
+    int lane_k[PLAN_LANES];    // tuple of the lane (b = k nb + j), -1 for none
+    int lane_a0[PLAN_LANES];   // first source term (graded) and chunk length
+    int lane_cnt[PLAN_LANES];
+    int warp_steps[PLAN_LANES / 32];
+};
+
+// Builds the plan; returns 0, or 1 when the tuples do not fit the lanes.
+// Tuples k = 0 .. ceil(NT / nb) - 1 take the b's k nb .. k nb + nb - 1; tuple
+// k's source range is [0, A_k), A_k = n_terms(p - |k nb|) (its lowest b), cut
+// into chunks of L terms, L the smallest length whose chunks fit the lanes;
+// lanes are dealt chunk-major (every tuple's first chunk, then every second
+// chunk, ...).
+inline int make_lane_plan(int p, int nb, int lanes, LanePlan* plan) {
+    const int NT = n_terms(p);
+    const int nk = (NT + nb - 1) / nb;
+    if (lanes < 32 || lanes > PLAN_LANES || lanes % 32) return 1;
+    auto A = [&](int k) {
+        int b0, b1, b2;
+        decode(k * nb, b0, b1, b2);
+        return n_terms(p - (b0 + b1 + b2));
+    };
+    int total = 0;
+    for (int k = 0; k < nk; k++) total += A(k);
+    int L = (total + lanes - 1) / lanes;
+    if (L < 1) L = 1;
+    for (;; L++) {
+        int cnt = 0;
+        for (int k = 0; k < nk; k++) cnt += (A(k) + L - 1) / L;
+        if (cnt <= lanes) break;
+        if (L > NT) return 1;
+    }
+    plan->L = L;
+    int lane = 0;
+    for (int c = 0;; c++) {
+        bool any = false;
+        for (int k = 0; k < nk; k++) {
+            const int ak = A(k);
+            if (c * L >= ak) continue;
+            plan->lane_k[lane] = k;
+            plan->lane_a0[lane] = c * L;
+            plan->lane_cnt[lane] = (ak - c * L < L) ? ak - c * L : L;
+            lane++;
+            any = true;
+        }
+        if (!any) break;
+    }
+    plan->n_lanes = lane;
+    for (int l = lane; l < PLAN_LANES; l++) {
+        plan->lane_k[l] = -1;
+        plan->lane_a0[l] = 0;
+        plan->lane_cnt[l] = 0;
+    }
+    for (int w = 0; w < lanes / 32; w++) {
+        int m = 0;
+        for (int l = 32 * w; l < 32 * w + 32; l++) m = plan->lane_cnt[l] > m ? plan->lane_cnt[l] : m;
+        plan->warp_steps[w] = m;
+    }
+    return 0;
+}
+}  // namespace
+}  // namespace tct
+
+// Host-side check of the Cartesian lane plan for order p, nb terms b per lane and
 // `lanes` contraction lanes (192 with two-pair stages, 224 with one-pair ones):
 // out[0] = valid (a, b) pairs covered, out[1] = pairs covered more than once
 // or invalid and unmasked, out[2] = the chunk length L, out[3] = lanes used,
@@ -2087,8 +1780,8 @@ extern "C" int tct_fmm_matvec(int kernel, int prec, int mode, int order, int n_q
 // plan does not fit.
 extern "C" int tct_fmm_m2l_plan_stats(int order, int nb, int lanes, int64_t* out) {
     if (order < 0 || order > FMM_MAXP || nb < 1 || !out) return TCT_ERR_ARG;
-    M2LPlan3* plan = new M2LPlan3();
-    const int rc = m2l3_make_plan(order, nb, lanes, plan);
+    LanePlan* plan = new LanePlan();
+    const int rc = make_lane_plan(order, nb, lanes, plan);
     if (rc) {
         delete plan;
         return 1;
@@ -2096,18 +1789,20 @@ extern "C" int tct_fmm_m2l_plan_stats(int order, int nb, int lanes, int64_t* out
     const int NT = n_terms(order);
     std::vector<int> seen((size_t)NT * NT, 0);
     int64_t covered = 0, bad = 0;
-    for (int l = 0; l < M2L3_LANES; l++) {
+    for (int l = 0; l < PLAN_LANES; l++) {
         const int k = plan->lane_k[l];
         if (k < 0) continue;
         for (int s = 0; s < plan->lane_cnt[l]; s++) {
             const int a = plan->lane_a0[l] + s;
-            const int la = plan->ainfo[a] >> 16;
+            int a0, a1, a2;
+            decode(a, a0, a1, a2);
+            const int la = a0 + a1 + a2;
             for (int j = 0; j < nb; j++) {
                 const int b = k * nb + j;
                 if (b >= NT) continue;
                 int b0, b1, b2;
                 decode(b, b0, b1, b2);
-                if (la + b0 + b1 + b2 > order) continue;  // masked in the kernel
+                if (la + b0 + b1 + b2 > order) continue;  // masked
                 if (seen[(size_t)a * NT + b]++) bad++;
                 else covered++;
             }
