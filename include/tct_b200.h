@@ -434,6 +434,37 @@ int tct_fmm_matvec(int kernel, int prec, int mode, int order, int n_q,
                    void* out, int accumulate, void* workspace, size_t workspace_bytes,
                    void* stream);
 
+/* Work plan of the near leaves (device arrays; the layouts fmm/p2p_plan.py
+ * writes): observation chunks of at most `chunk` triangles (64 for
+ * elasticRH3 in FP32 with a 3-, 4- or 7-point rule, else 32) against runs of
+ * list entries.
+ *   tasks    n_tasks x 4: first obs triangle (tree order), count, first and
+ *            end entry (at most 128 entries)
+ *   entries  first source triangle, count, first slot or -1 (one-sided)
+ *   chunks   n_chunks x 7: first obs triangle, count, first and end task,
+ *            first and end of its slots_in, offset of the chunk in its node
+ *   slots_in first slots of the entries whose source is the chunk's node
+ * sym: unordered pairs, both directions added (elasticRH3, one tree on both
+ * sides). */
+typedef struct tct_fmm_p2p_plan {
+    int64_t n_tasks, n_chunks, n_slots;
+    int chunk, sym;
+    const int32_t *tasks, *entries, *chunks, *slots_in;
+} tct_fmm_p2p_plan;
+
+/* tct_fmm_matvec with the near list as a work plan (`p2p` is not read). */
+size_t tct_fmm_planned_workspace_bytes(int kernel, int prec, int mode, int order, int n_q,
+                                       int64_t n_obs, int64_t n_src, int64_t n_obs_nodes,
+                                       int64_t n_src_nodes, const tct_fmm_p2p_plan* plan);
+int tct_fmm_matvec_planned(int kernel, int prec, int mode, int order, int n_q,
+                           const double* quad_pts, const double* quad_wts, const double* params,
+                           double out_scale, const void* obs_pts, const int32_t* obs_tris,
+                           int64_t n_obs, const tct_fmm_tree* obs_tree, const void* src_pts,
+                           const int32_t* src_tris, int64_t n_src, const tct_fmm_tree* src_tree,
+                           const tct_fmm_list* p2p, const tct_fmm_list* far, const void* in,
+                           void* out, int accumulate, void* workspace, size_t workspace_bytes,
+                           void* stream, const tct_fmm_p2p_plan* plan);
+
 /* ---- multi-RHS farfield on the tensor cores ------------------------------- */
 
 /* Direct farfield of elasticRH3 (FP32; n_q = 3, 4 or 7 point triangle rule,

@@ -172,6 +172,13 @@ class FmmList(ctypes.Structure):
     _fields_ = [("obs", c_p), ("start", c_p), ("src", c_p), ("n_obs", c_i64)]
 
 
+class FmmP2PPlan(ctypes.Structure):
+    """Mirror of tct_fmm_p2p_plan."""
+    _fields_ = [("n_tasks", c_i64), ("n_chunks", c_i64), ("n_slots", c_i64), ("chunk", c_i),
+                ("sym", c_i), ("tasks", c_p), ("entries", c_p), ("chunks", c_p),
+                ("slots_in", c_p)]
+
+
 _FMM_SIGS = {
     "tct_fmm_workspace_bytes": ([c_i, c_i, c_i, c_i, c_i, c_i64, c_i64, c_i64, c_i64], c_sz),
     "tct_fmm_m2l_plan_stats": ([c_i, c_i, c_i, ctypes.POINTER(c_i64)], c_i),
@@ -179,6 +186,13 @@ _FMM_SIGS = {
                         c_i64, ctypes.POINTER(FmmTree), c_p, c_p, c_i64,
                         ctypes.POINTER(FmmTree), ctypes.POINTER(FmmList),
                         ctypes.POINTER(FmmList), c_p, c_p, c_i, c_p, c_sz, c_p], c_i),
+    "tct_fmm_planned_workspace_bytes": ([c_i, c_i, c_i, c_i, c_i, c_i64, c_i64, c_i64, c_i64,
+                                         ctypes.POINTER(FmmP2PPlan)], c_sz),
+    "tct_fmm_matvec_planned": ([c_i, c_i, c_i, c_i, c_i, c_dp, c_dp, c_dp, ctypes.c_double, c_p,
+                                c_p, c_i64, ctypes.POINTER(FmmTree), c_p, c_p, c_i64,
+                                ctypes.POINTER(FmmTree), ctypes.POINTER(FmmList),
+                                ctypes.POINTER(FmmList), c_p, c_p, c_i, c_p, c_sz, c_p,
+                                ctypes.POINTER(FmmP2PPlan)], c_i),
 }
 for _name, (_args, _res) in _FMM_SIGS.items():
     _f = getattr(lib, _name)

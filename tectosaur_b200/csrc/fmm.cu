@@ -45,12 +45,13 @@
 //
 // Kept terms a, |a| = n <= p, are stored by order: hidx(a) = n^2 + a_2 (n + 1) + a_1.
 //
-// P2P runs the direct farfield's triangle-level pair loop (far_common.cuh) on
-// the listed leaf pairs, from the same per-source records the P2M reads.
+// P2P runs the direct farfield's triangle-level pair sums on the listed leaf
+// pairs (fmm_p2p.cu on a work plan).
 #include <algorithm>
 #include <vector>
 
 #include "far_common.cuh"
+#include "fmm_p2p.h"
 
 namespace tct {
 namespace {
@@ -465,19 +466,7 @@ fmm_m2m(int p, const int64_t* __restrict__ parents, const int64_t* __restrict__ 
     }
 }
 
-__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
-                     (uint32_t)__cvta_generic_to_shared(smem_dst)),
-                 "l"(gsrc)
-                 : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait_group() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
-// ---- P2P -------------------------------------------------------------------
+// ---- P2P without a plan (tct_fmm_matvec; fmm_p2p.cu has the planned one) ------
 // One block per obs leaf with a non-empty P2P list.  The leaf's m obs
 // triangles take m threads; the block's 128 threads form G = 128 / m groups,
 // and group g takes the g-th of G equal slices of the list's source
@@ -556,222 +545,6 @@ fmm_p2p(Consts<R> c, Rule2D<R> rule, const R* __restrict__ pts,
             for (int k = 0; k < NA; k++) {
                 R sacc = 0;
                 for (int g = 0; g < G; g++) sacc += red[(g * m + threadIdx.x) * NA + k];
-                w[k] = sacc;
-            }
-        }
-    }
-}
-
-// ---- P2P, packed elasticRH3 in FP32 ------------------------------------------
-// fmm_p2p with the direct farfield's packed pair sums (rh2_pair).  A chunk of
-// m <= 128 obs triangles of the leaf is split into T >= ceil(m / 64) teams of
-// mt = ceil(m / T) triangles (T chosen for the fewest idle lanes); a group of h = ceil(mt / 2) lanes covers a team
-// (a lane takes triangles li and li + h, one in each f32x2 half), a warp holds
-// Gw = 32 / h groups (at most P2P_CHW), and the block's 4 Gw groups are team
-// g % T and slice g / T of S = 4 Gw / T equal slices of the list's source
-// triangles (concatenated in list order), so that small leaves still fill
-// the lanes.  A group streams its slice through its own two shared-memory
-// buffers of CHg = min(P2P_CHW / Gw, h) packed records (cp.async, the next
-// chunk in flight while the current one is summed; records read as
-// broadcasts within the group), and Kahan-folds its packed sums into its
-// totals every 16 or more records.  Slice totals are added in a fixed order.
-// W[t] = the 9 sums of obs triangle t in the NAcc layout (overwritten).
-constexpr int P2P_CHW = 24;  // staged records per warp and buffer
-
-template <int NQ>
-constexpr size_t p2p_rh2_smem() {
-    return sizeof(float) * (128 * 18 + 4 * 2 * P2P_CHW * RecRH2<NQ>::LEN);
-}
-
-template <int NQ, bool UNIFORM>
-__global__ void __launch_bounds__(128, NQ == 3 ? 4 : 3)
-fmm_p2p_rh2(Rule2D<float> rule, const float* __restrict__ pts,
-            const int32_t* __restrict__ obs_tris, const int64_t* __restrict__ obs_nodes,
-            const int64_t* __restrict__ starts, const int64_t* __restrict__ srcs,
-            const int64_t* __restrict__ o_start, const int64_t* __restrict__ o_end,
-            const int64_t* __restrict__ s_start, const int64_t* __restrict__ s_end,
-            const float* __restrict__ rec, float* __restrict__ W) {
-    using L = RecRH2<NQ>;
-    constexpr int V4 = L::LEN / 4;  // float4s per record
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    float* red = reinterpret_cast<float*>(smem_raw);  // 128 x 18 slice totals
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    float* wbuf = red + 128 * 18 + warp * 2 * P2P_CHW * L::LEN;  // this warp's staging
-    const int64_t node = obs_nodes[blockIdx.x];
-    const int64_t l0 = starts[blockIdx.x], l1 = starts[blockIdx.x + 1];
-    const int64_t ob0 = o_start[node], n_o = o_end[node] - ob0;
-    f2_t wq[UNIFORM ? 1 : NQ * NQ];
-    wq[0] = 0ull;
-    if (!UNIFORM) {
-#pragma unroll
-        for (int q1 = 0; q1 < NQ; q1++)
-#pragma unroll
-            for (int q2 = 0; q2 < NQ; q2++) {
-                const float w = rule.w[q1] * rule.w[q2];
-                wq[q1 * NQ + q2] = pk(w, w);
-            }
-    }
-    const f2_t eps = pk(RH2_EPS, RH2_EPS);
-    int n_s = 0;  // source triangles over the whole list (warp reduction)
-    for (int64_t l = l0 + lane; l < l1; l += 32) {
-        const int64_t sn = srcs[l];
-        n_s += (int)(s_end[sn] - s_start[sn]);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) n_s += __shfl_xor_sync(0xffffffffu, n_s, o);
-
-    for (int64_t cb = 0; cb < n_o; cb += 128) {
-        const int m = (int)min((int64_t)128, n_o - cb);
-        // teams: the count (from ceil(m / 64) up to 8) with the most slices per
-        // obs triangle, m S, i.e. the fewest idle lanes and halves
-        int T = (m + 63) / 64;
-        {
-            int best = 0, bt = T;
-            for (int t = T; t <= 8; t++) {
-                const int mtt = (m + t - 1) / t, ht = (mtt + 1) / 2;
-                const int st = 4 * min(32 / ht, P2P_CHW) / t;
-                if (m * st > best) {
-                    best = m * st;
-                    bt = t;
-                }
-            }
-            T = bt;
-        }
-        const int mt = (m + T - 1) / T;
-        const int h = (mt + 1) / 2;
-        const int Gw = min(32 / h, P2P_CHW);
-        const int S = 4 * Gw / T;
-        const int gl = lane / h, li = lane - gl * h;
-        const int gi = warp * Gw + gl;
-        const int team = gi % T, slice = gi / T;
-        const bool active = gl < Gw && slice < S;
-        const int tb = team * mt, mteam = min(mt, m - tb);
-        const bool va = active && li < mteam, vb = active && li + h < mteam;
-        const int CHg = min(P2P_CHW / Gw, h);
-        const int gbase = gl * h;
-        const unsigned gmask = (h == 32 ? 0xffffffffu : ((1u << h) - 1u)) << (gbase & 31);
-        float* buf = wbuf + (gl < Gw ? gl : 0) * 2 * CHg * L::LEN;
-        float tot[2][9], cmp[2][9];
-#pragma unroll
-        for (int k = 0; k < 9; k++) {
-            tot[0][k] = tot[1][k] = 0.f;
-            cmp[0][k] = cmp[1][k] = 0.f;
-        }
-        if (active) {
-            f2_t negx[NQ][3];
-            {
-                TriGeom<float> oa, ob;
-                if (va) load_tri(oa, pts, obs_tris, ob0 + cb + tb + li, 0, false, true);
-                if (vb) load_tri(ob, pts, obs_tris, ob0 + cb + tb + li + h, 0, false, true);
-#pragma unroll
-                for (int q = 0; q < NQ; q++) {
-                    const float ox = rule.x[q], oy = rule.y[q];
-                    const float bq[3] = {1 - ox - oy, ox, oy};
-#pragma unroll
-                    for (int d = 0; d < 3; d++)
-                        negx[q][d] = pk(va ? -bary_point(oa, bq, d) : 0.f,
-                                        vb ? -bary_point(ob, bq, d) : 0.f);
-                }
-            }
-            // the slice [p0, p1) of the concatenated sources; the stream
-            // cursor (list entry l, its first record a, offset off, records
-            // left rem), the same in every lane of the group
-            const int p0 = (int)((int64_t)n_s * slice / S);
-            const int p1 = (int)((int64_t)n_s * (slice + 1) / S);
-            int64_t l = l0, a = 0;
-            int off = 0, rem = 0, skip = p0;
-            while (l < l1) {  // find the entry holding position p0
-                const int64_t sn = srcs[l];
-                a = s_start[sn];
-                rem = (int)(s_end[sn] - a);
-                if (skip < rem) break;
-                skip -= rem;
-                l++;
-            }
-            off = skip;
-            rem -= skip;
-            // copy the next `need` (<= CHg <= h) stream records into buffer b
-            auto issue = [&](int need, int b) {
-                int64_t gidx = 0;
-                int r_base = 0;
-                while (r_base < need) {
-                    while (rem == 0 && l + 1 < l1) {
-                        l++;
-                        const int64_t sn = srcs[l];
-                        a = s_start[sn];
-                        rem = (int)(s_end[sn] - a);
-                        off = 0;
-                    }
-                    const int take = min(rem, need - r_base);
-                    if (take <= 0) break;  // unreachable: the slice never outruns the list
-                    if (li >= r_base && li < r_base + take) gidx = a + off + (li - r_base);
-                    r_base += take;
-                    off += take;
-                    rem -= take;
-                }
-                float* dst = buf + b * CHg * L::LEN;
-                for (int e0 = 0; e0 < need * V4; e0 += h) {  // uniform within the group
-                    const int e = e0 + li;
-                    const int r = min(e / V4, need - 1), part = e - r * V4;
-                    const int64_t g = __shfl_sync(gmask, gidx, gbase + r);
-                    if (e < need * V4)
-                        cp_async16(dst + r * L::LEN + part * 4, rec + g * L::LEN + part * 4);
-                }
-                cp_async_commit();
-            };
-            const int n_mine = p1 - p0;
-            f2_t Wp[9];
-#pragma unroll
-            for (int k = 0; k < 9; k++) Wp[k] = 0ull;
-            int since = 0;
-            if (n_mine > 0) issue(min(CHg, n_mine), 0);
-            for (int c0 = 0; c0 < n_mine; c0 += CHg) {
-                const int cur = (c0 / CHg) & 1;
-                const int need = min(CHg, n_mine - c0);
-                if (c0 + CHg < n_mine) {
-                    issue(min(CHg, n_mine - c0 - CHg), cur ^ 1);
-                    cp_async_wait_group<1>();
-                } else {
-                    cp_async_wait_group<0>();
-                }
-                __syncwarp(gmask);
-                const float* rb = buf + cur * CHg * L::LEN;
-#pragma unroll 2
-                for (int j = 0; j < need; j++)
-                    rh2_pair<NQ, UNIFORM>(reinterpret_cast<const f2_t*>(rb + j * L::LEN), negx,
-                                          wq, eps, Wp);
-                since += need;
-                if (since >= 16 || c0 + CHg >= n_mine) {
-#pragma unroll
-                    for (int k = 0; k < 9; k++) {
-                        float wa, wb;
-                        upk(Wp[k], wa, wb);
-                        fold<float, true>(tot[0][k], cmp[0][k], wa);
-                        fold<float, true>(tot[1][k], cmp[1][k], wb);
-                        Wp[k] = 0ull;
-                    }
-                    since = 0;
-                }
-                __syncwarp(gmask);  // buffer cur is free for the chunk after next
-            }
-        }
-        __syncthreads();  // the previous chunk's reads of red are done
-#pragma unroll
-        for (int k = 0; k < 9; k++) {
-            red[threadIdx.x * 18 + k] = tot[0][k];
-            red[threadIdx.x * 18 + 9 + k] = tot[1][k];
-        }
-        __syncthreads();
-        for (int t = threadIdx.x; t < m; t += blockDim.x) {
-            const int tm = t / mt, within = t - tm * mt;
-            const int half = within / h, ln = within - half * h;
-            float* w = W + (ob0 + cb + t) * 9;
-            for (int k = 0; k < 9; k++) {
-                float sacc = 0.f;
-                for (int sl = 0; sl < S; sl++) {
-                    const int g = sl * T + tm, wg = g / Gw, lg = g - wg * Gw;
-                    sacc += red[(wg * 32 + lg * h + ln) * 18 + half * 9 + k];
-                }
                 w[k] = sacc;
             }
         }
@@ -1368,14 +1141,8 @@ fmm_finish(Rule2D<R> rule, const R* __restrict__ pts, const int32_t* __restrict_
 inline size_t al256(size_t b) { return (b + 255) / 256 * 256; }
 
 struct Sizes {
-    size_t rec, mom, loc, W, F, rec2;
+    size_t rec, mom, loc, W, F;
 };
-
-// The packed P2P runs for elasticRH3 in FP32 with the 3-, 4- and 7-point rules.
-template <typename R, int K, int NQ>
-constexpr bool p2p_packed() {
-    return sizeof(R) == 4 && K == kRH && (NQ == 3 || NQ == 4 || NQ == 7);
-}
 
 template <int K, int NQ>
 Sizes sizes_for(size_t rs, int mode, int order, int64_t n_obs, int64_t n_src, int64_t n_obs_nodes,
@@ -1387,9 +1154,6 @@ Sizes sizes_for(size_t rs, int mode, int order, int64_t n_obs, int64_t n_src, in
     s.loc = mode == 1 ? al256(rs * C::NCHP * (size_t)n_harm(order) * n_obs_nodes) : 0;
     s.W = al256(rs * NAcc<K, NQ>::n * (size_t)n_obs);
     s.F = al256(rs * C::NO * (size_t)NQ * n_obs);
-    s.rec2 = (rs == 4 && K == kRH && (NQ == 3 || NQ == 4 || NQ == 7))
-                 ? al256(4 * (size_t)RecRH2<NQ>::LEN * n_src)
-                 : 0;
     return s;
 }
 
@@ -1414,7 +1178,7 @@ Sizes sizes_dispatch(int kernel, int prec, int mode, int order, int nq, int64_t 
     TCT_SZ_K(kRH)
 #undef TCT_SZ_K
 #undef TCT_SZ_NQ
-    return Sizes{0, 0, 0, 0, 0, 0};
+    return Sizes{0, 0, 0, 0, 0};
 }
 
 template <typename KF>
@@ -1451,12 +1215,19 @@ inline SideStream* side_stream() {
     return &e;
 }
 
+// The plan of a planned apply (else null) and what its kernels take.
+struct P2PPart {
+    const tct_fmm_p2p_plan* plan;
+    P2PCall call;
+    int kernel, prec;
+};
+
 template <typename R, int K, int NQ>
 int run_fmm(int mode, int p, const Rule2D<R>& rule, const double* params, double scale,
             const R* obs_pts, const int32_t* obs_tris, int64_t n_obs, const tct_fmm_tree& ot,
             const R* src_pts, const int32_t* src_tris, int64_t n_src, const tct_fmm_tree& stt,
             const tct_fmm_list& near, const tct_fmm_list& far, const R* in, R* out,
-            int accumulate, unsigned char* ws, cudaStream_t st) {
+            int accumulate, unsigned char* ws, const P2PPart& p2p, cudaStream_t st) {
     using C = Chan<K>;
     constexpr int NA = NAcc<K, NQ>::n;
     const Consts<R> c = make_consts<R>(params);
@@ -1467,9 +1238,6 @@ int run_fmm(int mode, int p, const Rule2D<R>& rule, const double* params, double
     R* loc = reinterpret_cast<R*>(ws + sz.rec + sz.mom);
     R* W = reinterpret_cast<R*>(ws + sz.rec + sz.mom + sz.loc);
     R* F = reinterpret_cast<R*>(ws + sz.rec + sz.mom + sz.loc + sz.W);
-    float* rec2 = reinterpret_cast<float*>(ws + sz.rec + sz.mom + sz.loc + sz.W + sz.F);
-    bool uniform = true;
-    for (int q = 1; q < NQ; q++) uniform = uniform && (rule.w[q] == rule.w[0]);
     const R* scent = (const R*)stt.centers;
     const R* srad = (const R*)stt.radii;
     const R* ocent = (const R*)ot.centers;
@@ -1494,40 +1262,18 @@ int run_fmm(int mode, int p, const Rule2D<R>& rule, const double* params, double
     if (cudaEventRecord(side->fork, st) != cudaSuccess ||
         cudaStreamWaitEvent(se, side->fork, 0) != cudaSuccess)
         return launch_status("fmm fork");
-    if (near.n_obs > 0) {
-        if constexpr (p2p_packed<R, K, NQ>()) {
-            const Rule2D<float>& rf = rule;
-            const unsigned pb = (unsigned)((n_src + 127) / 128);
-            const size_t smem = p2p_rh2_smem<NQ>();
-            if ((rc = set_smem(fmm_p2p_rh2<NQ, true>, smem)) ||
-                (rc = set_smem(fmm_p2p_rh2<NQ, false>, smem)))
-                return rc;
-            if (uniform) {
-                far_prep_rh2<NQ, true><<<pb, 128, 0, sp>>>(c, rf, (const float*)src_pts,
-                                                            src_tris, n_src, (const float*)in,
-                                                            stt.orig, rec2);
-                if ((rc = launch_status("fmm prep (packed)"))) return rc;
-                fmm_p2p_rh2<NQ, true><<<(unsigned)near.n_obs, 128, smem, sp>>>(
-                    rf, (const float*)obs_pts, obs_tris, near.obs, near.start, near.src, ot.start,
-                    ot.end, stt.start, stt.end, rec2, (float*)W);
-            } else {
-                far_prep_rh2<NQ, false><<<pb, 128, 0, sp>>>(c, rf, (const float*)src_pts,
-                                                             src_tris, n_src, (const float*)in,
-                                                             stt.orig, rec2);
-                if ((rc = launch_status("fmm prep (packed)"))) return rc;
-                fmm_p2p_rh2<NQ, false><<<(unsigned)near.n_obs, 128, smem, sp>>>(
-                    rf, (const float*)obs_pts, obs_tris, near.obs, near.start, near.src, ot.start,
-                    ot.end, stt.start, stt.end, rec2, (float*)W);
-            }
-            if ((rc = launch_status("fmm p2p (packed)"))) return rc;
-        } else {
-            const size_t smem = sizeof(R) * 128 * NA;
-            if ((rc = set_smem(fmm_p2p<R, K, NQ>, smem))) return rc;
-            fmm_p2p<R, K, NQ><<<(unsigned)near.n_obs, 128, smem, sp>>>(
-                c, rule, obs_pts, obs_tris, near.obs, near.start, near.src, ot.start, ot.end,
-                stt.start, stt.end, rec, W);
-            if ((rc = launch_status("fmm p2p"))) return rc;
-        }
+    if (p2p.plan) {
+        P2PCall call = p2p.call;
+        call.rec = rec;
+        call.W = W;
+        if ((rc = p2p_planned(p2p.kernel, p2p.prec, NQ, call, *p2p.plan, sp))) return rc;
+    } else if (near.n_obs > 0) {
+        const size_t smem = sizeof(R) * 128 * NA;
+        if ((rc = set_smem(fmm_p2p<R, K, NQ>, smem))) return rc;
+        fmm_p2p<R, K, NQ><<<(unsigned)near.n_obs, 128, smem, sp>>>(
+            c, rule, obs_pts, obs_tris, near.obs, near.start, near.src, ot.start, ot.end,
+            stt.start, stt.end, rec, W);
+        if ((rc = launch_status("fmm p2p"))) return rc;
     }
     if (stt.n_leaves > 0) {
         const size_t smem = sizeof(R) * (size_t)p2m_reals<K>(p);
@@ -1610,10 +1356,10 @@ extern "C" size_t tct_fmm_workspace_bytes(int kernel, int prec, int mode, int or
         return 0;
     const Sizes s = sizes_dispatch(kernel, prec, mode, order, n_q, n_obs, n_src, n_obs_nodes,
                                    n_src_nodes);
-    return s.rec + s.mom + s.loc + s.W + s.F + s.rec2;
+    return s.rec + s.mom + s.loc + s.W + s.F;
 }
 
-extern "C" int tct_fmm_matvec(int kernel, int prec, int mode, int order, int n_q,
+static int fmm_matvec(int kernel, int prec, int mode, int order, int n_q,
                               const double* quad_pts, const double* quad_wts,
                               const double* params, double out_scale, const void* obs_pts,
                               const int32_t* obs_tris, int64_t n_obs,
@@ -1621,7 +1367,8 @@ extern "C" int tct_fmm_matvec(int kernel, int prec, int mode, int order, int n_q
                               const int32_t* src_tris, int64_t n_src,
                               const tct_fmm_tree* src_tree, const tct_fmm_list* p2p,
                               const tct_fmm_list* far, const void* in, void* out, int accumulate,
-                              void* workspace, size_t workspace_bytes, void* stream) {
+                              void* workspace, size_t workspace_bytes, void* stream,
+                      const tct_fmm_p2p_plan* plan) {
     TCT_CHECK_ARG(order >= 0 && order <= FMM_MAXP, "tct_fmm_matvec: order must be 0..%d",
                   FMM_MAXP);
     TCT_CHECK_ARG(mode == 0 || mode == 1, "tct_fmm_matvec: mode must be 0 (treecode) or 1 (fmm)");
@@ -1643,12 +1390,17 @@ extern "C" int tct_fmm_matvec(int kernel, int prec, int mode, int order, int n_q
                   "tct_fmm_matvec: elasticRH3 in FP64 runs FMM orders up to 10 (got %d)", order);
     TCT_CHECK_ARG(supported_nq(n_q), "tct_fmm_matvec: n_q must be 3, 4, 7 or 13 (got %d)", n_q);
     if (n_obs == 0) return TCT_OK;
-    const size_t need = tct_fmm_workspace_bytes(kernel, prec, mode, order, n_q, n_obs, n_src,
+    const size_t base = tct_fmm_workspace_bytes(kernel, prec, mode, order, n_q, n_obs, n_src,
                                                 obs_tree->n_nodes, src_tree->n_nodes);
+    const size_t need = base + (plan ? p2p_workspace_bytes(kernel, prec, n_q, n_src, *plan) : 0);
     TCT_CHECK_ARG(workspace && workspace_bytes >= need && aligned(workspace, 256),
                   "tct_fmm_matvec: workspace of %zu bytes (256-aligned) required", need);
     unsigned char* ws = reinterpret_cast<unsigned char*>(workspace);
     cudaStream_t st = as_stream(stream);
+    const P2PPart part{plan,
+                       P2PCall{quad_pts, quad_wts, params, obs_pts, obs_tris, src_pts, src_tris, n_src,
+                               src_tree->orig, in, nullptr, nullptr, ws + base},
+                       kernel, prec};
 #define TCT_FMM_NQ(R, KID, NQV)                                                                \
     if (n_q == NQV) {                                                                         \
         Rule2D<R> rule;                                                                       \
@@ -1660,7 +1412,7 @@ extern "C" int tct_fmm_matvec(int kernel, int prec, int mode, int order, int n_q
         return run_fmm<R, KID, NQV>(mode, order, rule, params, out_scale, (const R*)obs_pts, \
                                     obs_tris, n_obs, *obs_tree, (const R*)src_pts, src_tris,  \
                                     n_src, *src_tree, *p2p, *far, (const R*)in, (R*)out,      \
-                                    accumulate, ws, st);                                      \
+                                    accumulate, ws, part, st);                                \
     }
 #define TCT_FMM_K(R, KID)      \
     if (kernel == KID) {       \
@@ -1684,6 +1436,53 @@ extern "C" int tct_fmm_matvec(int kernel, int prec, int mode, int order, int n_q
 #undef TCT_FMM_NQ
     set_error("tct_fmm_matvec: unsupported kernel %d / n_q %d", kernel, n_q);
     return TCT_ERR_ARG;
+}
+
+extern "C" int tct_fmm_matvec(int kernel, int prec, int mode, int order, int n_q,
+                              const double* quad_pts, const double* quad_wts,
+                              const double* params, double out_scale, const void* obs_pts,
+                              const int32_t* obs_tris, int64_t n_obs,
+                              const tct_fmm_tree* obs_tree, const void* src_pts,
+                              const int32_t* src_tris, int64_t n_src,
+                              const tct_fmm_tree* src_tree, const tct_fmm_list* p2p,
+                              const tct_fmm_list* far, const void* in, void* out, int accumulate,
+                              void* workspace, size_t workspace_bytes, void* stream) {
+    return fmm_matvec(kernel, prec, mode, order, n_q, quad_pts, quad_wts, params, out_scale,
+                      obs_pts, obs_tris, n_obs, obs_tree, src_pts, src_tris, n_src, src_tree,
+                      p2p, far, in, out, accumulate, workspace, workspace_bytes, stream, nullptr);
+}
+
+extern "C" size_t tct_fmm_planned_workspace_bytes(int kernel, int prec, int mode, int order, int n_q,
+                                                  int64_t n_obs, int64_t n_src,
+                                                  int64_t n_obs_nodes, int64_t n_src_nodes,
+                                                  const tct_fmm_p2p_plan* plan) {
+    const size_t base = tct_fmm_workspace_bytes(kernel, prec, mode, order, n_q, n_obs, n_src,
+                                                n_obs_nodes, n_src_nodes);
+    return base && plan ? base + p2p_workspace_bytes(kernel, prec, n_q, n_src, *plan) : 0;
+}
+
+extern "C" int tct_fmm_matvec_planned(int kernel, int prec, int mode, int order, int n_q,
+                              const double* quad_pts, const double* quad_wts,
+                              const double* params, double out_scale, const void* obs_pts,
+                              const int32_t* obs_tris, int64_t n_obs,
+                              const tct_fmm_tree* obs_tree, const void* src_pts,
+                              const int32_t* src_tris, int64_t n_src,
+                              const tct_fmm_tree* src_tree, const tct_fmm_list* p2p,
+                              const tct_fmm_list* far, const void* in, void* out, int accumulate,
+                              void* workspace, size_t workspace_bytes, void* stream,
+                                      const tct_fmm_p2p_plan* plan) {
+    TCT_CHECK_ARG(plan, "tct_fmm_matvec_planned: null plan");
+    TCT_CHECK_ARG(plan->n_tasks >= 0 && plan->n_chunks >= 0 && plan->n_slots >= 0 &&
+                      (plan->n_tasks == 0 || (plan->tasks && plan->entries && plan->chunks)) &&
+                      (plan->n_slots == 0 || plan->slots_in),
+                  "tct_fmm_matvec_planned: bad plan");
+    TCT_CHECK_ARG(plan->chunk == (prec == TCT_F32 && p2p_is_rh(kernel, n_q) ? 64 : 32),
+                  "tct_fmm_matvec_planned: plan chunk %d", plan->chunk);
+    TCT_CHECK_ARG(!plan->sym || p2p_is_rh(kernel, n_q),
+                  "tct_fmm_matvec_planned: symmetric plan for kernel %d", kernel);
+    return fmm_matvec(kernel, prec, mode, order, n_q, quad_pts, quad_wts, params, out_scale,
+                      obs_pts, obs_tris, n_obs, obs_tree, src_pts, src_tris, n_src, src_tree,
+                      p2p, far, in, out, accumulate, workspace, workspace_bytes, stream, plan);
 }
 
 namespace tct {

@@ -1,0 +1,439 @@
+// The FMM's and treecode's near leaves (P2P) on a work plan.
+//
+// The plan (fmm/p2p_plan.py) cuts the interaction list into tasks of one
+// chunk of an observation leaf (at most 64 triangles for the packed FP32
+// elasticRH3 kernel, 32 otherwise) against about a thousand source triangles
+// of its list entries, so that blocks do about the same work whatever the
+// leaves' sizes; fmm_p2p (fmm.cu) gives a leaf's whole list to one block.
+// A block's four warps share the chunk and take a quarter of every staged
+// tile of 64 sources each.
+//
+// elasticRH3 on a symmetric list (the same tree on both sides): an unordered
+// leaf pair is one entry, its geometry formed once for both directions
+// (rh_sym.cuh); the contribution to the sources goes to the entry's slots, and
+// the last kernel adds a triangle's task sums and slots in plan order in
+// double (no atomics: the same bits every run, and for every row shard).
+// Bound by the FMA pipe (elasticRH3) or the kernel's own arithmetic, at the
+// leaves' filling of the chunks (mean leaf 59 triangles: about 70 % of the
+// lanes).  elasticRH3, FP32 3-point rule, 119,656 triangles, 1.54e9 listed pairs:
+// 32.8 ms with a block per leaf (packed, one-sided), 11.2 ms here; FP64 4-point
+// rule, 72,200 triangles, 7.3e8 pairs: 127 ms (one triangle a lane, records
+// through L1), 18.0 ms.  The whole applies: 37.4 -> 13.6 and 145.7 -> 23.3 ms.
+#include "fmm_p2p.h"
+#include "rh_sym.cuh"
+
+namespace tct {
+namespace {
+
+constexpr int P2P_TILE = 64;     // staged sources
+constexpr int P2P_MAXE = 128;    // most entries of a task
+
+struct P2PArgs {
+    const int32_t* tasks;    // first obs triangle, count, first and end entry
+    const int32_t* entries;  // first source triangle, count, first slot or -1
+};
+
+// The task's entries in shared memory: position of the first source of entry e
+// in the concatenated sources, its first triangle and slot.
+struct P2PTable {
+    int pos[P2P_MAXE + 1], src[P2P_MAXE], slot[P2P_MAXE];
+};
+
+__device__ __forceinline__ void load_table(P2PTable& t, const int32_t* __restrict__ entries, int e0,
+                                           int ne) {
+    for (int e = threadIdx.x; e < ne; e += blockDim.x) {
+        t.src[e] = entries[3 * (e0 + e)];
+        t.pos[e + 1] = entries[3 * (e0 + e) + 1];
+        t.slot[e] = entries[3 * (e0 + e) + 2];
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int s = 0;
+        t.pos[0] = 0;
+        for (int e = 0; e < ne; e++) {
+            s += t.pos[e + 1];
+            t.pos[e + 1] = s;
+        }
+    }
+    __syncthreads();
+}
+
+// Entry of source position p.
+__device__ __forceinline__ int find_entry(const P2PTable& t, int ne, int p) {
+    int lo = 0, hi = ne - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (t.pos[mid] <= p) lo = mid;
+        else hi = mid - 1;
+    }
+    return lo;
+}
+
+template <class V, int NQ, bool UNIFORM, bool SYM>
+__global__ void __launch_bounds__(128, V::H == 2 && NQ == 7 ? 2 : 3)
+p2p_rh(P2PArgs a, PairWeights<V, NQ> pw, Rule2D<typename V::real> rule,
+       const typename V::real* __restrict__ opts, const int32_t* __restrict__ otris,
+       const typename V::vec* __restrict__ rec, typename V::real* __restrict__ Wp,
+       typename V::real* __restrict__ Vp) {
+    using R = typename V::real;
+    using vec = typename V::vec;
+    using L = RecSelf<NQ>;
+    constexpr int CH = 32 * V::H;
+    __shared__ P2PTable tab;
+    __shared__ int srcs[P2P_TILE], slots[P2P_TILE];
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    vec* sm = reinterpret_cast<vec*>(smem_raw);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int64_t o0 = a.tasks[4 * (int64_t)blockIdx.x];
+    const int cnt = a.tasks[4 * (int64_t)blockIdx.x + 1];
+    const int e0 = a.tasks[4 * (int64_t)blockIdx.x + 2];
+    const int ne = a.tasks[4 * (int64_t)blockIdx.x + 3] - e0;
+    load_table(tab, a.entries, e0, ne);
+    const int ns = tab.pos[ne];
+
+    // a chunk of at most half the lanes' triangles: the half-warps hold the
+    // same triangles and take different sources
+    const bool halves = cnt <= CH / 2;
+    const int li = halves ? lane & 15 : lane, step = halves ? 16 : 32;
+    const bool va = li < cnt, vb = V::H == 2 && li + step < cnt;
+    vec negx[NQ][3], S[18], tot[9];
+    {
+        TriGeom<R> oa, ob;
+        if (va) load_tri(oa, opts, otris, o0 + li, 0, false, false);
+        if (vb) load_tri(ob, opts, otris, o0 + li + step, 0, false, false);
+#pragma unroll
+        for (int q = 0; q < NQ; q++) {
+            const R ox = rule.x[q], oy = rule.y[q];
+            const R bq[3] = {1 - ox - oy, ox, oy};
+#pragma unroll
+            for (int d = 0; d < 3; d++)
+                negx[q][d] = V::make(va ? -bary_point(oa, bq, d) : R(0),
+                                     vb ? -bary_point(ob, bq, d) : R(0));
+        }
+        if (SYM) {
+            const R* pa = reinterpret_cast<const R*>(rec + (o0 + (va ? li : 0)) * L::LEN);
+            const R* pb = reinterpret_cast<const R*>(rec + (o0 + (vb ? li + step : 0)) * L::LEN);
+#pragma unroll
+            for (int k = 0; k < 18; k++)
+                S[k] = V::make(va ? pa[V::H * (L::P + k)] : R(0), vb ? pb[V::H * (L::P + k)] : R(0));
+        }
+#pragma unroll
+        for (int k = 0; k < 9; k++) tot[k] = V::make(0, 0);
+    }
+    for (int t0 = 0; t0 < ns; t0 += P2P_TILE) {
+        const int nt = min(P2P_TILE, ns - t0);
+        __syncthreads();
+        if (tid < P2P_TILE) {
+            int s = -1, v = -1;
+            if (tid < nt) {
+                const int e = find_entry(tab, ne, t0 + tid), off = t0 + tid - tab.pos[e];
+                s = tab.src[e] + off;
+                v = tab.slot[e] < 0 ? -1 : tab.slot[e] + off;
+            }
+            srcs[tid] = s;
+            slots[tid] = v;
+        }
+        __syncthreads();
+        {
+            constexpr int V2 = L::LEN / 2;
+            ulonglong2* dstv = reinterpret_cast<ulonglong2*>(sm);
+            // an odd last source is paired with one of zero points and input
+            for (int k = tid; k < ((nt + 1) & ~1) * V2; k += 128) {
+                const int j = k / V2, s = srcs[j];
+                dstv[k] = s < 0 ? make_ulonglong2(0ull, 0ull)
+                                : __ldg(reinterpret_cast<const ulonglong2*>(rec + (int64_t)s * L::LEN) +
+                                        (k - j * V2));
+            }
+        }
+        __syncthreads();
+        vec W[9];
+#pragma unroll
+        for (int k = 0; k < 9; k++) W[k] = V::make(0, 0);
+        const int j1 = min(nt, 16 * warp + 16);
+#pragma unroll 1
+        for (int j = 16 * warp; j < j1; j += 2) {
+            R s[2][9], lo, hi;
+            const int np = halves ? 1 : 2;
+#pragma unroll
+            for (int u = 0; u < 2; u++) {
+                if (u < np) {
+                    vec T[6], pm[18];
+                    const vec* r = sm + (j + (halves ? lane >> 4 : u)) * L::LEN;
+                    self_tensor<V, NQ, UNIFORM>(r, negx, pw, T);
+                    const vec S0 = V::add(V::add(T[0], T[3]), T[5]);
+                    self_load_pm<V, NQ>(r, pm);
+                    self_apply<V>(T, S0, pm, W);
+                    if (SYM) {
+                        vec v[9];
+#pragma unroll
+                        for (int k = 0; k < 9; k++) v[k] = V::make(0, 0);
+                        self_apply<V>(T, S0, S, v);
+#pragma unroll
+                        for (int k = 0; k < 9; k++) s[u][k] = V::hsum(v[k]);
+                    }
+                }
+            }
+            if (SYM) {
+                if (halves) half_sum9<R>(s[0], lane, lo, hi);
+                else warp_sum2x9<R>(s[0], s[1], lane, lo, hi);
+                const int slot = slots[j + (lane >> 4)];
+                if (slot >= 0) {
+                    R* vo = Vp + (int64_t)slot * 9;
+                    if ((lane & 1) == 0) vo[(lane >> 1) & 7] = lo;
+                    if ((lane & 15) == 0) vo[8] = hi;
+                }
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 9; k++) tot[k] = V::add(tot[k], W[k]);
+    }
+    // the warps' (half-warps') sums in a fixed order
+    R* red = reinterpret_cast<R*>(smem_raw);  // 4 x CH x 9
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 9; k++) {
+        R o[V::H];
+        V::split(tot[k], o);
+        // lane's values at (half, triangle): halves hold CH / 2 triangles each
+        const int base = warp * CH + (halves ? (lane >> 4) * (CH / 2) : 0) + li;
+        red[base * 9 + k] = o[0];
+        if (V::H == 2) red[(base + step) * 9 + k] = o[V::H - 1];
+    }
+    __syncthreads();
+    R* wo = Wp + (int64_t)blockIdx.x * CH * 9;
+    for (int e = tid; e < cnt * 9; e += 128) {
+        R s = 0;
+#pragma unroll
+        for (int w = 0; w < 4; w++) {
+            s += red[w * CH * 9 + e];
+            if (halves) s += red[(w * CH + CH / 2) * 9 + e];
+        }
+        wo[e] = s;
+    }
+}
+
+// Any other kernel or rule: the direct farfield's one-sided pair loop
+// (far_pair), one observation triangle a lane.
+template <typename R, int K, int NQ>
+__global__ void __launch_bounds__(128)
+p2p_any(P2PArgs a, Consts<R> c, Rule2D<R> rule, const R* __restrict__ opts,
+        const int32_t* __restrict__ otris, const R* __restrict__ rec, R* __restrict__ Wp) {
+    using L = Rec<K, NQ>;
+    constexpr int NA = NAcc<K, NQ>::n, CH = 32;
+    __shared__ P2PTable tab;
+    __shared__ int srcs[P2P_TILE];
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    R* sm = reinterpret_cast<R*>(smem_raw);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int64_t o0 = a.tasks[4 * (int64_t)blockIdx.x];
+    const int cnt = a.tasks[4 * (int64_t)blockIdx.x + 1];
+    const int e0 = a.tasks[4 * (int64_t)blockIdx.x + 2];
+    const int ne = a.tasks[4 * (int64_t)blockIdx.x + 3] - e0;
+    load_table(tab, a.entries, e0, ne);
+    const int ns = tab.pos[ne];
+    // a chunk of at most 16 triangles: the half-warps take different sources
+    const bool halves = cnt <= CH / 2;
+    const int li = halves ? lane & 15 : lane;
+    const bool valid = li < cnt;
+    TriGeom<R> o;
+    load_tri(o, opts, otris, o0 + (valid ? li : 0), 0, false, K == kRA || K == kRH);
+    R x[NQ][3];
+#pragma unroll
+    for (int q = 0; q < NQ; q++) {
+        const R ox = rule.x[q], oy = rule.y[q];
+        const R bq[3] = {1 - ox - oy, ox, oy};
+#pragma unroll
+        for (int d = 0; d < 3; d++) x[q][d] = bary_point(o, bq, d);
+    }
+    R tot[NA];
+#pragma unroll
+    for (int k = 0; k < NA; k++) tot[k] = 0;
+    for (int t0 = 0; t0 < ns; t0 += P2P_TILE) {
+        const int nt = min(P2P_TILE, ns - t0);
+        __syncthreads();
+        if (tid < nt) {
+            const int e = find_entry(tab, ne, t0 + tid);
+            srcs[tid] = tab.src[e] + (t0 + tid - tab.pos[e]);
+        }
+        __syncthreads();
+        {
+            constexpr int PER = 16 / sizeof(R), V2 = L::LEN / PER;
+            ulonglong2* dstv = reinterpret_cast<ulonglong2*>(sm);
+            for (int k = tid; k < nt * V2; k += 128) {
+                const int j = k / V2;
+                dstv[k] = __ldg(reinterpret_cast<const ulonglong2*>(rec + (int64_t)srcs[j] * L::LEN) +
+                                (k - j * V2));
+            }
+        }
+        __syncthreads();
+        R acc[NA];
+#pragma unroll
+        for (int k = 0; k < NA; k++) acc[k] = 0;
+        const int j1 = min(nt, 16 * warp + 16), by = halves ? 2 : 1;
+#pragma unroll 1
+        for (int j = 16 * warp + (halves ? lane >> 4 : 0); j < j1; j += by)
+            far_pair<R, K, NQ>(c, rule, o, x, sm + j * L::LEN, acc);
+#pragma unroll
+        for (int k = 0; k < NA; k++) tot[k] += acc[k];
+    }
+    // the warps' (half-warps') sums in a fixed order
+    __syncthreads();
+    const int base = warp * CH + (halves ? (lane >> 4) * (CH / 2) : 0) + li;
+#pragma unroll
+    for (int k = 0; k < NA; k++) sm[base * NA + k] = tot[k];
+    __syncthreads();
+    R* wo = Wp + (int64_t)blockIdx.x * CH * NA;
+    for (int e = tid; e < cnt * NA; e += 128) {
+        R s = 0;
+#pragma unroll
+        for (int w = 0; w < 4; w++) {
+            s += sm[w * CH * NA + e];
+            if (halves) s += sm[(w * CH + CH / 2) * NA + e];
+        }
+        wo[e] = s;
+    }
+}
+
+// A chunk's sums: its tasks' and its slots', in plan order, in double.
+template <typename R>
+__global__ void __launch_bounds__(256)
+p2p_reduce(const int32_t* __restrict__ chunks, const int32_t* __restrict__ vin, int na, int ch,
+           const R* __restrict__ Wp, const R* __restrict__ Vp, R* __restrict__ W) {
+    const int32_t* c = chunks + 7 * (int64_t)blockIdx.x;
+    const int64_t o0 = c[0];
+    const int cnt = c[1], t0 = c[2], t1 = c[3], v0 = c[4], v1 = c[5], off = c[6];
+    for (int e = threadIdx.x; e < cnt * na; e += blockDim.x) {
+        double s = 0;
+        for (int t = t0; t < t1; t++) s += (double)Wp[(int64_t)t * ch * na + e];
+#pragma unroll 8
+        for (int v = v0; v < v1; v++) s += (double)Vp[(int64_t)(vin[v] + off) * na + e];
+        W[o0 * na + e] = (R)s;
+    }
+}
+
+inline size_t al256(size_t b) { return (b + 255) / 256 * 256; }
+
+template <typename KF>
+int smem_limit(KF kfn, size_t smem) {
+    if (smem > 48 * 1024 &&
+        cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
+            cudaSuccess)
+        return launch_status("p2p shared-memory attribute");
+    return TCT_OK;
+}
+
+template <class V, int NQ, bool UNIFORM>
+int run_rh(const P2PCall& k, const tct_fmm_p2p_plan& plan, cudaStream_t st) {
+    using R = typename V::real;
+    using vec = typename V::vec;
+    using L = RecSelf<NQ>;
+    const Consts<R> c = make_consts<R>(k.params);
+    Rule2D<R> rule;
+    PairWeights<V, NQ> pw;
+    self_rule<V, NQ>(k.qp, k.qw, rule, pw);
+    vec* rec = reinterpret_cast<vec*>(k.ws);
+    R* Wp = reinterpret_cast<R*>(k.ws + al256(8 * (size_t)L::LEN * k.n_src));
+    R* Vp = Wp + plan.n_tasks * plan.chunk * 9;
+    far_self_prep<V, NQ, UNIFORM><<<(unsigned)((k.n_src + 127) / 128), 128, 0, st>>>(
+        c, rule, (const R*)k.src_pts, k.src_tris, k.n_src, (const R*)k.in, k.src_orig, rec);
+    int rc = launch_status("p2p prep");
+    if (rc) return rc;
+    const P2PArgs a{plan.tasks, plan.entries};
+    const size_t smem = std::max(sizeof(vec) * L::LEN * (size_t)P2P_TILE,
+                                 sizeof(R) * 4 * 32 * V::H * 9);
+    if (plan.sym)
+        p2p_rh<V, NQ, UNIFORM, true><<<(unsigned)plan.n_tasks, 128, smem, st>>>(
+            a, pw, rule, (const R*)k.obs_pts, k.obs_tris, rec, Wp, Vp);
+    else
+        p2p_rh<V, NQ, UNIFORM, false><<<(unsigned)plan.n_tasks, 128, smem, st>>>(
+            a, pw, rule, (const R*)k.obs_pts, k.obs_tris, rec, Wp, Vp);
+    if ((rc = launch_status("p2p (elasticRH3)"))) return rc;
+    p2p_reduce<R><<<(unsigned)plan.n_chunks, 256, 0, st>>>(plan.chunks, plan.slots_in, 9, plan.chunk,
+                                                          Wp, Vp, (R*)k.W);
+    return launch_status("p2p reduce");
+}
+
+template <typename R, int K, int NQ>
+int run_any(const P2PCall& k, const tct_fmm_p2p_plan& plan, cudaStream_t st) {
+    using L = Rec<K, NQ>;
+    constexpr int NA = NAcc<K, NQ>::n;
+    const Consts<R> c = make_consts<R>(k.params);
+    Rule2D<R> rule;
+    for (int q = 0; q < MAXQ; q++) {
+        rule.x[q] = q < NQ ? (R)k.qp[2 * q] : R(0);
+        rule.y[q] = q < NQ ? (R)k.qp[2 * q + 1] : R(0);
+        rule.w[q] = q < NQ ? (R)k.qw[q] : R(0);
+    }
+    R* Wp = reinterpret_cast<R*>(k.ws);
+    const P2PArgs a{plan.tasks, plan.entries};
+    const size_t smem = sizeof(R) * std::max((size_t)L::LEN * P2P_TILE, (size_t)4 * 32 * NA);
+    int rc = smem_limit(p2p_any<R, K, NQ>, smem);
+    if (rc) return rc;
+    p2p_any<R, K, NQ><<<(unsigned)plan.n_tasks, 128, smem, st>>>(
+        a, c, rule, (const R*)k.obs_pts, k.obs_tris, (const R*)k.rec, Wp);
+    if ((rc = launch_status("p2p"))) return rc;
+    p2p_reduce<R><<<(unsigned)plan.n_chunks, 256, 0, st>>>(plan.chunks, plan.slots_in, NA, plan.chunk,
+                                                          Wp, nullptr, (R*)k.W);
+    return launch_status("p2p reduce");
+}
+
+template <typename R>
+int any_dispatch(int kernel, int nq, const P2PCall& k, const tct_fmm_p2p_plan& plan,
+                 cudaStream_t st) {
+#define TCT_P2P_NQ(KID, NQV) \
+    if (nq == NQV) return run_any<R, KID, NQV>(k, plan, st);
+#define TCT_P2P_K(KID)      \
+    if (kernel == KID) {    \
+        TCT_P2P_NQ(KID, 3)  \
+        TCT_P2P_NQ(KID, 4)  \
+        TCT_P2P_NQ(KID, 7)  \
+        TCT_P2P_NQ(KID, 13) \
+    }
+    TCT_P2P_K(kU)
+    TCT_P2P_K(kRT)
+    TCT_P2P_K(kRA)
+    if (kernel == kRH) {
+        TCT_P2P_NQ(kRH, 13)
+    }
+#undef TCT_P2P_K
+#undef TCT_P2P_NQ
+    set_error("p2p: unsupported kernel %d / n_q %d", kernel, nq);
+    return TCT_ERR_ARG;
+}
+
+template <class V>
+int rh_dispatch(int nq, const P2PCall& k, const tct_fmm_p2p_plan& plan, cudaStream_t st) {
+    bool uniform = true;
+    for (int q = 1; q < nq; q++) uniform = uniform && k.qw[q] == k.qw[0];
+    if (nq == 3 && uniform) return run_rh<V, 3, true>(k, plan, st);
+    if (nq == 3) return run_rh<V, 3, false>(k, plan, st);
+    if (nq == 4) return run_rh<V, 4, false>(k, plan, st);
+    return run_rh<V, 7, false>(k, plan, st);
+}
+
+}  // namespace
+
+// elasticRH3 with a 3-, 4- or 7-point rule.
+bool p2p_is_rh(int kernel, int nq) { return kernel == kRH && self_rec_len(nq) > 0; }
+
+size_t p2p_workspace_bytes(int kernel, int prec, int nq, int64_t n_src,
+                           const tct_fmm_p2p_plan& plan) {
+    const size_t rs = prec == TCT_F64 ? 8 : 4;
+    if (p2p_is_rh(kernel, nq))
+        return al256(8 * (size_t)self_rec_len(nq) * n_src) +
+               al256(rs * 9 * ((size_t)plan.n_tasks * plan.chunk + (size_t)plan.n_slots));
+    const size_t na = kernel == kRH ? 9 : (kernel == kRA ? 3 * nq + 3 : 3 * nq);
+    return al256(rs * na * (size_t)plan.n_tasks * plan.chunk);
+}
+
+int p2p_planned(int kernel, int prec, int nq, const P2PCall& k, const tct_fmm_p2p_plan& plan,
+                cudaStream_t st) {
+    if (plan.n_tasks == 0) return TCT_OK;
+    if (p2p_is_rh(kernel, nq))
+        return prec == TCT_F32 ? rh_dispatch<VecF32>(nq, k, plan, st)
+                               : rh_dispatch<VecF64>(nq, k, plan, st);
+    return prec == TCT_F32 ? any_dispatch<float>(kernel, nq, k, plan, st)
+                           : any_dispatch<double>(kernel, nq, k, plan, st);
+}
+
+}  // namespace tct

@@ -1,0 +1,135 @@
+"""Work plan of the P2P kernels (csrc/fmm_p2p.cu): the near list of a tree pair
+cut into tasks of about equal work.
+
+An observation node of m triangles is cut into ceil(m / chunk) chunks of equal
+size; a chunk's list entries, in list order, are cut into tasks where the
+sources passed reach a multiple of about a thousand (or 128 entries).  On a
+symmetric list (one tree on both sides, leaves only: the FMM's) an unordered
+leaf pair keeps one entry: the kernel adds both directions, the sources' side
+into the entry's slots, one per source triangle.  Which leaf takes the lanes
+alternates with the parity of the two node indices, so that all leaves keep
+about half of their entries.
+
+Row shards (`keep`): the tasks are cut on the whole list; a kept node's tasks
+stay whole, of the others the entries whose source is kept stay, so a kept
+row's sums hold the same terms in the same order as without sharding.
+"""
+import numpy as np
+
+from ..util import device
+
+# most slots (one per source triangle of a symmetric entry and chunk), and the
+# bytes they may take; beyond, every ordered pair keeps its own entry
+MAX_SLOTS = 2 ** 31 - 1
+MAX_SLOT_BYTES = 8 << 30
+MAX_TASK_ENTRIES = 128
+
+
+class P2PPlan:
+    """Device arrays tasks (n, 4), entries (n, 3), chunks (n, 7), slots_in
+    (int32, layouts in include/tct_b200.h) and their counts."""
+
+    def __init__(self, sym, chunk, n_slots, tasks, entries, chunks, slots_in):
+        self.sym, self.chunk, self.n_slots = bool(sym), int(chunk), int(n_slots)
+        self.tasks, self.entries, self.chunks, self.slots_in = tasks, entries, chunks, slots_in
+
+
+def build(obs_tree, src_tree, lst, chunk, want_sym, slot_bytes, keep=None, dev="cuda"):
+    """The plan of the near list `lst` (a CompressedList over the two trees);
+    want_sym: the kernel can add both directions (needs the same tree);
+    slot_bytes: bytes of one slot; keep: boolean per obs node (row shards)."""
+    t = device.torch()
+
+    def up(a):
+        return t.as_tensor(np.ascontiguousarray(a, dtype=np.int64), device=dev)
+
+    ostart, osize = up(obs_tree.start), up(obs_tree.end) - up(obs_tree.start)
+    sstart, ssize = up(src_tree.start), up(src_tree.end) - up(src_tree.start)
+    group, first = up(lst.obs_n_idxs), up(lst.obs_src_starts)
+    src = up(lst.src_n_idxs)
+    n_nodes = max(int(osize.numel()), int(ssize.numel()))
+    own = t.repeat_interleave(group, first[1:] - first[:-1])
+    gid = t.repeat_interleave(t.arange(group.numel(), device=dev), first[1:] - first[:-1])
+    use = (osize[own] > 0) & (ssize[src] > 0)
+    own, gid, src = own[use], gid[use], src[use]
+
+    sym = bool(want_sym) and obs_tree is src_tree
+    if sym:
+        leaf = t.zeros(n_nodes, dtype=t.bool, device=dev)
+        leaf[up(obs_tree.leaves())] = True
+        fwd, _ = t.sort(own * n_nodes + src)
+        rev, _ = t.sort(src * n_nodes + own)
+        sym = bool(leaf[own].all()) and bool(t.equal(fwd, rev)) and \
+            bool((fwd[1:] != fwd[:-1]).all())
+    nch = (osize + chunk - 1) // chunk
+    if sym:
+        side = t.where((own + src) % 2 == 0, own <= src, own >= src)
+        slots = int((ssize[src] * nch[own])[side & (own != src)].sum())
+        if slots > MAX_SLOTS or slots * slot_bytes > MAX_SLOT_BYTES:
+            sym = False
+        else:
+            own, gid, src = own[side], gid[side], src[side]
+
+    # (group, chunk) pairs, and their rows: every entry of the group
+    cs = (osize + nch.clamp(min=1) - 1) // nch.clamp(min=1)
+    g_n = nch[group]
+    gc_g = t.repeat_interleave(t.arange(group.numel(), device=dev), g_n)
+    gc_c = t.arange(gc_g.numel(), device=dev) - t.repeat_interleave(t.cumsum(g_n, 0) - g_n, g_n)
+    n_e = t.bincount(gid, minlength=max(int(group.numel()), 1))[:group.numel()]
+    e_first = t.cumsum(n_e, 0) - n_e
+    rows_n = n_e[gc_g]
+    row0 = t.cumsum(rows_n, 0) - rows_n
+    r_gc = t.repeat_interleave(t.arange(gc_g.numel(), device=dev), rows_n)
+    r_i = t.arange(r_gc.numel(), device=dev) - row0[r_gc]
+    r_e = e_first[gc_g[r_gc]] + r_i
+    r_own, r_src = own[r_e], src[r_e]
+    r_n = ssize[r_src]
+    # tasks: about eight for each of three blocks an SM, 128 to 1,024 sources
+    total = int(r_n.sum()) if r_n.numel() else 0
+    size = min(max(total // (148 * 3 * 8), 128), 1024)
+    before = t.cumsum(r_n, 0) - r_n
+    base = before[row0.clamp(max=max(r_gc.numel() - 1, 0))][r_gc] if r_gc.numel() else before
+    cut = (before - base) // size * (1 << 20) + r_i // MAX_TASK_ENTRIES
+    new = t.ones(r_gc.numel(), dtype=t.bool, device=dev)
+    if r_gc.numel() > 1:
+        new[1:] = (r_gc[1:] != r_gc[:-1]) | (cut[1:] != cut[:-1])
+    r_task = t.cumsum(new.long(), 0) - 1
+    gc_keep = t.ones(gc_g.numel(), dtype=t.bool, device=dev)
+    if keep is not None:
+        k = t.as_tensor(np.asarray(keep, dtype=bool), device=dev)
+        gc_keep = k[group[gc_g]]
+        stay = gc_keep[r_gc]
+        if sym:
+            stay = stay | k[r_src]
+        r_gc, r_own, r_src, r_n, r_task = (a[stay] for a in (r_gc, r_own, r_src, r_n, r_task))
+        _, r_task = t.unique_consecutive(r_task, return_inverse=True)
+
+    n_rows = r_gc.numel()
+    n_tasks = int(r_task[-1]) + 1 if n_rows else 0
+    both = (r_own != r_src) if sym else t.zeros(n_rows, dtype=t.bool, device=dev)
+    cnt = t.where(both, r_n, t.zeros_like(r_n))
+    slot = t.cumsum(cnt, 0) - cnt
+    entries = t.stack([sstart[r_src], r_n, t.where(both, slot, t.full_like(slot, -1))], dim=1)
+    rows_of = t.bincount(r_task, minlength=max(n_tasks, 1))[:n_tasks]
+    t_end = t.cumsum(rows_of, 0)
+    t_first = t_end - rows_of
+    t_gc = r_gc[t_first] if n_tasks else r_gc
+    gc_own = group[gc_g]
+    gc_start = ostart[gc_own] + gc_c * cs[gc_own]
+    gc_cnt = t.minimum(cs[gc_own], osize[gc_own] - gc_c * cs[gc_own]).clamp(min=0)
+    tasks = t.stack([gc_start[t_gc], gc_cnt[t_gc], t_first, t_end], dim=1)
+    # chunks: their tasks and the slots that hold sums for their node
+    k_gc = t.nonzero(gc_keep & (gc_cnt > 0)).flatten()
+    b_rows = t.nonzero(both).flatten()
+    b_node, order = t.sort(r_src[b_rows], stable=True)
+    slots_in = slot[b_rows[order]]
+    node = gc_own[k_gc]
+    chunks = t.stack([gc_start[k_gc], gc_cnt[k_gc],
+                      t.searchsorted(t_gc.contiguous(), k_gc),
+                      t.searchsorted(t_gc.contiguous(), k_gc, right=True),
+                      t.searchsorted(b_node.contiguous(), node),
+                      t.searchsorted(b_node.contiguous(), node, right=True),
+                      gc_c[k_gc] * cs[node]], dim=1)
+    i32 = lambda a: a.to(t.int32).contiguous()  # noqa: E731
+    return P2PPlan(sym, chunk, int(cnt.sum()) if n_rows else 0, i32(tasks), i32(entries),
+                   i32(chunks), i32(slots_in))

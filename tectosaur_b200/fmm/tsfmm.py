@@ -24,6 +24,7 @@ from .. import _lib
 from ..kernels import kernels
 from ..util import device
 from ..util.quadrature import gauss2d_tri
+from . import p2p_plan
 from .tree import CompressedList, Tree, interactions, tri_centers_radii
 
 SUPPORTED = ("elasticU3", "elasticRT3", "elasticRA3", "elasticRH3")
@@ -90,6 +91,7 @@ class TSFMM:
             lists = interactions(self.obs_tree, self.src_tree, mac, mac, 0, False)
             far = lists["m2l"]
         self.obs_rows = obs_rows
+        near = lists["p2p"]  # of the whole observation set: the P2P plan is cut on it
         touch = None
         if obs_rows is not None:
             touch = touching_nodes(self.obs_tree, int(obs_rows[0]), int(obs_rows[1]))
@@ -121,16 +123,30 @@ class TSFMM:
         self.obs_desc, self._obs_off = self._tree_desc(self.obs_tree, dev, ft, obs=True,
                                                        keep=touch)
         self.src_desc, self._src_off = self._tree_desc(self.src_tree, dev, ft, obs=False)
-        self.p2p_desc = self._list_desc(self.p2p, dev)
         self.far_desc = self._list_desc(far, dev)
+        self._plan_p2p(near)
         self.n_obs = np.asarray(obs_m[1]).shape[0]
         self.n_src = np.asarray(src_m[1]).shape[0]
-        self.ws_bytes = _lib.lib.tct_fmm_workspace_bytes(
+        self.ws_bytes = int(_lib.lib.tct_fmm_planned_workspace_bytes(
             self.kid, self.prec, MODES[mode], self.order, self.nq, self.n_obs, self.n_src,
-            self.obs_tree.n_nodes, self.src_tree.n_nodes)
+            self.obs_tree.n_nodes, self.src_tree.n_nodes, ctypes.byref(self.plan_desc)))
         if self.ws_bytes == 0:
             raise ValueError("unsupported treecode configuration (rule of %d points)" % self.nq)
         self.workspace = device.workspace(self.ws_bytes)
+
+    def _plan_p2p(self, near):
+        """Cut the near list into the P2P kernels' tasks (p2p_plan.py)."""
+        rh = self.K.name == "elasticRH3" and self.nq in (3, 4, 7)
+        f32 = self.prec == _lib.TCT_F32
+        plan = p2p_plan.build(self.obs_tree, self.src_tree, near, 64 if rh and f32 else 32, rh,
+                              9 * self.float_type.itemsize, keep=self.touch)
+        self.p2p_plan = plan
+        self.p2p_desc = _lib.FmmList()  # the plan stands for the list
+        self.plan_desc = _lib.FmmP2PPlan(
+            n_tasks=plan.tasks.shape[0], n_chunks=plan.chunks.shape[0], n_slots=plan.n_slots,
+            chunk=plan.chunk, sym=int(plan.sym), tasks=_lib.tptr(plan.tasks),
+            entries=_lib.tptr(plan.entries), chunks=_lib.tptr(plan.chunks),
+            slots_in=_lib.tptr(plan.slots_in))
 
     @staticmethod
     def _tree_desc(tree, dev, ft, obs, keep=None):
@@ -172,14 +188,14 @@ class TSFMM:
     def dot_device(self, x, y, scale=1.0, accumulate=False, stream=None):
         """y (+)= scale * farfield(x) for device tensors in original order."""
         t = _lib.tptr
-        _lib.check(_lib.lib.tct_fmm_matvec(
+        _lib.check(_lib.lib.tct_fmm_matvec_planned(
             self.kid, self.prec, MODES[self.mode], self.order, self.nq, _lib.dptr(self.qx),
             _lib.dptr(self.qw), _lib.dptr(self.params), float(scale), t(self.obs_pts),
             t(self.obs_tris), self.n_obs, ctypes.byref(self.obs_desc), t(self.src_pts),
             t(self.src_tris), self.n_src, ctypes.byref(self.src_desc),
             ctypes.byref(self.p2p_desc), ctypes.byref(self.far_desc), t(x), t(y),
-            int(bool(accumulate)), t(self.workspace), self.ws_bytes, _lib.stream_ptr(stream)),
-            "tct_fmm_matvec")
+            int(bool(accumulate)), t(self.workspace), self.ws_bytes, _lib.stream_ptr(stream),
+            ctypes.byref(self.plan_desc)), "tct_fmm_matvec_planned")
         return y
 
     def dot(self, v):

@@ -1,0 +1,70 @@
+"""The planned P2P (csrc/fmm_p2p.cu) against the unplanned entry point's
+(tct_fmm_matvec: one block per leaf, the direct farfield's pair loop) inside
+whole applies with the same expansions: leaf sizes around the lanes' halves and
+the chunks, every kernel, rules, one mesh and two, trees of both modes."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from tectosaur_b200 import _lib
+from tectosaur_b200.fmm.tsfmm import MODES, TSFMM
+from tectosaur_b200.util import device
+
+from helpers import bumpy_mesh, rel
+
+pytestmark = pytest.mark.gpu
+
+# both sides sum the same n terms in FP32 partial sums of at most a few
+# hundred (the planned totals are added in double)
+TOL = {np.float32: 4 * np.sqrt(256) * 6e-8, np.float64: 4 * np.sqrt(256) * 1.2e-16}
+
+
+def _unplanned(f, x):
+    keep = []
+
+    def dev(a, dt=None):
+        a = np.ascontiguousarray(a, dtype=np.int64)
+        t = device.to_dev(a if a.size else np.zeros(1, np.int64))
+        keep.append(t)
+        return t
+
+    lst = f._list_desc(f.p2p, dev)
+    nbytes = _lib.lib.tct_fmm_workspace_bytes(f.kid, f.prec, MODES[f.mode], f.order, f.nq, f.n_obs,
+                                              f.n_src, f.obs_tree.n_nodes, f.src_tree.n_nodes)
+    ws = device.workspace(nbytes)
+    y = device.empty(9 * f.n_obs, f.float_type)
+    t = _lib.tptr
+    _lib.check(_lib.lib.tct_fmm_matvec(
+        f.kid, f.prec, MODES[f.mode], f.order, f.nq, _lib.dptr(f.qx), _lib.dptr(f.qw),
+        _lib.dptr(f.params), 1.0, t(f.obs_pts), t(f.obs_tris), f.n_obs, ctypes.byref(f.obs_desc),
+        t(f.src_pts), t(f.src_tris), f.n_src, ctypes.byref(f.src_desc), ctypes.byref(lst),
+        ctypes.byref(f.far_desc), t(x), t(y), 0, t(ws), nbytes, _lib.stream_ptr()), "tct_fmm_matvec")
+    device.torch().cuda.synchronize()
+    return y.cpu().numpy()
+
+
+CASES = [("elasticRH3", ft, 1, "fmm", leaf, False) for ft in (np.float32, np.float64)
+         for leaf in (1, 15, 16, 33, 64, 65, 130, 2000)]
+CASES += [("elasticRH3", ft, nq, mode, 40, two) for ft in (np.float32, np.float64)
+          for nq in (2, 3, 4) for mode, two in (("fmm", False), ("treecode", False), ("fmm", True))]
+CASES += [(K, ft, nq, "fmm", leaf, two) for K in ("elasticU3", "elasticRT3", "elasticRA3")
+          for ft in (np.float32, np.float64) for nq, leaf, two in ((1, 20, False), (4, 70, True))]
+
+
+@pytest.mark.parametrize("K,ft,nq,mode,leaf,two", CASES)
+def test_planned_matches_unplanned(cuda, K, ft, nq, mode, leaf, two):
+    m = bumpy_mesh(24, seed=1, amp=0.3)
+    m2 = m
+    if two:
+        p, t = bumpy_mesh(17, seed=2)
+        m2 = (p + 0.2, t)
+    f = TSFMM(m, m2, [1.0, 0.25], 3, nq, ft, K, 2.0, leaf, mode)
+    assert f.p2p_plan.sym == (K == "elasticRH3" and nq < 4 and mode == "fmm" and not two)
+    x = device.to_dev(np.random.default_rng(3).standard_normal(9 * f.n_src), ft)
+    y = device.empty(9 * f.n_obs, ft)
+    f.dot_device(x, y)
+    z = y.clone()
+    f.dot_device(x, z)
+    assert cuda.equal(y, z)
+    assert rel(y.cpu().numpy(), _unplanned(f, x)) < TOL[ft]
