@@ -1,0 +1,248 @@
+// Point-pair sums of elasticU3/T3/A3/H3/RT3/RA3 with everything that does not
+// depend on the pair taken out of the pair loop: two observation points sets
+// per lane in FP32 (f32x2 halves), one in FP64 (VecF32 / VecF64).
+//
+// The kernels' vector forms (kernels/__init__.py:28-36, 67-99, 147-173,
+// far_common.cuh vec_utah) are linear in the source value a, so J w and the
+// kernel's constant go into it once per source; with D = y - x, i = 1/r:
+//   U   i (c0 a) + i^3 (D.a) D
+//   T   -c0 i^3 (p a + s n) + (c0 i^3 (n.a) - c1 i^5 p s) D,  p = n.D, s = a.D
+//   A    c0 i^3 (m a - s no) + (c0 i^3 (no.a) + c1 i^5 m s) D, m = no.D
+//   H   with Q = i^3, e = i^2 s, P = 3 n.D:
+//       no Q (h2 (n.a) + h1 P e) + n Q (h1 (no.a) + h3 m e)
+//       + a Q (nu i^2 P m + h1 mn)
+//       + D Q i^2 (3 h1 (n.a) m + h3 mn s + P (nu (no.a) - 5 m e))
+//   RT  i c1 + i^3 (D.c0) D + i^3 (n.D) a   (c1 = CsRT1 J c, c0 = CsRT0 J c)
+//   RA  u-part i (q1 a) + i^3 q0 (D.a) D summed over the obs points with their
+//       weights, -i^3 (no.D) (q2 a) per obs point
+// n.a is formed once per source point, mn = no.n once per triangle pair, the
+// coefficient of n is summed over a triangle's points before it multiplies n,
+// that of no over all sources.  H takes 45 operations per point pair where the
+// direct evaluation takes 78, RT 25 against 36, T 27 against 38, U 18 against 21.
+// r^2 == 0 pairs contribute nothing (i = 0 by select), as in the reference
+// (matrix_free.cl:79-81).
+#pragma once
+
+#include "rh_sym.cuh"
+
+namespace tct {
+namespace {
+
+constexpr bool has_vec_form(int k) { return k != kRH; }
+
+// Record of a source triangle, in Reals (staged as vecs): points (3 NQ), values
+// a (3 NQ), then n (T, H, RT), n.a (NQ; T, H), c (RT).
+template <int K, int NQ>
+struct RecVec {
+    static constexpr int Y = 0, A = 3 * NQ, N = 6 * NQ;
+    static constexpr bool HAS_N = K == kT || K == kH || K == kRT;
+    static constexpr int NA = N + (HAS_N ? 3 : 0);            // n.a
+    static constexpr int C = NA + (K == kT || K == kH ? NQ : 0);
+    static constexpr int RAW = C + (K == kRT ? 3 : 0);
+    static constexpr int LEN = (RAW + 1) / 2 * 2;             // 16 bytes of vecs
+};
+
+// Sums of one observation point set (NO points): per point the 3-vector (RA:
+// its own part) and for A and H the coefficient of no; RA: the u-part (3).
+template <int K, int NO>
+struct AccVec {
+    static constexpr int PER = (K == kA || K == kH) ? 4 : 3;
+    static constexpr int n = PER * NO + (K == kRA ? 3 : 0);
+};
+
+template <typename R, int K, int NQ>
+__device__ __forceinline__ void vec_record(const Consts<R>& c, const Rule2D<R>& rule,
+                                           const TriGeom<R>& s, const R (&in9)[9],
+                                           R (&r)[RecVec<K, NQ>::LEN]) {
+    using L = RecVec<K, NQ>;
+    // constant of the value: U CsU1 (c0 / c1 = 3 - 4 nu), T, A their own below
+    const R ca = K == kU ? c.CsU1 : (K == kH ? c.CsH0 : (K == kRT ? c.CsRT2 : R(1)));
+#pragma unroll
+    for (int q = 0; q < NQ; q++) {
+        const R sx = rule.x[q], sy = rule.y[q];
+        const R sb[3] = {1 - sx - sy, sx, sy};
+        const R f = s.J * rule.w[q] * ca;
+        R na = 0;
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            r[L::Y + 3 * q + d] = bary_point(s, sb, d);
+            const R a = f * (in9[d] * sb[0] + in9[3 + d] * sb[1] + in9[6 + d] * sb[2]);
+            r[L::A + 3 * q + d] = a;
+            na += a * s.n[d];
+        }
+        if (K == kT || K == kH) r[L::NA + q] = na;
+    }
+    if (L::HAS_N) {
+#pragma unroll
+        for (int d = 0; d < 3; d++) r[L::N + d] = s.n[d];
+    }
+    if (K == kRT) {
+        // surface curl of the input, then c[p] = sum e[m][p][j] ssc[j][m]
+        R ssc[3][3];
+#pragma unroll
+        for (int j = 0; j < 3; j++)
+#pragma unroll
+            for (int d = 0; d < 3; d++) {
+                R a = 0;
+#pragma unroll
+                for (int b = 0; b < 3; b++) a += s.sc[b][j] * in9[b * 3 + d];
+                ssc[d][j] = a;
+            }
+#pragma unroll
+        for (int p = 0; p < 3; p++) {
+            R a = 0;
+#pragma unroll
+            for (int m = 0; m < 3; m++)
+#pragma unroll
+                for (int j = 0; j < 3; j++)
+                    if (levi(m, p, j) != 0) a += (R)levi(m, p, j) * ssc[j][m];
+            r[L::C + p] = s.J * a;
+        }
+    }
+#pragma unroll
+    for (int k = L::RAW; k < L::LEN; k++) r[k] = 0;
+}
+
+template <class V>
+__device__ __forceinline__ typename V::vec vdup(typename V::real a) { return V::make(a, a); }
+template <class V>
+__device__ __forceinline__ typename V::vec dot3(const typename V::vec (&a)[3],
+                                                const typename V::vec (&b)[3]) {
+    return V::fma(a[2], b[2], V::fma(a[1], b[1], V::mul(a[0], b[0])));
+}
+
+// One staged record against this lane's points x (negated) with normals no and
+// rule weights wo (RA): adds to acc.
+template <class V, int K, int NO, int NQ>
+__device__ __forceinline__ void vec_pair(const Consts<typename V::real>& c,
+                                         const Rule2D<typename V::real>& rule,
+                                         const typename V::vec* __restrict__ r,
+                                         const typename V::vec (&negx)[NO][3],
+                                         const typename V::vec (&no)[3],
+                                         typename V::vec (&acc)[AccVec<K, NO>::n]) {
+    using vec = typename V::vec;
+    using R = typename V::real;
+    using L = RecVec<K, NQ>;
+    constexpr int PER = AccVec<K, NO>::PER;
+    constexpr bool OBS_N = K == kA || K == kH || K == kRA;
+    vec n[3], cc[3], mn = V::make(0, 0);
+    if (L::HAS_N) {
+#pragma unroll
+        for (int d = 0; d < 3; d++) n[d] = r[L::N + d];
+    }
+    if (K == kH) mn = dot3<V>(no, n);
+    if (K == kRT) {
+#pragma unroll
+        for (int d = 0; d < 3; d++) cc[d] = r[L::C + d];
+    }
+    vec tn[NO];  // per point: coefficient of n (T, H) or c (RT)
+#pragma unroll
+    for (int q = 0; q < NO; q++) tn[q] = V::make(0, 0);
+#pragma unroll
+    for (int q2 = 0; q2 < NQ; q2++) {
+        vec a[3], sm = V::make(0, 0), na = V::make(0, 0);
+#pragma unroll
+        for (int d = 0; d < 3; d++) a[d] = r[L::A + 3 * q2 + d];
+        if (K == kA || K == kH) sm = dot3<V>(no, a);
+        if (K == kT || K == kH) na = r[L::NA + q2];
+#pragma unroll
+        for (int q1 = 0; q1 < NO; q1++) {
+            vec D[3];
+#pragma unroll
+            for (int d = 0; d < 3; d++) D[d] = V::add(r[L::Y + 3 * q2 + d], negx[q1][d]);
+            const vec r2 = dot3<V>(D, D);
+            const vec i = V::rsqrt0(r2);
+            const vec i2 = V::mul(i, i), i3 = V::mul(i2, i);
+            vec* ac = acc + PER * q1;
+            if (K == kU) {
+                const vec f = V::mul(i3, dot3<V>(D, a));
+                const vec g = V::mul(vdup<V>(c.CsU0 / c.CsU1), i);
+#pragma unroll
+                for (int d = 0; d < 3; d++) ac[d] = V::fma(g, a[d], V::fma(f, D[d], ac[d]));
+            } else if (K == kT || K == kA) {
+                const vec p = K == kT ? dot3<V>(n, D) : dot3<V>(no, D);
+                const vec s = dot3<V>(a, D);
+                const vec q = V::mul(vdup<V>(K == kT ? -c.CsT0 : c.CsT0), i3);  // coefficient of p a
+                const vec k1 = V::mul(vdup<V>(K == kT ? -c.CsT1 : c.CsT1), i2);
+                // D (c0 i^3 (n.a) -+ c1 i^5 p s): T uses n.a, A no.a
+                const vec ps = V::mul(p, s);
+                const vec dn = K == kT ? V::mul(vdup<V>(c.CsT0), na) : V::mul(vdup<V>(c.CsT0), sm);
+                const vec dd = V::mul(i3, V::fma(k1, ps, dn));
+                const vec qp = V::mul(q, p);
+                if (K == kT) tn[q1] = V::fma(q, s, tn[q1]);
+                else ac[PER - 1] = V::fma(V::mul(vdup<V>(-c.CsT0), i3), s, ac[PER - 1]);
+#pragma unroll
+                for (int d = 0; d < 3; d++) ac[d] = V::fma(qp, a[d], V::fma(dd, D[d], ac[d]));
+            } else if (K == kH) {
+                const vec p = V::mul(vdup<V>(R(3)), dot3<V>(n, D));
+                const vec m = dot3<V>(no, D);
+                const vec s = dot3<V>(a, D);
+                const vec e = V::mul(i2, s);
+                const vec me = V::mul(m, e);
+                const vec mt = V::fma(V::mul(vdup<V>(c.CsH1), p), e, V::mul(vdup<V>(c.CsH2), na));
+                const vec nt = V::fma(vdup<V>(c.CsH3), me, V::mul(vdup<V>(c.CsH1), sm));
+                const vec st = V::fma(V::mul(vdup<V>(c.nu), V::mul(i2, p)), m,
+                                      V::mul(vdup<V>(c.CsH1), mn));
+                const vec u = V::fma(vdup<V>(R(-5)), me, V::mul(vdup<V>(c.nu), sm));
+                vec dt = V::mul(V::mul(vdup<V>(R(3) * c.CsH1), na), m);
+                dt = V::fma(V::mul(vdup<V>(c.CsH3), mn), s, dt);
+                dt = V::fma(p, u, dt);
+                dt = V::mul(V::mul(i3, i2), dt);
+                const vec sq = V::mul(i3, st);
+                ac[PER - 1] = V::fma(i3, mt, ac[PER - 1]);
+                tn[q1] = V::fma(i3, nt, tn[q1]);
+#pragma unroll
+                for (int d = 0; d < 3; d++) ac[d] = V::fma(sq, a[d], V::fma(dt, D[d], ac[d]));
+            } else if (K == kRT) {
+                const vec w = vdup<V>(rule.w[q2]);
+                const vec f = V::mul(V::mul(V::mul(vdup<V>(c.CsRT0), w), i3), dot3<V>(D, cc));
+                const vec g = V::mul(i3, dot3<V>(n, D));
+                tn[q1] = V::fma(w, i, tn[q1]);
+#pragma unroll
+                for (int d = 0; d < 3; d++) ac[d] = V::fma(g, a[d], V::fma(f, D[d], ac[d]));
+            } else {  // RA
+                const vec w = vdup<V>(rule.w[q1]);
+                const vec f = V::mul(V::mul(V::mul(vdup<V>(c.CsRT0), w), i3), dot3<V>(D, a));
+                const vec g = V::mul(V::mul(vdup<V>(c.CsRT1), w), i);
+                const vec h = V::mul(V::mul(vdup<V>(-c.CsRT2), i3), dot3<V>(no, D));
+#pragma unroll
+                for (int d = 0; d < 3; d++) {
+                    acc[3 * NO + d] = V::fma(g, a[d], V::fma(f, D[d], acc[3 * NO + d]));
+                    ac[d] = V::fma(h, a[d], ac[d]);
+                }
+            }
+        }
+    }
+    if (K == kT || K == kH || K == kRT) {
+#pragma unroll
+        for (int q = 0; q < NO; q++) {
+            const vec t = K == kRT ? V::mul(vdup<V>(c.CsRT1), tn[q]) : tn[q];
+#pragma unroll
+            for (int d = 0; d < 3; d++)
+                acc[PER * q + d] = V::fma(t, K == kRT ? cc[d] : n[d], acc[PER * q + d]);
+        }
+    }
+    (void)OBS_N;
+}
+
+// The NAcc layout of far_epilogue (far_common.cuh) from a lane half's sums.
+template <typename R, int K, int NQ>
+__device__ __forceinline__ void vec_totals(const R (&a)[AccVec<K, NQ>::n], const R (&no)[3],
+                                           R (&tot)[NAcc<K, NQ>::n]) {
+    constexpr int PER = AccVec<K, NQ>::PER;
+#pragma unroll
+    for (int q = 0; q < NQ; q++)
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            R v = a[PER * q + d];
+            if (PER == 4) v += a[PER * q + 3] * no[d];
+            tot[3 * q + d] = v;
+        }
+    if constexpr (K == kRA) {
+#pragma unroll
+        for (int d = 0; d < 3; d++) tot[3 * NQ + d] = a[3 * NQ + d];
+    }
+}
+
+}  // namespace
+}  // namespace tct

@@ -23,8 +23,9 @@
 //    148 SMs several times over; chunk partials are summed in a fixed order
 //    by a second kernel, so results are deterministic.
 #include <algorithm>
+#include <type_traits>
 
-#include "far_common.cuh"
+#include "far_vec.cuh"
 
 namespace tct {
 namespace {
@@ -224,14 +225,169 @@ far_main_rh2(Consts<float> c, Rule2D<float> rule, const float* __restrict__ pts,
     }
 }
 
+// ---- elasticU3/T3/A3/H3/RT3/RA3, 3-, 4- and 7-point rules (far_vec.cuh) ---------
+template <typename R, int K, int NQ>
+__global__ void __launch_bounds__(128)
+far_prep_vec(Consts<R> c, Rule2D<R> rule, const R* __restrict__ pts,
+             const int32_t* __restrict__ src_tris, int64_t n_src, const R* __restrict__ in,
+             R* __restrict__ rec) {
+    using L = RecVec<K, NQ>;
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n_src) return;
+    TriGeom<R> s;
+    load_tri(s, pts, src_tris, i, 0, false, K == kRT);
+    R in9[9], r[L::LEN];
+#pragma unroll
+    for (int k = 0; k < 9; k++) in9[k] = in[i * 9 + k];
+    vec_record<R, K, NQ>(c, rule, s, in9, r);
+#pragma unroll
+    for (int k = 0; k < L::LEN; k++) rec[i * L::LEN + k] = r[k];
+}
+
+// Sources per staged tile, and shared memory: the tile and, in FP32 with more
+// than four points a lane, the running sums and their compensation (as many
+// registers are not left).
+constexpr int vec_ts(int nq) { return nq <= 4 ? 64 : 16; }
+template <class V, int K, int NO>
+constexpr bool vec_smem_sums() { return V::H == 2 && NO > 4; }
+template <class V, int K, int NO, int NQ>
+constexpr size_t vec_smem() {
+    return 8 * ((size_t)RecVec<K, NQ>::LEN * vec_ts(NQ) +
+                (vec_smem_sums<V, K, NO>() ? 2 * 128 * (size_t)AccVec<K, NO>::n : 0));
+}
+
+// The sums of sources [s_begin, s_end) over this lane's points.  Tile sums are
+// added with Kahan compensation in FP32.
+template <class V, int K, int NO, int NQ>
+__device__ __forceinline__ void vec_sources(const Consts<typename V::real>& c,
+                                            const Rule2D<typename V::real>& rule,
+                                            const typename V::real* __restrict__ rec,
+                                            int64_t s_begin, int64_t s_end,
+                                            typename V::vec* __restrict__ sm,
+                                            const typename V::vec (&negx)[NO][3],
+                                            const typename V::vec (&no)[3],
+                                            typename V::vec (&out)[AccVec<K, NO>::n]) {
+    using vec = typename V::vec;
+    using L = RecVec<K, NQ>;
+    constexpr int NA = AccVec<K, NO>::n, TS = vec_ts(NQ);
+    constexpr bool SMEM = vec_smem_sums<V, K, NO>();
+    vec tot[SMEM ? 1 : NA], cmp[V::H == 2 && !SMEM ? NA : 1];
+    vec* st = sm + L::LEN * TS + threadIdx.x;  // SMEM: sum k at 256 k, compensation 128 on
+#pragma unroll
+    for (int k = 0; k < NA; k++) {
+        if constexpr (SMEM) {
+            st[256 * k] = V::make(0, 0);
+            st[256 * k + 128] = V::make(0, 0);
+        } else {
+            tot[k] = V::make(0, 0);
+            if (V::H == 2) cmp[k] = V::make(0, 0);
+        }
+    }
+    for (int64_t t0 = s_begin; t0 < s_end; t0 += TS) {
+        const int nt = (int)min((int64_t)TS, s_end - t0);
+        __syncthreads();
+        for (int k = threadIdx.x; k < nt * L::LEN; k += blockDim.x) {
+            const typename V::real v = __ldg(rec + t0 * L::LEN + k);
+            sm[k] = V::make(v, v);
+        }
+        __syncthreads();
+        vec acc[NA];
+#pragma unroll
+        for (int k = 0; k < NA; k++) acc[k] = V::make(0, 0);
+#pragma unroll 1
+        for (int j = 0; j < nt; j++)
+            vec_pair<V, K, NO, NQ>(c, rule, sm + j * L::LEN, negx, no, acc);
+#pragma unroll
+        for (int k = 0; k < NA; k++) {
+            if constexpr (V::H == 2) {
+                vec& s = SMEM ? st[256 * k] : tot[SMEM ? 0 : k];
+                vec& e = SMEM ? st[256 * k + 128] : cmp[SMEM ? 0 : k];
+                const vec y = V::sub(acc[k], e);
+                const vec t = V::add(s, y);
+                e = V::sub(V::sub(t, s), y);
+                s = t;
+            } else {
+                tot[k] = V::add(tot[k], acc[k]);
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < NA; k++) {
+        if constexpr (SMEM) out[k] = st[256 * k];
+        else out[k] = tot[k];
+    }
+}
+
+// 128 threads take 128 H observation triangles (H = 2 in FP32) against a chunk
+// of sources.  Bound by the FMA pipe.  Against far_main with one triangle a lane
+// and the kernels' direct forms, 5,003 triangles on themselves, 3-point rule,
+// FP32: U 0.407 -> 0.219 ms, T 0.482 -> 0.287, A 0.474 -> 0.305, H 0.689 -> 0.417,
+// RT 0.397 -> 0.260, RA 0.397 -> 0.299; FP64: U 0.811 -> 0.480, H 1.29 -> 0.91,
+// RA 0.81 -> 0.63.
+template <class V, int K, int NQ>
+__global__ void __launch_bounds__(128)
+far_main_vec(Consts<typename V::real> c, Rule2D<typename V::real> rule,
+             const typename V::real* __restrict__ pts, const int32_t* __restrict__ obs_tris,
+             int64_t n_obs, const typename V::real* __restrict__ rec, int64_t n_src,
+             int64_t src_per_chunk, typename V::real* __restrict__ dst, int direct,
+             int accumulate) {
+    using R = typename V::real;
+    using vec = typename V::vec;
+    constexpr int NA = AccVec<K, NQ>::n;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int64_t ia = (int64_t)blockIdx.x * (128 * V::H) + threadIdx.x, ib = ia + 128;
+    const bool va = ia < n_obs, vb = V::H == 2 && ib < n_obs;
+    const int64_t s_begin = (int64_t)blockIdx.y * src_per_chunk;
+    const int64_t s_end = min(n_src, s_begin + src_per_chunk);
+    vec negx[NQ][3], no[3];
+    {
+        TriGeom<R> oa, ob;
+        load_tri(oa, pts, obs_tris, va ? ia : 0, 0, false, false);
+        load_tri(ob, pts, obs_tris, vb ? ib : 0, 0, false, false);
+#pragma unroll
+        for (int q = 0; q < NQ; q++) {
+            const R ox = rule.x[q], oy = rule.y[q];
+            const R bq[3] = {1 - ox - oy, ox, oy};
+#pragma unroll
+            for (int d = 0; d < 3; d++)
+                negx[q][d] = V::make(-bary_point(oa, bq, d), -bary_point(ob, bq, d));
+        }
+#pragma unroll
+        for (int d = 0; d < 3; d++) no[d] = V::make(oa.n[d], ob.n[d]);
+    }
+    vec tot[NA];
+    vec_sources<V, K, NQ, NQ>(c, rule, rec, s_begin, s_end, reinterpret_cast<vec*>(smem_raw), negx,
+                              no, tot);
+#pragma unroll
+    for (int h = 0; h < V::H; h++) {
+        if (!(h == 0 ? va : vb)) continue;
+        const int64_t i = h == 0 ? ia : ib;
+        TriGeom<R> o;
+        load_tri(o, pts, obs_tris, i, 0, false, K == kRA);
+        R a[NA], t[NAcc<K, NQ>::n], out9[9];
+#pragma unroll
+        for (int k = 0; k < NA; k++) {
+            R v[V::H];
+            V::split(tot[k], v);
+            a[k] = v[h];
+        }
+        vec_totals<R, K, NQ>(a, o.n, t);
+        far_epilogue<R, K, NQ>(rule, o, t, out9);
+        R* op = direct ? dst + i * 9 : dst + ((int64_t)blockIdx.y * n_obs + i) * 9;
+#pragma unroll
+        for (int k = 0; k < 9; k++) op[k] = direct && accumulate ? op[k] + out9[k] : out9[k];
+    }
+}
+
 template <typename R>
 __global__ void chunk_reduce(const R* __restrict__ partial, int n_chunks, int64_t n,
                              R* __restrict__ out, int accumulate) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    R s = accumulate ? out[i] : R(0);
-    for (int c = 0; c < n_chunks; c++) s += partial[(int64_t)c * n + i];
-    out[i] = s;
+    double s = accumulate ? (double)out[i] : 0.0;
+#pragma unroll 8
+    for (int c = 0; c < n_chunks; c++) s += (double)partial[(int64_t)c * n + i];
+    out[i] = (R)s;
 }
 
 inline size_t align256(size_t b) { return (b + 255) / 256 * 256; }
@@ -282,15 +438,83 @@ constexpr int64_t MAX_CHUNKS = 64;
 // at most one chunk per CHUNK_GRAIN sources, at most MAX_CHUNKS, and no more
 // than the workspace's partial-sum space (after rec_bytes of records) holds.
 int64_t choose_chunks(int kernel, int prec, int nq, int64_t n_obs, int64_t n_src,
-                      int64_t heuristic, size_t rec_bytes, size_t real_bytes, size_t ws_bytes) {
+                      int64_t heuristic, size_t rec_bytes, size_t real_bytes, size_t ws_bytes,
+                      int64_t grain = CHUNK_GRAIN) {
     int64_t chunks = heuristic;
     int v0 = 0, v1 = 0;
     if (tune_lookup(kTuneFar, kernel, prec, nq, 1, n_obs, n_src, &v0, &v1)) chunks = v0;
-    chunks = std::min<int64_t>(chunks, std::max<int64_t>(1, n_src / CHUNK_GRAIN));
+    chunks = std::min<int64_t>(chunks, std::max<int64_t>(1, n_src / grain));
     chunks = std::min<int64_t>(chunks, MAX_CHUNKS);
     while (chunks > 1 && rec_bytes + align256(real_bytes * 9 * (size_t)n_obs * chunks) > ws_bytes)
         chunks--;
     return std::max<int64_t>(1, chunks);
+}
+
+// Source chunks for the packed RH kernel (256 observation triangles per block).
+int64_t n_chunks_rh2(int64_t n_obs, int64_t n_src) {
+    const int64_t obs_blocks = (n_obs + 255) / 256;
+    int64_t want = (148 * 8 + obs_blocks - 1) / std::max<int64_t>(obs_blocks, 1);
+    int64_t max_by_src = std::max<int64_t>(1, n_src / CHUNK_GRAIN);
+    return std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(want, max_by_src), 32));
+}
+
+// Whether the vec kernels (far_main_vec) serve a kernel and rule.
+constexpr bool use_vec(int kernel, int nq) { return has_vec_form(kernel) && nq <= 7; }
+
+// Source chunks of a far_main_vec launch: in FP32 a block takes 256 triangles,
+// so twice the chunks of at least half the sources (300 triangles otherwise
+// ran on 36 blocks), unless records and partials would pass the 32 MiB that
+// the allocation-free entry point has.
+constexpr int64_t VEC_GRAIN = 8;
+int64_t n_chunks_vec(int prec, int64_t n_obs, int64_t n_src, size_t rec_bytes) {
+    const int64_t base = n_chunks_for(n_obs, n_src, 0);
+    if (prec != TCT_F32) return base;
+    const int64_t strips = (n_obs + 255) / 256;
+    const int64_t more =
+        std::min<int64_t>(std::min<int64_t>((148 * 8 + strips - 1) / std::max<int64_t>(strips, 1),
+                                            std::max<int64_t>(n_src / VEC_GRAIN, 1)), MAX_CHUNKS);
+    return rec_bytes + align256(4 * 9 * (size_t)n_obs * more) <= TCT_NOALLOC_SCRATCH_BYTES
+               ? std::max(base, more) : base;
+}
+
+template <class V, int K, int NQ>
+int run_far_vec(const Consts<typename V::real>& c, const Rule2D<typename V::real>& rule,
+                typename V::real* out, const typename V::real* in, const typename V::real* pts,
+                const int32_t* obs_tris, int64_t n_obs, const int32_t* src_tris, int64_t n_src,
+                int accumulate, unsigned char* ws, size_t ws_bytes, cudaStream_t st) {
+    using R = typename V::real;
+    using L = RecVec<K, NQ>;
+    static_assert(L::LEN <= Rec<K, NQ>::LEN, "the workspace is sized by Rec");
+    constexpr int PREC = sizeof(R) == 8 ? TCT_F64 : TCT_F32;
+    R* rec = reinterpret_cast<R*>(ws);
+    const size_t rec_bytes = align256(sizeof(R) * Rec<K, NQ>::LEN * (size_t)n_src);
+    far_prep_vec<R, K, NQ><<<(unsigned)((n_src + 127) / 128), 128, 0, st>>>(c, rule, pts, src_tris,
+                                                                          n_src, in, rec);
+    int rc = launch_status("farfield prep");
+    if (rc) return rc;
+    const int64_t grain = V::H == 2 ? VEC_GRAIN : CHUNK_GRAIN;
+    const int64_t chunks = choose_chunks(K, PREC, NQ, n_obs, n_src,
+                                         n_chunks_vec(PREC, n_obs, n_src, rec_bytes), rec_bytes,
+                                         sizeof(R), ws_bytes, grain);
+    const int64_t per_chunk = ((n_src + chunks - 1) / chunks + grain - 1) / grain * grain;
+    const int64_t real_chunks = (n_src + per_chunk - 1) / per_chunk;
+    const size_t smem = vec_smem<V, K, NQ, NQ>();
+    if (smem > 48 * 1024 &&
+        cudaFuncSetAttribute(far_main_vec<V, K, NQ>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)smem) != cudaSuccess)
+        return launch_status("farfield shared memory");
+    const int strip = 128 * V::H;
+    dim3 grid((unsigned)((n_obs + strip - 1) / strip), (unsigned)real_chunks);
+    R* partial = reinterpret_cast<R*>(ws + rec_bytes);
+    far_main_vec<V, K, NQ><<<grid, 128, smem, st>>>(c, rule, pts, obs_tris, n_obs, rec, n_src,
+                                                    per_chunk, real_chunks == 1 ? out : partial,
+                                                    real_chunks == 1, accumulate);
+    rc = launch_status("farfield main");
+    if (rc || real_chunks == 1) return rc;
+    const int64_t n = n_obs * 9;
+    chunk_reduce<R><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(partial, (int)real_chunks, n, out,
+                                                                accumulate);
+    return launch_status("farfield chunk reduce");
 }
 
 template <typename R, int K, int NQ>
@@ -331,14 +555,6 @@ int run_far(const Consts<R>& c, const Rule2D<R>& rule, R* out, const R* in, cons
     chunk_reduce<R><<<(unsigned)((n + 255) / 256), 256, 0, st>>>(partial, (int)real_chunks, n, out,
                                                                 accumulate);
     return launch_status("farfield chunk reduce");
-}
-
-// Source chunks for the packed RH kernel (256 observation triangles per block).
-int64_t n_chunks_rh2(int64_t n_obs, int64_t n_src) {
-    const int64_t obs_blocks = (n_obs + 255) / 256;
-    int64_t want = (148 * 8 + obs_blocks - 1) / std::max<int64_t>(obs_blocks, 1);
-    int64_t max_by_src = std::max<int64_t>(1, n_src / CHUNK_GRAIN);
-    return std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(want, max_by_src), 32));
 }
 
 int rec_len_rh2(int nq) {
@@ -419,6 +635,19 @@ template <typename R, int K>
 int run_far_nq(int nq, const Consts<R>& c, const Rule2D<R>& rule, R* out, const R* in,
                const R* pts, const int32_t* ot, int64_t n_obs, const int32_t* stris,
                int64_t n_src, int acc, unsigned char* ws, size_t wsb, cudaStream_t st) {
+    if constexpr (has_vec_form(K)) {
+        using V = std::conditional_t<sizeof(R) == 4, VecF32, VecF64>;
+        switch (nq) {
+            case 3: return run_far_vec<V, K, 3>(c, rule, out, in, pts, ot, n_obs, stris, n_src, acc, ws, wsb, st);
+            case 4: return run_far_vec<V, K, 4>(c, rule, out, in, pts, ot, n_obs, stris, n_src, acc, ws, wsb, st);
+            case 7: return run_far_vec<V, K, 7>(c, rule, out, in, pts, ot, n_obs, stris, n_src, acc, ws, wsb, st);
+            default: break;
+        }
+        if (nq == 13) return run_far<R, K, 13>(c, rule, out, in, pts, ot, n_obs, stris, n_src, acc, ws, wsb, st);
+        set_error("tct_farfield_tris_matvec: %d-point triangle rules are not supported "
+                  "(supported: 3, 4, 7, 13 = gauss2d_tri(1..4))", nq);
+        return TCT_ERR_ARG;
+    } else
     switch (nq) {
         case 3: return run_far<R, K, 3>(c, rule, out, in, pts, ot, n_obs, stris, n_src, acc, ws, wsb, st);
         case 4: return run_far<R, K, 4>(c, rule, out, in, pts, ot, n_obs, stris, n_src, acc, ws, wsb, st);
@@ -659,8 +888,9 @@ size_t farfield_workspace_bytes_chunks(int kernel, int prec, int64_t n_obs, int6
     if (len < 0 || n_src < 0 || n_obs < 0) return 0;
     const size_t rs = prec == TCT_F64 ? 8 : 4;
     const size_t rec_bytes = align256(rs * len * (size_t)n_src);
-    const int64_t chunks = max_chunks > 0 ? std::min(max_chunks, MAX_CHUNKS)
-                                          : n_chunks_for(n_obs, n_src, tile_for(n_q));
+    const int64_t heuristic = use_vec(kernel, n_q) ? n_chunks_vec(prec, n_obs, n_src, rec_bytes)
+                                                   : n_chunks_for(n_obs, n_src, tile_for(n_q));
+    const int64_t chunks = max_chunks > 0 ? std::min(max_chunks, MAX_CHUNKS) : heuristic;
     const size_t part = chunks > 1 ? align256(rs * 9 * (size_t)n_obs * chunks) : 0;
     return rec_bytes + part;
 }
@@ -741,22 +971,127 @@ extern "C" int tct_farfield_pts(int kernel, int prec, void* out, const void* obs
 
 namespace tct {
 namespace {
-// Source chunks of the triangle-to-point farfield: about two blocks per SM
-// over the observation blocks, at least 512 source points per chunk, at
-// most 64 chunks.
-int64_t t2p_chunks(int64_t n_obs, int64_t n_src_pts) {
-    const int64_t obs_blocks = std::max<int64_t>((n_obs + 127) / 128, 1);
-    int64_t want = (2 * 148 + obs_blocks - 1) / obs_blocks;
-    want = std::min<int64_t>(want, std::max<int64_t>(n_src_pts / 512, 1));
+
+// Triangle-to-point farfield of the point kernels by far_vec.cuh: 128 H points
+// a block against a chunk of source triangles.
+template <class V, int K, int NQ>
+__global__ void __launch_bounds__(128)
+t2p_main_vec(Consts<typename V::real> c, Rule2D<typename V::real> rule,
+             const typename V::real* __restrict__ obs_pts,
+             const typename V::real* __restrict__ obs_ns, int64_t n_obs,
+             const typename V::real* __restrict__ rec, int64_t n_src, int64_t src_per_chunk,
+             typename V::real* __restrict__ out) {
+    using R = typename V::real;
+    using vec = typename V::vec;
+    constexpr int NA = AccVec<K, 1>::n;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int64_t ia = (int64_t)blockIdx.x * (128 * V::H) + threadIdx.x, ib = ia + 128;
+    const bool va = ia < n_obs, vb = V::H == 2 && ib < n_obs;
+    const int64_t s_begin = (int64_t)blockIdx.y * src_per_chunk;
+    const int64_t s_end = min(n_src, s_begin + src_per_chunk);
+    const int64_t la = va ? ia : 0, lb = vb ? ib : la;
+    vec negx[1][3], no[3], tot[NA];
+#pragma unroll
+    for (int d = 0; d < 3; d++) {
+        negx[0][d] = V::make(-obs_pts[3 * la + d], -obs_pts[3 * lb + d]);
+        no[d] = V::make(obs_ns[3 * la + d], obs_ns[3 * lb + d]);
+    }
+    vec_sources<V, K, 1, NQ>(c, rule, rec, s_begin, s_end, reinterpret_cast<vec*>(smem_raw), negx,
+                             no, tot);
+#pragma unroll
+    for (int h = 0; h < V::H; h++) {
+        if (!(h == 0 ? va : vb)) continue;
+        const int64_t i = h == 0 ? ia : ib;
+        R a[NA];
+#pragma unroll
+        for (int k = 0; k < NA; k++) {
+            R v[V::H];
+            V::split(tot[k], v);
+            a[k] = v[h];
+        }
+        R* op = out + ((int64_t)blockIdx.y * n_obs + i) * 3;
+#pragma unroll
+        for (int d = 0; d < 3; d++) op[d] = NA == 4 ? a[d] + a[NA - 1] * obs_ns[3 * i + d] : a[d];
+    }
+}
+
+inline bool t2p_vec(int kernel, int n_q) {
+    return kernel >= kU && kernel <= kH && (n_q == 3 || n_q == 4 || n_q == 7);
+}
+
+// Source chunks of the triangle-to-point farfield, at most 64: the vec kernels
+// take about four blocks per SM over the observation strips, with at least 16
+// triangles a chunk; the point kernel (other rules) two blocks per SM and 512
+// source points a chunk.
+int64_t t2p_chunks(int kernel_vec, int prec, int64_t n_obs, int64_t n_src, int n_q) {
+    const int64_t strip = kernel_vec && prec == TCT_F32 ? 256 : 128;
+    const int64_t obs_blocks = std::max<int64_t>((n_obs + strip - 1) / strip, 1);
+    int64_t want = ((kernel_vec ? 4 : 2) * 148 + obs_blocks - 1) / obs_blocks;
+    want = std::min<int64_t>(want, kernel_vec ? std::max<int64_t>(n_src / 16, 1)
+                                              : std::max<int64_t>(n_src * n_q / 512, 1));
     return std::max<int64_t>(1, std::min<int64_t>(want, 64));
 }
+
+template <class V, int K, int NQ>
+int run_t2p_vec(const double* qp, const double* qw, const double* params, void* out,
+                const void* in, const void* obs_pts, const void* obs_ns, int64_t n_obs,
+                const void* pts, const int32_t* tris, int64_t n_src, unsigned char* ws,
+                size_t rec_bytes, cudaStream_t st) {
+    using R = typename V::real;
+    using L = RecVec<K, NQ>;
+    static_assert(L::LEN <= 9 * NQ, "the workspace holds 9 values a source point");
+    const Consts<R> c = make_consts<R>(params);
+    Rule2D<R> rule;
+    for (int q = 0; q < MAXQ; q++) {
+        rule.x[q] = q < NQ ? (R)qp[2 * q] : R(0);
+        rule.y[q] = q < NQ ? (R)qp[2 * q + 1] : R(0);
+        rule.w[q] = q < NQ ? (R)qw[q] : R(0);
+    }
+    R* rec = reinterpret_cast<R*>(ws);
+    int rc;
+    if (n_src > 0) {
+        far_prep_vec<R, K, NQ><<<(unsigned)((n_src + 127) / 128), 128, 0, st>>>(
+            c, rule, (const R*)pts, tris, n_src, (const R*)in, rec);
+        if ((rc = launch_status("tct_farfield_tris_to_pts prep"))) return rc;
+    }
+    const int64_t chunks = t2p_chunks(1, sizeof(R) == 4 ? TCT_F32 : TCT_F64, n_obs, n_src, NQ);
+    const int64_t per = std::max<int64_t>((n_src + chunks - 1) / chunks, 1);
+    const int64_t real = std::max<int64_t>((n_src + per - 1) / per, 1);
+    const int strip = 128 * V::H;
+    dim3 grid((unsigned)((n_obs + strip - 1) / strip), (unsigned)real);
+    R* part = real > 1 ? reinterpret_cast<R*>(ws + rec_bytes) : (R*)out;
+    t2p_main_vec<V, K, NQ><<<grid, 128, vec_smem<V, K, 1, NQ>(), st>>>(
+        c, rule, (const R*)obs_pts, (const R*)obs_ns, n_obs, rec, n_src, per, part);
+    if ((rc = launch_status("tct_farfield_tris_to_pts main")) || real == 1) return rc;
+    const int64_t n3 = n_obs * 3;
+    chunk_reduce<R><<<(unsigned)((n3 + 255) / 256), 256, 0, st>>>(part, (int)real, n3, (R*)out, 0);
+    return launch_status("tct_farfield_tris_to_pts reduce");
+}
+
+template <class V, int K>
+int run_t2p_vec_nq(int n_q, const double* qp, const double* qw, const double* params, void* out,
+                   const void* in, const void* obs_pts, const void* obs_ns, int64_t n_obs,
+                   const void* pts, const int32_t* tris, int64_t n_src, unsigned char* ws,
+                   size_t rec_bytes, cudaStream_t st) {
+    if (n_q == 3)
+        return run_t2p_vec<V, K, 3>(qp, qw, params, out, in, obs_pts, obs_ns, n_obs, pts, tris,
+                                    n_src, ws, rec_bytes, st);
+    if (n_q == 4)
+        return run_t2p_vec<V, K, 4>(qp, qw, params, out, in, obs_pts, obs_ns, n_obs, pts, tris,
+                                    n_src, ws, rec_bytes, st);
+    return run_t2p_vec<V, K, 7>(qp, qw, params, out, in, obs_pts, obs_ns, n_obs, pts, tris, n_src,
+                                ws, rec_bytes, st);
+}
+
 }  // namespace
 }  // namespace tct
 
 extern "C" size_t tct_farfield_tris_to_pts_workspace_bytes(int prec, int64_t n_obs,
                                                            int64_t n_src, int n_q) {
+    // of the kernel that needs more (the query does not name it)
     const size_t r = prec == TCT_F32 ? 4 : 8;
-    const int64_t chunks = tct::t2p_chunks(n_obs, n_src * n_q);
+    const int64_t chunks = std::max(tct::t2p_chunks(1, prec, n_obs, n_src, n_q),
+                                    tct::t2p_chunks(0, prec, n_obs, n_src, n_q));
     const size_t recs = ((size_t)n_src * n_q * 9 * r + 255) / 256 * 256;
     const size_t part = chunks > 1 ? ((size_t)chunks * n_obs * 3 * r + 255) / 256 * 256 : 0;
     return recs + part + 256;
@@ -781,6 +1116,24 @@ extern "C" int tct_farfield_tris_to_pts(int kernel, int prec, void* out, const v
     cudaStream_t st = as_stream(stream);
     const int64_t m = n_src * n_q;
     const unsigned blocks = (unsigned)((m + 127) / 128);
+    if (t2p_vec(kernel, n_q) && (prec == TCT_F32 || prec == TCT_F64)) {
+        unsigned char* ws = reinterpret_cast<unsigned char*>(workspace);
+        const size_t recs = ((size_t)m * 9 * (prec == TCT_F32 ? 4 : 8) + 255) / 256 * 256;
+#define TCT_T2P_VEC(KID)                                                                       \
+    if (kernel == KID)                                                                         \
+        return prec == TCT_F32                                                                 \
+                   ? run_t2p_vec_nq<VecF32, KID>(n_q, quad_pts, quad_wts, params, out, in,     \
+                                                 obs_pts, obs_ns, n_obs, pts, src_tris, n_src, \
+                                                 ws, recs, st)                                 \
+                   : run_t2p_vec_nq<VecF64, KID>(n_q, quad_pts, quad_wts, params, out, in,     \
+                                                 obs_pts, obs_ns, n_obs, pts, src_tris, n_src, \
+                                                 ws, recs, st);
+        TCT_T2P_VEC(kU)
+        TCT_T2P_VEC(kT)
+        TCT_T2P_VEC(kA)
+        TCT_T2P_VEC(kH)
+#undef TCT_T2P_VEC
+    }
 #define TCT_T2P(R, PREC)                                                                    \
     if (prec == PREC) {                                                                     \
         Rule2D<R> rule;                                                                     \
@@ -798,7 +1151,7 @@ extern "C" int tct_farfield_tris_to_pts(int kernel, int prec, void* out, const v
             int rc = launch_status("tct_farfield_tris_to_pts prep");                        \
             if (rc) return rc;                                                              \
         }                                                                                   \
-        const int64_t chunks = t2p_chunks(n_obs, m);                                        \
+        const int64_t chunks = t2p_chunks(0, prec, n_obs, n_src, n_q);                                     \
         if (chunks <= 1)                                                                    \
             return pts_dispatch<R>(kernel, params, out, obs_pts, obs_ns, n_obs, yq, nq, m,  \
                                    vq, st);                                                 \

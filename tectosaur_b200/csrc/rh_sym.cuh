@@ -30,6 +30,13 @@ struct VecF32 {
         upk(a, x, y);
         return pk(rsqrtf(x), rsqrtf(y));
     }
+    // 0 at 0
+    static __device__ __forceinline__ vec rsqrt0(vec a) {
+        float x, y;
+        upk(a, x, y);
+        return pk(x != 0.f ? rsqrtf(x) : 0.f, y != 0.f ? rsqrtf(y) : 0.f);
+    }
+    static __device__ __forceinline__ vec sub(vec a, vec b) { return fma2(b, pk(-1.f, -1.f), a); }
     static __device__ __forceinline__ float hsum(vec a) {
         float x, y;
         upk(a, x, y);
@@ -48,6 +55,8 @@ struct VecF64 {
     static __device__ __forceinline__ vec mul(vec a, vec b) { return a * b; }
     static __device__ __forceinline__ vec fma(vec a, vec b, vec c) { return ::fma(a, b, c); }
     static __device__ __forceinline__ vec rsqrt(vec a) { return ::rsqrt(a); }
+    static __device__ __forceinline__ vec rsqrt0(vec a) { return a != 0.0 ? ::rsqrt(a) : 0.0; }
+    static __device__ __forceinline__ vec sub(vec a, vec b) { return a - b; }
     static __device__ __forceinline__ double hsum(vec a) { return a; }
     static __device__ __forceinline__ void split(vec a, double (&o)[1]) { o[0] = a; }
 };

@@ -1,0 +1,75 @@
+"""The vec-form farfield kernels (csrc/far_vec.cuh: U, T, A, H, RT, RA with 3-,
+4- and 7-point rules) at the edges of their strips, tiles and chunks: the
+triangle farfield against the dense farfield matrix (tct_farfield_tris_dense,
+the tensor forms), the triangle-to-point farfield against the point kernel on
+the quadrature points."""
+import numpy as np
+import pytest
+
+from tectosaur_b200.farfield import farfield_pts_direct
+from tectosaur_b200.interior import TriToPtDirectFarfieldOp
+from tectosaur_b200.ops.dense_integral_op import farfield_tris
+from tectosaur_b200.ops.sparse_farfield_op import TriToTriDirectFarfieldOp
+from tectosaur_b200.util import device
+from tectosaur_b200.util.quadrature import gauss2d_tri
+
+from helpers import PARAMS, bumpy_mesh, rel
+
+pytestmark = pytest.mark.gpu
+
+# the references are FP64; FP32 adds the rounding of coordinates (size 2) over
+# separations above 0.5, 4 x 6e-8 relative, cubed in the kernels' r^-3, and
+# compensated sums
+TOL = {np.float32: 3 * 4 * 6e-8 * 2, np.float64: 1e-13}
+KERNELS = ["elasticU3", "elasticT3", "elasticA3", "elasticH3", "elasticRT3", "elasticRA3"]
+
+
+def _two(n_obs, n_src):
+    p1, t1 = bumpy_mesh(int(np.ceil(np.sqrt(n_obs / 2))) + 1, seed=1)
+    p2, t2 = bumpy_mesh(int(np.ceil(np.sqrt(n_src / 2))) + 1, seed=2)
+    pts = np.vstack([p1, p2 + [0.1, 0.2, 1.0]]).astype(np.float32).astype(np.float64)
+    tris = np.vstack([t1[:n_obs], t2[:n_src] + p1.shape[0]])
+    return pts, tris, np.arange(n_obs), np.arange(n_obs, n_obs + n_src)
+
+
+@pytest.mark.parametrize("ft", [np.float32, np.float64])
+@pytest.mark.parametrize("nq,n_obs,n_src", [(1, 1, 1), (1, 127, 63), (1, 129, 65), (1, 257, 130),
+                                            (2, 255, 7), (2, 60, 301), (3, 130, 17), (3, 33, 150)])
+@pytest.mark.parametrize("K", KERNELS)
+def test_vec_matches_dense(cuda, K, nq, n_obs, n_src, ft):
+    pts, tris, obs, src = _two(n_obs, n_src)
+    x = np.random.default_rng(3).standard_normal(9 * n_src).astype(np.float32)
+    A = farfield_tris(K, PARAMS, pts, tris[obs], tris[src], nq, np.float64)
+    want = np.asarray(A).reshape(9 * n_obs, 9 * n_src) @ x.astype(np.float64)
+    op = TriToTriDirectFarfieldOp(nq, K, PARAMS, pts, tris, ft, obs, src)
+    y = op.dot(device.to_dev(x, ft))
+    assert rel(y.cpu().numpy(), want) < TOL[ft]
+    op.dot_device(device.to_dev(x, ft), y, accumulate=True)
+    assert rel(y.cpu().numpy(), 2 * want) < TOL[ft]
+
+
+@pytest.mark.parametrize("ft", [np.float32, np.float64])
+@pytest.mark.parametrize("nq,n_obs,n_src", [(1, 1, 1), (1, 255, 0), (1, 257, 31), (2, 500, 129),
+                                            (3, 129, 40), (4, 60, 9)])
+@pytest.mark.parametrize("K", KERNELS[:4])
+def test_tris_to_pts_matches_points(cuda, K, nq, n_obs, n_src, ft):
+    rng = np.random.default_rng(4)
+    pts, tris, _, src = _two(2, max(n_src, 1))
+    st = tris[src][:n_src]
+    o = (rng.uniform(-1, 1, (n_obs, 3)) - [0, 0, 2]).astype(np.float32).astype(np.float64)
+    ns = rng.standard_normal((n_obs, 3)).astype(np.float32).astype(np.float64)
+    x = rng.standard_normal(9 * n_src).astype(np.float32)
+    got = TriToPtDirectFarfieldOp(o, ns, (pts, st), K, nq, PARAMS, ft).dot(x)
+    if n_src == 0:
+        assert np.all(got == 0)
+        return
+    q, w = gauss2d_tri(nq)
+    b = np.stack([1 - q[:, 0] - q[:, 1], q[:, 0], q[:, 1]], axis=1)
+    v = pts[st]
+    un = np.cross(v[:, 2] - v[:, 0], v[:, 2] - v[:, 1])
+    J = np.linalg.norm(un, axis=1)
+    y = np.einsum("qb,nbd->nqd", b, v).reshape(-1, 3)
+    n = np.repeat(un / J[:, None], len(w), axis=0)
+    a = np.einsum("qb,nbd,q,n->nqd", b, x.reshape(-1, 3, 3).astype(np.float64), w, J)
+    want = farfield_pts_direct(K, o, ns, y, n, a.reshape(-1), PARAMS, np.float64)
+    assert rel(got, want) < TOL[ft]
