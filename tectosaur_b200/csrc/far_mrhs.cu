@@ -10,10 +10,10 @@
 //   W_o[d][j] += S0 P_s[d][j] + sum_k T[d][k] M_s[k][j].
 // With R inputs this is a GEMM:
 //   W[o, (dj, r)] = sum_{s, c} A[o, (s, c)] B[(s, c), (dj, r)]
-// with A = (S0, T00, T01, T02, T11, T12, T22) per triangle pair -- generated
-// on the fly by the CUDA cores, never stored in HBM -- and B built once per
+// with A = (T00, T01, T02, T11, T12, T22) per triangle pair (S0 is T's trace:
+// P goes into the rows of the diagonal) -- generated on the fly by the CUDA cores, never stored in HBM -- and B built once per
 // apply from the input panel.  Per tile of 128 observation and 8 source
-// triangles: the 128 threads compute A (K = 56) into shared memory, the tile
+// triangles: the generating threads compute A (K = 48) into shared memory, the tile
 // of B is copied in, and one thread issues tcgen05.mma (kind::tf32, M = 128,
 // N = 9R) accumulating in tensor memory.  Split TF32: A = Ah + Al and
 // B = Bh + Bl with every part rounded to TF32; Ah Bh + Ah Bl + Al Bh are
@@ -34,10 +34,15 @@
 // layout, tile by tile (hi block, then lo block), so a tile is one contiguous
 // copy.
 //
-// Waits on the MMA completion barrier are bounded in time (TC_WAIT_NS, by
-// %globaltimer) and their outcome is made CTA-uniform with
-// __syncthreads_and, so no thread is left at a barrier; on timeout the kernel
-// records an error word in the workspace, waits once more (bounded), frees
+// Two A and two B buffers, and mbarriers in place of CTA barriers between the
+// generating warps and the thread that copies B and issues the MMAs (the
+// pipeline is described at the loop).  Against one A buffer, a CTA barrier per
+// tile and S0 as a seventh row: 57.8 -> 44.6 ms (59,858 triangles, 3-point
+// rule, 16 vectors), 23.0 -> 17.3 ms (32,258, 4-point rule).
+//
+// Waits are bounded in time (TC_WAIT_NS, by %globaltimer); the first that runs
+// out sets a shared flag that ends the others, the CTA waits (bounded) for its
+// own copies and MMAs in flight, records an error word in the workspace, frees
 // its tensor memory and returns; CTAs that start after an error exit before
 // allocating tensor memory.
 #include <algorithm>
@@ -50,14 +55,15 @@ namespace {
 
 constexpr int MR_M = TC_M;           // observation triangles per CTA (MMA M)
 constexpr int MR_S = 8;              // source triangles per tile
-constexpr int MR_K = 7 * MR_S;       // 56: GEMM K per tile
+constexpr int MR_C = 6;              // A values per triangle pair
+constexpr int MR_K = MR_C * MR_S;    // 48: GEMM K per tile
 constexpr int MR_KSTEPS = MR_K / 8;  // tf32 MMA K = 8
 constexpr float MR_EPS = 1e-24f;     // r^2 offset (see far_main_rh2)
 constexpr int MR_FLUSH = 8;          // tiles per tensor-memory accumulation
 
-// ---- B panel: per source triangle and RHS, the 7 x 9 GEMM rows --------------
-// B[(s, c), (dj, r)]: c = 0 (S0): P_r[d][j]; c = T_ab: (d == a) M_r[b][j] +
-// (d == b, a != b) M_r[a][j].  One thread per (padded source triangle, r).
+// ---- B panel: per source triangle and RHS, the 6 x 9 GEMM rows --------------
+// B[(s, T_ab), (dj, r)] = (d == a) M_r[b][j] + (d == b, a != b) M_r[a][j] +
+// (a == b) P_r[d][j].  One thread per (padded source triangle, r).
 __global__ void __launch_bounds__(128)
 mrhs_prep(Consts<float> c, float w2, const float* __restrict__ pts,
           const int32_t* __restrict__ src_tris, int64_t n_src, int64_t n_src_pad,
@@ -97,19 +103,15 @@ mrhs_prep(Consts<float> c, float w2, const float* __restrict__ pts,
     unsigned char* base = reinterpret_cast<unsigned char*>(Bg) + tile * (int64_t)2 * N * MR_K * 4;
     const int ab[6][2] = {{0, 0}, {0, 1}, {0, 2}, {1, 1}, {1, 2}, {2, 2}};
 #pragma unroll
-    for (int cc = 0; cc < 7; cc++) {
-        const int k = 7 * sl + cc;
+    for (int cc = 0; cc < MR_C; cc++) {
+        const int k = MR_C * sl + cc;
+        const int a = ab[cc][0], b = ab[cc][1];
 #pragma unroll
         for (int d = 0; d < 3; d++)
 #pragma unroll
             for (int j = 0; j < 3; j++) {
-                float v;
-                if (cc == 0) {
-                    v = P[d][j];
-                } else {
-                    const int a = ab[cc - 1][0], b = ab[cc - 1][1];
-                    v = (d == a ? M[b][j] : 0.f) + ((d == b && a != b) ? M[a][j] : 0.f);
-                }
+                const float v = (a == b ? P[d][j] : 0.f) + (d == a ? M[b][j] : 0.f) +
+                                ((d == b && a != b) ? M[a][j] : 0.f);
                 const int n = (d * 3 + j) * R + r;
                 const float hi = tf32_round(v);
                 const float lo = tf32_round(v - hi);
@@ -122,14 +124,13 @@ mrhs_prep(Consts<float> c, float w2, const float* __restrict__ pts,
 
 // ---- main: generate A, copy B, tcgen05.mma into TMEM ------------------------
 // Observation quadrature points of the rule (barycentric 1 - x - y, x, y).
-// grid (obs blocks of 128, source chunks); G x 128 threads: thread
-// (row, group) generates row `row` of A for the group's 8 / G of the tile's 8
-// source triangles (G = 4 keeps 16 warps in flight where the registers allow,
-// G = 2 for the 7-point rule); one thread issues the B tiles as bulk async
+// grid (obs blocks of 128, source chunks); G x 128 threads generate A: thread
+// (row, group) takes row `row` and the group's 8 / G of the tile's 8 source
+// triangles; one more warp's first thread issues the B tiles as bulk async
 // copies (completing on bar_b[buffer]) and the MMAs (completing on
-// bar_mma).  The G warp groups split the tensor-memory columns of the fold
-// and the epilogue.  Dynamic smem: A hi/lo (2 x 128 x 56 x 4), two B
-// buffers of hi/lo (2 x 2 x N x 56 x 4).
+// bar_m[buffer]).  The G warp groups split the tensor-memory columns of the
+// fold and the epilogue.  Dynamic smem: two A buffers hi/lo (2 x 2 x 128 x 48
+// x 4), two B buffers hi/lo (2 x 2 x N x 48 x 4).
 constexpr int MR_COPIES = 4;  // bulk copies per B tile
 
 template <int R, int NQ, bool UNIFORM, int G>
@@ -140,19 +141,18 @@ mrhs_main(Rule2D<float> rule, const float* __restrict__ pts, const int32_t* __re
           const float* __restrict__ Bg, float* __restrict__ partial, int* __restrict__ err) {
     constexpr int N = 9 * R;
     constexpr int SG = MR_S / G;  // source triangles per thread group
-    constexpr int KG = 7 * SG;    // A values per thread and tile
+    constexpr int KG = MR_C * SG;  // A values per thread and tile
+    static_assert(KG % 4 == 0, "whole 16-byte stores");
     static_assert(3 * N <= 512, "D, S and C must fit the 512 tensor-memory columns");
-    static_assert(N % 8 == 0 && MR_S % G == 0 && KG % 2 == 0, "tile split");
+    static_assert(N % 8 == 0 && MR_S % G == 0 && SG % 2 == 0, "tile split");
     constexpr int NCOL = 512;
     constexpr uint32_t B_BYTES = 2u * N * MR_K * 4;
     static_assert(B_BYTES % (16 * MR_COPIES) == 0, "bulk copies must be 16-byte multiples");
     extern __shared__ __align__(128) unsigned char smem[];
-    unsigned char* Ah = smem;
-    unsigned char* Al = Ah + MR_M * MR_K * 4;
-    // two B buffers (tile t and t + 1), each hi then lo, 2 * N * MR_K * 4
-    unsigned char* Bs0 = Al + MR_M * MR_K * 4;
-    __shared__ __align__(8) uint64_t bar_mma;
-    __shared__ __align__(8) uint64_t bar_b[2];
+    constexpr uint32_t A_BYTES = 2u * MR_M * MR_K * 4;
+    unsigned char* As0 = smem;                // two A buffers, each hi then lo
+    unsigned char* Bs0 = As0 + 2 * A_BYTES;   // two B buffers, each hi then lo
+    __shared__ __align__(8) uint64_t bar_a[2], bar_b[2], bar_m[2], bar_f;
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
 
@@ -180,17 +180,20 @@ mrhs_main(Rule2D<float> rule, const float* __restrict__ pts, const int32_t* __re
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&bar_mma)), "r"(1));
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&bar_b[0])), "r"(1));
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&bar_b[1])), "r"(1));
+        for (int b = 0; b < 2; b++) {
+            mbar_init(smem_u32(&bar_a[b]), 4 * G);  // the generating warps
+            mbar_init(smem_u32(&bar_b[b]), 1);
+            mbar_init(smem_u32(&bar_m[b]), 1);
+        }
+        mbar_init(smem_u32(&bar_f), 4 * G);
         asm volatile("fence.mbarrier_init.release.cluster;");
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
     const uint32_t tmem = tmem_slot;
-    const uint32_t barm = smem_u32(&bar_mma);
-    const uint32_t barb0 = smem_u32(&bar_b[0]), barb1 = smem_u32(&bar_b[1]);
+    const uint32_t bara = smem_u32(bar_a), barb = smem_u32(bar_b), barm = smem_u32(bar_m),
+                   barf = smem_u32(&bar_f);
 
     // obs quadrature points of the rule; weight products for non-uniform rules
     // (a uniform rule's w^2 is folded into B by mrhs_prep)
@@ -232,105 +235,141 @@ mrhs_main(Rule2D<float> rule, const float* __restrict__ pts, const int32_t* __re
         }
     const f2_t eps2 = pk(MR_EPS, MR_EPS);
 
-    // Pipeline per tile t: the A values of tile t are generated in registers
-    // while the MMAs of tile t - 1 run on the tensor cores and the B tile of t
-    // (issued one tile ahead) is in flight; then, once the MMAs of t - 1 have
-    // completed, A is stored to shared memory, the B tile of t + 1 is issued
-    // into the buffer the MMAs of t - 1 read, and the MMAs of t are issued.
-    // (per-buffer state in scalars: a runtime-indexed array would live in local memory)
-    uint32_t phase_m = 0, phase_b0 = 0, phase_b1 = 0;
-    bool pend0 = false, pend1 = false;  // CTA-uniform: B copies issued, not waited for
-    bool ok = true;            // CTA-uniform
-    bool mma_pending = false;  // CTA-uniform: a commit not yet waited for
+    // Pipeline.  Tile i of the chunk (i = t - t0) uses A and B buffer i & 1; its
+    // barriers complete once per use, so use i >> 1 has parity (i >> 1) & 1:
+    //   generators  form A(i) in registers, wait for the MMAs of i - 2 (they read
+    //               the buffer), store A(i), arrive on bar_a; at a group start
+    //               they then wait for the MMAs of i - 1, fold D, arrive on bar_f
+    //   MMA thread  waits for A(i) and B(i) (and the fold), issues the MMAs and
+    //               their commit to bar_m; once the MMAs of i - 1 are done, copies
+    //               B(i + 1) into their buffer
+    // so the generators run up to two tiles ahead of the tensor core and meet no
+    // CTA barrier.
+    const int n_loc = (int)(t1 - t0);
     const uint32_t idesc = mr_instr_desc(N);
     const uint32_t lane_base = tmem + ((uint32_t)((warp & 3) * 32) << 16);
     // this warp's tensor-memory columns: whole 8-column groups, split over G
     const int col0 = (grp * (N / 8) / G) * 8, col1 = ((grp + 1) * (N / 8) / G) * 8;
-    auto issue_b = [&](int64_t tile, int buf) {
-        const uint32_t bar = buf ? barb1 : barb0;
-        if (mma_lead) {
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
-                         "r"(B_BYTES)
-                         : "memory");
-            const unsigned char* src =
-                reinterpret_cast<const unsigned char*>(Bg) + tile * (int64_t)B_BYTES;
-            const uint32_t dst = smem_u32(Bs0) + (uint32_t)buf * B_BYTES;
-#pragma unroll
-            for (int cpy = 0; cpy < MR_COPIES; cpy++)
-                bulk_g2s(dst + cpy * (B_BYTES / MR_COPIES), src + cpy * (B_BYTES / MR_COPIES),
-                         B_BYTES / MR_COPIES, bar);
-        }
-        if (buf) pend1 = true;
-        else pend0 = true;
+    volatile int* stop = &abort_flag;
+    // bounded wait; on a timeout the whole CTA stops
+    auto wait = [&](uint32_t bar, int use) -> bool {
+        if (mbar_wait_or(bar, (uint32_t)(use & 1), stop)) return true;
+        *stop = 1;
+        return false;
     };
-    if (t0 < t1) issue_b(t0, 0);
-    for (int64_t t = t0; t < t1; t++) {
-        const int buf = (int)((t - t0) & 1);
-        // A: this thread's SG source triangles of the tile, KG values, two
-        // source triangles per packed instruction (the MMA warp has no rows)
-        float av[KG];
+    if (mma_warp) {
+        if (mma_lead) {
+            int b_issued = 0, b_seen = 0, committed = 0, m_seen = 0;
+            auto issue_b = [&](int i) {
+                const uint32_t bar = barb + 8 * (i & 1);
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
+                             "r"(B_BYTES)
+                             : "memory");
+                const unsigned char* src =
+                    reinterpret_cast<const unsigned char*>(Bg) + (t0 + i) * (int64_t)B_BYTES;
+                const uint32_t dst = smem_u32(Bs0) + (uint32_t)(i & 1) * B_BYTES;
 #pragma unroll
-        for (int sp = 0; sp < (mma_warp ? 0 : SG / 2); sp++) {
-            const f2_t* y = reinterpret_cast<const f2_t*>(srcy) +
-                            ((t * MR_S + grp * SG) / 2 + sp) * (3 * NQ);
-            f2_t T00 = 0ull, T01 = 0ull, T02 = 0ull, T11 = 0ull, T12 = 0ull, T22 = 0ull;
+                for (int cpy = 0; cpy < MR_COPIES; cpy++)
+                    bulk_g2s(dst + cpy * (B_BYTES / MR_COPIES), src + cpy * (B_BYTES / MR_COPIES),
+                             B_BYTES / MR_COPIES, bar);
+                b_issued++;
+            };
+            if (n_loc > 0) issue_b(0);
+            if (n_loc > 1) issue_b(1);
+            for (int i = 0; i < n_loc; i++) {
+                const int buf = i & 1, use = i >> 1;
+                if (!wait(bara + 8 * buf, use)) break;
+                if (!wait(barb + 8 * buf, use)) break;
+                b_seen++;
+                if (i > 0 && i % MR_FLUSH == 0 && !wait(barf, i / MR_FLUSH - 1)) break;
+                asm volatile("tcgen05.fence::after_thread_sync;");
+                const uint32_t lboA = MR_M / 8 * 128, lboB = N / 8 * 128;
+                const uint32_t aH = smem_u32(As0) + (uint32_t)buf * A_BYTES,
+                               aL = aH + A_BYTES / 2,
+                               bH = smem_u32(Bs0) + (uint32_t)buf * B_BYTES,
+                               bL = bH + N * MR_K * 4;
 #pragma unroll
-            for (int q2 = 0; q2 < NQ; q2++) {
-                const f2_t y0 = __ldg(y + 3 * q2), y1 = __ldg(y + 3 * q2 + 1),
-                           y2 = __ldg(y + 3 * q2 + 2);
-#pragma unroll
-                for (int q1 = 0; q1 < NQ; q1++) {
-                    const f2_t D0 = add2(y0, negx[q1][0]);
-                    const f2_t D1 = add2(y1, negx[q1][1]);
-                    const f2_t D2 = add2(y2, negx[q1][2]);
-                    f2_t r2 = fma2(D0, D0, eps2);
-                    r2 = fma2(D1, D1, r2);
-                    r2 = fma2(D2, D2, r2);
-                    float ra, rb;
-                    upk(r2, ra, rb);
-                    const f2_t ir = pk(rsqrtf(ra), rsqrtf(rb));
-                    f2_t g = mul2(mul2(ir, ir), ir);
-                    if constexpr (WPACK) g = mul2(g, wq2[q1 * NQ + q2]);
-                    else if constexpr (!UNIFORM)
-                        g = mul2(g, pk(wq[q1 * NQ + q2], wq[q1 * NQ + q2]));
-                    const f2_t g0 = mul2(g, D0), g1 = mul2(g, D1), g2 = mul2(g, D2);
-                    T00 = fma2(g0, D0, T00);
-                    T01 = fma2(g0, D1, T01);
-                    T02 = fma2(g0, D2, T02);
-                    T11 = fma2(g1, D1, T11);
-                    T12 = fma2(g1, D2, T12);
-                    T22 = fma2(g2, D2, T22);
+                for (int ks = 0; ks < MR_KSTEPS; ks++) {
+                    const uint64_t dAh = mr_smem_desc(aH + 2 * ks * lboA, lboA, 128);
+                    const uint64_t dAl = mr_smem_desc(aL + 2 * ks * lboA, lboA, 128);
+                    // D restarts at the first tile of every MR_FLUSH group
+                    const uint32_t first = (i % MR_FLUSH == 0 && ks == 0) ? 0u : 1u;
+                    const uint64_t dBh = mr_smem_desc(bH + 2 * ks * lboB, lboB, 128);
+                    const uint64_t dBl = mr_smem_desc(bL + 2 * ks * lboB, lboB, 128);
+                    mma_tf32(tmem, dAh, dBh, idesc, first);
+                    mma_tf32(tmem, dAh, dBl, idesc, 1u);
+                    mma_tf32(tmem, dAl, dBh, idesc, 1u);
+                }
+                asm volatile(
+                    "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::
+                        "r"(barm + 8 * buf)
+                    : "memory");
+                committed++;
+                if (i > 0 && i + 1 < n_loc) {
+                    if (!wait(barm + 8 * (buf ^ 1), (i - 1) >> 1)) break;
+                    m_seen = i;
+                    issue_b(i + 1);
                 }
             }
-            const f2_t S0 = add2(add2(T00, T11), T22);
-            const f2_t Tc[7] = {S0, T00, T01, T02, T11, T12, T22};
+            // nothing of this CTA may be in flight when it gives its memory back
+            for (int i = b_seen; i < b_issued; i++) mbar_wait(barb + 8 * (i & 1), (i >> 1) & 1);
+            for (int i = max(m_seen, committed - 2); i < committed; i++)
+                mbar_wait(barm + 8 * (i & 1), (i >> 1) & 1);
+        }
+        __syncwarp();
+    } else {
+        bool ok = true;
+        for (int i = 0; i < n_loc; i++) {
+            const int64_t t = t0 + i;
+            const int buf = i & 1;
+            // A: this thread's SG source triangles of the tile, KG values, two
+            // source triangles per packed instruction
+            float av[KG];
 #pragma unroll
-            for (int c = 0; c < 7; c++) {
-                float va, vb;
-                upk(Tc[c], va, vb);
-                av[7 * (2 * sp) + c] = valid ? va : 0.f;
-                av[7 * (2 * sp + 1) + c] = valid ? vb : 0.f;
+            for (int sp = 0; sp < SG / 2; sp++) {
+                const f2_t* y = reinterpret_cast<const f2_t*>(srcy) +
+                                ((t * MR_S + grp * SG) / 2 + sp) * (3 * NQ);
+                f2_t T00 = 0ull, T01 = 0ull, T02 = 0ull, T11 = 0ull, T12 = 0ull, T22 = 0ull;
+#pragma unroll
+                for (int q2 = 0; q2 < NQ; q2++) {
+                    const f2_t y0 = __ldg(y + 3 * q2), y1 = __ldg(y + 3 * q2 + 1),
+                               y2 = __ldg(y + 3 * q2 + 2);
+#pragma unroll
+                    for (int q1 = 0; q1 < NQ; q1++) {
+                        const f2_t D0 = add2(y0, negx[q1][0]);
+                        const f2_t D1 = add2(y1, negx[q1][1]);
+                        const f2_t D2 = add2(y2, negx[q1][2]);
+                        f2_t r2 = fma2(D0, D0, eps2);
+                        r2 = fma2(D1, D1, r2);
+                        r2 = fma2(D2, D2, r2);
+                        float ra, rb;
+                        upk(r2, ra, rb);
+                        const f2_t ir = pk(rsqrtf(ra), rsqrtf(rb));
+                        f2_t g = mul2(mul2(ir, ir), ir);
+                        if constexpr (WPACK) g = mul2(g, wq2[q1 * NQ + q2]);
+                        else if constexpr (!UNIFORM)
+                            g = mul2(g, pk(wq[q1 * NQ + q2], wq[q1 * NQ + q2]));
+                        const f2_t g0 = mul2(g, D0), g1 = mul2(g, D1), g2 = mul2(g, D2);
+                        T00 = fma2(g0, D0, T00);
+                        T01 = fma2(g0, D1, T01);
+                        T02 = fma2(g0, D2, T02);
+                        T11 = fma2(g1, D1, T11);
+                        T12 = fma2(g1, D2, T12);
+                        T22 = fma2(g2, D2, T22);
+                    }
+                }
+                const f2_t Tc[MR_C] = {T00, T01, T02, T11, T12, T22};
+#pragma unroll
+                for (int c = 0; c < MR_C; c++) {
+                    float va, vb;
+                    upk(Tc[c], va, vb);
+                    av[MR_C * (2 * sp) + c] = valid ? va : 0.f;
+                    av[MR_C * (2 * sp + 1) + c] = valid ? vb : 0.f;
+                }
             }
-        }
-        // the MMAs of tile t - 1 have read A and B buffer buf ^ 1
-        if (mma_pending) {
-            // the MMA warp polls; the others wait at the CTA barrier
-            const bool w = mma_warp ? mbar_wait(barm, phase_m) : true;
-            if (!__syncthreads_and(w)) {
-                ok = false;  // the MMAs of the previous tile did not complete in time
-                break;
-            }
-            phase_m ^= 1;
-            mma_pending = false;
-            if ((t - t0) % MR_FLUSH == 0) {
-                asm volatile("tcgen05.fence::after_thread_sync;");
-                if (!mma_warp) tmem_fold<N>(lane_base, col0, col1, t - t0 == MR_FLUSH);
-                asm volatile("tcgen05.fence::before_thread_sync;");
-            }
-        }
-        if (t + 1 < t1) issue_b(t + 1, buf ^ 1);
-        if (mma_warp) {
-        } else if constexpr (KG % 4 == 0) {
+            if (i >= 2 && !(ok = wait(barm + 8 * buf, (i - 2) >> 1))) break;
+            unsigned char* Ah = As0 + (uint32_t)buf * A_BYTES;
+            unsigned char* Al = Ah + A_BYTES / 2;
 #pragma unroll
             for (int ch = 0; ch < KG / 4; ch++) {
                 float4 h, l;
@@ -346,72 +385,25 @@ mrhs_main(Rule2D<float> rule, const float* __restrict__ pts, const int32_t* __re
                 *reinterpret_cast<float4*>(Ah + off) = h;
                 *reinterpret_cast<float4*>(Al + off) = l;
             }
-        } else {  // KG = 14: the group's k range starts at an even k
-#pragma unroll
-            for (int ch = 0; ch < KG / 2; ch++) {
-                float2 h, l;
-                h.x = tf32_round(av[2 * ch + 0]);
-                h.y = tf32_round(av[2 * ch + 1]);
-                l.x = tf32_round(av[2 * ch + 0] - h.x);
-                l.y = tf32_round(av[2 * ch + 1] - h.y);
-                const uint32_t off = mr_off(row, grp * KG + 2 * ch, MR_M);
-                *reinterpret_cast<float2*>(Ah + off) = h;
-                *reinterpret_cast<float2*>(Al + off) = l;
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if ((tid & 31) == 0) mbar_arrive(bara + 8 * buf);
+            if (i > 0 && i % MR_FLUSH == 0) {
+                if (!(ok = wait(barm + 8 * (buf ^ 1), (i - 1) >> 1))) break;
+                __syncwarp();
+                asm volatile("tcgen05.fence::after_thread_sync;");
+                tmem_fold<N>(lane_base, col0, col1, i == MR_FLUSH);
+                asm volatile("tcgen05.fence::before_thread_sync;");
+                __syncwarp();
+                if ((tid & 31) == 0) mbar_arrive(barf);
             }
         }
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        {
-            const bool wb = mma_warp ? mbar_wait(buf ? barb1 : barb0, buf ? phase_b1 : phase_b0)
-                                     : true;
-            if (!__syncthreads_and(wb)) {
-                ok = false;
-                break;
-            }
-            if (buf) {
-                phase_b1 ^= 1;
-                pend1 = false;
-            } else {
-                phase_b0 ^= 1;
-                pend0 = false;
-            }
-        }
-        if (mma_lead) {
-            asm volatile("tcgen05.fence::after_thread_sync;");
-            const uint32_t lboA = MR_M / 8 * 128, lboB = N / 8 * 128;
-            const uint32_t aH = smem_u32(Ah), aL = smem_u32(Al),
-                           bH = smem_u32(Bs0) + (uint32_t)buf * B_BYTES,
-                           bL = bH + N * MR_K * 4;
-#pragma unroll
-            for (int ks = 0; ks < MR_KSTEPS; ks++) {
-                const uint64_t dAh = mr_smem_desc(aH + 2 * ks * lboA, lboA, 128);
-                const uint64_t dAl = mr_smem_desc(aL + 2 * ks * lboA, lboA, 128);
-                // D restarts at the first tile of every MR_FLUSH group
-                const uint32_t first = ((t - t0) % MR_FLUSH == 0 && ks == 0) ? 0u : 1u;
-                const uint64_t dBh = mr_smem_desc(bH + 2 * ks * lboB, lboB, 128);
-                const uint64_t dBl = mr_smem_desc(bL + 2 * ks * lboB, lboB, 128);
-                mma_tf32(tmem, dAh, dBh, idesc, first);
-                mma_tf32(tmem, dAh, dBl, idesc, 1u);
-                mma_tf32(tmem, dAl, dBh, idesc, 1u);
-            }
-            asm volatile(
-                "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                    barm)
-                : "memory");
-        }
-        mma_pending = true;
+        if (ok && n_loc > 0) ok = wait(barm + 8 * ((n_loc - 1) & 1), (n_loc - 1) >> 1);
+        __syncwarp();
     }
-    if (ok && mma_pending) {
-        const bool w = mma_warp ? mbar_wait(barm, phase_m) : true;
-        if (!__syncthreads_and(w)) ok = false;
-        else mma_pending = false;
-    }
-    if (!ok) {
-        if (tid == 0) atomicExch(err, 1);
-        // one more bounded wait for whatever is still in flight
-        if (mma_pending) mbar_wait(barm, phase_m);
-        if (pend0) mbar_wait(barb0, phase_b0);
-        if (pend1) mbar_wait(barb1, phase_b1);
-    }
+    __syncthreads();
+    const bool ok = abort_flag == 0;
+    if (!ok && tid == 0) atomicExch(err, 1);
     asm volatile("tcgen05.fence::after_thread_sync;");
 
     // epilogue: fold the last group, then S - C of this thread's row and
@@ -555,8 +547,12 @@ int run_mrhs(const Consts<float>& c, const Rule2D<float>& rule, float* out, cons
     const int64_t chunks = mrhs_chunks(n_obs, n_tiles);
     const int64_t per = (n_tiles + chunks - 1) / chunks;
     const int64_t real = (n_tiles + per - 1) / per;
-    const size_t smem = (size_t)2 * MR_M * MR_K * 4 + (size_t)2 * 2 * N * MR_K * 4;
-    constexpr int G = 2;  // 8 A-generating warps (16 measured slower: 266 vs 277 applies/s)
+    const size_t smem = (size_t)2 * 2 * MR_M * MR_K * 4 + (size_t)2 * 2 * N * MR_K * 4;
+    // A-generating warps 4 G: 16 for the 4-point rule (32,258 triangles, 16
+    // vectors: 17.3 ms against 18.3 with 8); the 3-point rule, bound by the
+    // operands' way through shared memory, takes 8 (44.6 ms at 59,858 with
+    // either), the 7-point rule's registers allow no more
+    constexpr int G = NQ == 4 ? 4 : 2;
     auto kfn = mrhs_main<R, NQ, UNIFORM, G>;
     if (cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
         cudaSuccess)

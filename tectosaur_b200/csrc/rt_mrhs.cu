@@ -10,18 +10,18 @@
 // where c is the source triangle's curl of the input and a_q2 the input
 // interpolated at y.  Summed over the source points of one source triangle
 // this is linear in (c, a) with coefficients that do not depend on the input:
-//   A[x, s] = (S0, T00, T01, T02, T11, T12, T22, V0, V1, V2),
-//   T_kl = sum_q2 g D_k D_l,  S0 = T00 + T11 + T22 = sum_q2 1/r,
+//   A[x, s] = (T00, T01, T02, T11, T12, T22, V0, V1, V2),
+//   T_kl = sum_q2 g D_k D_l,  T00 + T11 + T22 = sum_q2 1/r,
 //   V_q2 = g (n_s . D),  g = w_q2 / r^3 (w_q2 folded into B for equal weights),
 // and with R inputs the farfield is the GEMM
 //   W[x, (d, r)] = sum_{s, c} A[x, (s, c)] B[(s, c), (d, r)]
-// with B (CsRT1 c_d; CsRT0 ((d == k) c_l + (d == l, k != l) c_k); CsRT2 a_q2,d)
-// times J_s, built once per apply from the input panel.  The observation-side
+// with B ((k == l) CsRT1 c_d + CsRT0 ((d == k) c_l + (d == l, k != l) c_k);
+// CsRT2 a_q2,d) times J_s, built once per apply from the input panel.  The observation-side
 // contraction out[b][d] = J_o sum_q1 w_q1 phi_b(q1) W[(o, q1), d] follows in
 // the reduce kernel.
 //
 // A CTA owns 128 observation points (the MMA's M rows: lane = point); per
-// tile of 8 source triangles (K = 80) each thread generates its row of A in
+// tile of 8 source triangles (K = 72) each thread generates its row of A in
 // registers and stores it straight into tensor memory (tcgen05.st, hi and
 // lo TF32 parts), so the MMAs read A from tensor memory and only B (N = 48
 // columns) streams through shared memory -- with A in shared memory too the
@@ -31,7 +31,7 @@
 // fixed order (deterministic), bounded mbarrier waits with the error word
 // and clean-up of far_mrhs.cu.  The D = 0 point pair (a source point on the
 // observation point) contributes exactly nothing, as in the reference's
-// "skip r^2 == 0": r^2 is offset by 1e-24 and S0 is formed as the trace of
+// "skip r^2 == 0": r^2 is offset by 1e-24 and the 1/r sum is the trace of
 // T, so every A entry carries a factor of D.
 #include <algorithm>
 
@@ -45,9 +45,9 @@ constexpr int RT_M = TC_M;            // observation points per CTA (MMA M)
 constexpr int RT_NQ = 3;              // points of the rule (both sides)
 constexpr int RT_R = 16;              // right-hand sides per panel
 constexpr int RT_N = 3 * RT_R;        // 48: GEMM N, column n = d * R + r
-constexpr int RT_C = 7 + RT_NQ;       // 10 A columns per source triangle
+constexpr int RT_C = 6 + RT_NQ;       // 9 A columns per source triangle
 constexpr int RT_S = 8;               // source triangles per tile
-constexpr int RT_K = RT_C * RT_S;     // 80: GEMM K per tile
+constexpr int RT_K = RT_C * RT_S;     // 72: GEMM K per tile
 constexpr int RT_KSTEPS = RT_K / 8;   // tf32 MMA K = 8
 constexpr int RT_G = 2;               // A-generating warp groups (2 packed pairs each)
 constexpr int RT_FLUSH = 8;           // tiles per tensor-memory accumulation
@@ -111,8 +111,8 @@ rt_points(Rule2D<float> rule, const float* __restrict__ pts, const int32_t* __re
     for (int d = 0; d < 3; d++) y[2 * (3 * RT_NQ + d)] = t.n[d];
 }
 
-// ---- B panel: per source triangle and RHS, the 10 x 48 GEMM rows ------------
-// One thread per (padded source triangle, r); rows k = 10 sl + c of tile
+// ---- B panel: per source triangle and RHS, the 9 x 48 GEMM rows ------------
+// One thread per (padded source triangle, r); rows k = 9 sl + c of tile
 // s / RT_S, hi block then lo block, in the canonical K-major layout.
 __global__ void __launch_bounds__(128)
 rt_prep(Consts<float> c, Rule2D<float> rule, float wbar, const float* __restrict__ pts,
@@ -171,13 +171,13 @@ rt_prep(Consts<float> c, Rule2D<float> rule, float wbar, const float* __restrict
 #pragma unroll
         for (int d = 0; d < 3; d++) {
             float v;
-            if (cc == 0) {
-                v = c.CsRT1 * cv[d];
-            } else if (cc < 7) {
-                const int a = ab[cc - 1][0], b = ab[cc - 1][1];
-                v = c.CsRT0 * ((d == a ? cv[b] : 0.f) + ((d == b && a != b) ? cv[a] : 0.f));
+            if (cc < 6) {
+                // the sum of 1 / r is the trace of the D D^T / r^3 sums
+                const int a = ab[cc][0], b = ab[cc][1];
+                v = (a == b ? c.CsRT1 * cv[d] : 0.f) +
+                    c.CsRT0 * ((d == a ? cv[b] : 0.f) + ((d == b && a != b) ? cv[a] : 0.f));
             } else {
-                v = c.CsRT2 * av[cc - 7][d];
+                v = c.CsRT2 * av[cc - 6][d];
             }
             v *= scale;
             const int n = d * RT_R + r;
@@ -193,18 +193,11 @@ rt_prep(Consts<float> c, Rule2D<float> rule, float wbar, const float* __restrict
 // ---- main: generate A into tensor memory, copy B, tcgen05.mma --------------
 // grid (point blocks of 128, source chunks); RT_G x 128 threads generate A
 // (thread (row, group): observation point `row`, the group's 4 of the tile's
-// 8 source triangles as two packed pairs, their records loaded while the
-// previous tile is stored), one more warp issues the B copies and the MMAs.
-// Per tile t: A(t) is generated in registers while the MMAs of t - 1 run;
-// each thread waits (itself, on the mbarrier) for the MMAs of t - 2, which
-// read A buffer t & 1, and stores A(t) there; the B tile of t + 1 goes into
-// the B buffer those MMAs read (three B buffers); after one CTA barrier the
-// MMAs of t are issued behind those of t - 1.  At the end of each group of
-// RT_FLUSH tiles all MMAs complete and D is folded into the Kahan pair.
-// Measured on the 60k-triangle surface (16 vectors, 152 ms): timing copies
-// without the MMAs take 98 ms, without the A arithmetic 126 ms -- the
-// per-tile B traffic from L2 (every CTA of 128 points re-reads the 230 MB B
-// operand) and the per-tile barrier, not the arithmetic, set the pace.
+// 8 source triangles as two packed pairs), one more warp's first thread issues
+// the B copies and the MMAs; mbarriers between them (the pipeline is described
+// at the loop).  Against a CTA barrier per tile and the 1 / r sum as a tenth
+// column: 17.9 -> 13.4 ms (20,000 triangles, 16 vectors), 3.07 -> 2.29 ms
+// (7,441, 11 vectors).
 template <bool UNIFORM>
 __global__ void __launch_bounds__(128 * RT_G + 32, 1)
 rt_main(Rule2D<float> rule, const float* __restrict__ pts, const int32_t* __restrict__ obs_tris,
@@ -216,8 +209,7 @@ rt_main(Rule2D<float> rule, const float* __restrict__ pts, const int32_t* __rest
     static_assert(SG % 2 == 0 && KG % 4 == 0, "whole packed pairs, 4-column stores");
     extern __shared__ __align__(128) unsigned char smem[];
     unsigned char* Bs0 = smem;  // three B buffers, each hi then lo
-    __shared__ __align__(8) uint64_t bar_m[2];
-    __shared__ __align__(8) uint64_t bar_b[3];
+    __shared__ __align__(8) uint64_t bar_a[2], bar_m[2], bar_b[3], bar_f;
     __shared__ uint32_t tmem_slot;
     __shared__ int abort_flag;
 
@@ -242,21 +234,20 @@ rt_main(Rule2D<float> rule, const float* __restrict__ pts, const int32_t* __rest
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
     }
     if (tid == 0) {
-        for (int i = 0; i < 2; i++)
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&bar_m[i])),
-                         "r"(1));
-        for (int i = 0; i < 3; i++)
-            asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(&bar_b[i])),
-                         "r"(1));
+        for (int i = 0; i < 2; i++) {
+            mbar_init(smem_u32(&bar_a[i]), 4 * RT_G);  // the generating warps
+            mbar_init(smem_u32(&bar_m[i]), 1);
+        }
+        for (int i = 0; i < 3; i++) mbar_init(smem_u32(&bar_b[i]), 1);
+        mbar_init(smem_u32(&bar_f), 4 * RT_G);
         asm volatile("fence.mbarrier_init.release.cluster;");
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;");
     const uint32_t tmem = tmem_slot;
-    const uint32_t barm0 = smem_u32(&bar_m[0]), barm1 = smem_u32(&bar_m[1]);
-    const uint32_t barb0 = smem_u32(&bar_b[0]), barb1 = smem_u32(&bar_b[1]),
-                   barb2 = smem_u32(&bar_b[2]);
+    const uint32_t bara = smem_u32(bar_a), barb = smem_u32(bar_b), barm = smem_u32(bar_m),
+                   barf = smem_u32(&bar_f);
 
     // this thread's observation point (packed, negated: D = y_pair + negx);
     // a row past the last point sits 1e18 away, where every A entry
@@ -282,78 +273,104 @@ rt_main(Rule2D<float> rule, const float* __restrict__ pts, const int32_t* __rest
     }
     const f2_t eps2 = pk(RT_EPS, RT_EPS);
 
-    // Pipeline state, the same in every thread (each thread runs every wait
-    // itself): MMAs of tile t commit to bar_m[t & 1]; B tiles rotate through
-    // three buffers, so the copy of tile t + 1 needs only the MMAs of t - 2
-    // to have completed, and the MMAs of t queue behind those of t - 1.
-    uint32_t ph_m0 = 0, ph_m1 = 0, ph_b0 = 0, ph_b1 = 0, ph_b2 = 0;
-    bool pm0 = false, pm1 = false;              // MMA commit not yet observed
-    bool pb0 = false, pb1 = false, pb2 = false;  // B copy not yet observed
-    bool ok = true;                             // CTA-uniform after each barrier
+    // Pipeline, as in far_mrhs.cu: tile i of the chunk (i = t - t0) uses A buffer
+    // i & 1 (tensor memory) and B buffer i % 3; a barrier's use u has parity u & 1.
+    //   generators  form A(i) in registers (its records were loaded while A(i - 1)
+    //               was stored), wait for the MMAs of i - 2, store A(i), arrive on
+    //               bar_a; at a group start they then wait for the MMAs of i - 1,
+    //               fold D and arrive on bar_f
+    //   MMA thread  waits for A(i) and B(i) (and the fold), issues the MMAs and
+    //               their commit to bar_m; once the MMAs of i - 1 are done, copies
+    //               B(i + 2) into their buffer
+    const int n_loc = (int)(t1 - t0);
     const uint32_t idesc = mr_instr_desc(RT_N);
     const uint32_t lane_off = (uint32_t)((warp & 3) * 32) << 16;
     const uint32_t lane_base = tmem + lane_off;
     // this warp's accumulator columns in the fold and the epilogue
     const int col0 = (grp * (RT_N / 8) / RT_G) * 8, col1 = ((grp + 1) * (RT_N / 8) / RT_G) * 8;
-    auto wait_m = [&](int i, bool& good) {
-        if (i == 0 && pm0) {
-            good = mbar_wait(barm0, ph_m0) && good;
-            ph_m0 ^= 1;
-            pm0 = false;
-        } else if (i == 1 && pm1) {
-            good = mbar_wait(barm1, ph_m1) && good;
-            ph_m1 ^= 1;
-            pm1 = false;
-        }
+    volatile int* stop = &abort_flag;
+    // bounded wait; on a timeout the whole CTA stops
+    auto wait = [&](uint32_t bar, int use) -> bool {
+        if (mbar_wait_or(bar, (uint32_t)(use & 1), stop)) return true;
+        *stop = 1;
+        return false;
     };
-    auto issue_b = [&](int64_t tile, int buf) {
-        const uint32_t bar = buf == 0 ? barb0 : (buf == 1 ? barb1 : barb2);
+    if (mma_warp) {
         if (mma_lead) {
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
-                         "r"(RT_B_BYTES)
-                         : "memory");
-            const unsigned char* src =
-                reinterpret_cast<const unsigned char*>(Bg) + tile * (int64_t)RT_B_BYTES;
-            const uint32_t dst = smem_u32(Bs0) + (uint32_t)buf * RT_B_BYTES;
+            int b_issued = 0, b_seen = 0, committed = 0, m_seen = 0;
+            auto issue_b = [&](int i) {
+                const uint32_t bar = barb + 8 * (i % 3);
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
+                             "r"(RT_B_BYTES)
+                             : "memory");
+                const unsigned char* src =
+                    reinterpret_cast<const unsigned char*>(Bg) + (t0 + i) * (int64_t)RT_B_BYTES;
+                const uint32_t dst = smem_u32(Bs0) + (uint32_t)(i % 3) * RT_B_BYTES;
 #pragma unroll
-            for (int cpy = 0; cpy < RT_COPIES; cpy++)
-                bulk_g2s(dst + cpy * (RT_B_BYTES / RT_COPIES),
-                         src + cpy * (RT_B_BYTES / RT_COPIES), RT_B_BYTES / RT_COPIES, bar);
+                for (int cpy = 0; cpy < RT_COPIES; cpy++)
+                    bulk_g2s(dst + cpy * (RT_B_BYTES / RT_COPIES),
+                             src + cpy * (RT_B_BYTES / RT_COPIES), RT_B_BYTES / RT_COPIES, bar);
+                b_issued++;
+            };
+            for (int i = 0; i < 3 && i < n_loc; i++) issue_b(i);
+            for (int i = 0; i < n_loc; i++) {
+                const int abuf = i & 1, bbuf = i % 3;
+                if (!wait(bara + 8 * abuf, i >> 1)) break;
+                if (!wait(barb + 8 * bbuf, i / 3)) break;
+                b_seen++;
+                if (i > 0 && i % RT_FLUSH == 0 && !wait(barf, i / RT_FLUSH - 1)) break;
+                asm volatile("tcgen05.fence::after_thread_sync;");
+                const uint32_t lboB = RT_N / 8 * 128;
+                const uint32_t bH = smem_u32(Bs0) + (uint32_t)bbuf * RT_B_BYTES,
+                               bL = bH + RT_N * RT_K * 4;
+                const uint32_t aH = tmem + RT_COL_A + 2 * RT_K * abuf, aL = aH + RT_K;
+#pragma unroll
+                for (int ks = 0; ks < RT_KSTEPS; ks++) {
+                    // D restarts at the first tile of every RT_FLUSH group
+                    const uint32_t first = (i % RT_FLUSH == 0 && ks == 0) ? 0u : 1u;
+                    const uint64_t dBh = mr_smem_desc(bH + 2 * ks * lboB, lboB, 128);
+                    const uint64_t dBl = mr_smem_desc(bL + 2 * ks * lboB, lboB, 128);
+                    mma_tf32_ts(tmem, aH + 8 * ks, dBh, idesc, first);
+                    mma_tf32_ts(tmem, aH + 8 * ks, dBl, idesc, 1u);
+                    mma_tf32_ts(tmem, aL + 8 * ks, dBh, idesc, 1u);
+                }
+                asm volatile(
+                    "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::
+                        "r"(barm + 8 * abuf)
+                    : "memory");
+                committed++;
+                if (i > 0 && i + 2 < n_loc) {
+                    if (!wait(barm + 8 * (abuf ^ 1), (i - 1) >> 1)) break;
+                    m_seen = i;
+                    issue_b(i + 2);
+                }
+            }
+            // nothing of this CTA may be in flight when it gives its memory back
+            for (int i = b_seen; i < b_issued; i++) mbar_wait(barb + 8 * (i % 3), (i / 3) & 1);
+            for (int i = max(m_seen, committed - 2); i < committed; i++)
+                mbar_wait(barm + 8 * (i & 1), (i >> 1) & 1);
         }
-        if (buf == 0) pb0 = true;
-        else if (buf == 1) pb1 = true;
-        else pb2 = true;
-    };
-    // this thread's source pair record of tile t
-    const f2_t* recs = reinterpret_cast<const f2_t*>(srcy) + grp * NP * RT_REC;
-    constexpr int64_t REC_STRIDE = (RT_S / 2) * RT_REC;  // f2 values per tile
-    f2_t yc[NP][RT_REC];
-    if (!mma_warp && t0 < t1) {
-#pragma unroll
-        for (int sp = 0; sp < NP; sp++)
-#pragma unroll
-            for (int k = 0; k < RT_REC; k++)
-                yc[sp][k] = __ldg(recs + t0 * REC_STRIDE + sp * RT_REC + k);
-    }
-    if (t0 < t1) issue_b(t0, 0);
-    for (int64_t t = t0; t < t1; t++) {
-        const int64_t k = t - t0;
-        const int abuf = (int)(k & 1), bbuf = (int)(k % 3);
+        __syncwarp();
+    } else {
+        // this thread's source pair records of a tile
+        const f2_t* recs = reinterpret_cast<const f2_t*>(srcy) + grp * NP * RT_REC;
+        constexpr int64_t REC_STRIDE = (RT_S / 2) * RT_REC;  // f2 values per tile
+        f2_t yc[NP][RT_REC];
         bool good = true;
-        if (k > 0 && k % RT_FLUSH == 0) {
-            // an accumulation group ends: its MMAs (up to those of t - 1)
-            // complete, then D is folded into the Kahan pair before the
-            // MMAs of t restart it
-            wait_m(0, good);
-            wait_m(1, good);
-            asm volatile("tcgen05.fence::after_thread_sync;");
-            if (!mma_warp) tmem_fold<RT_N>(lane_base, col0, col1, k == RT_FLUSH);
+        if (n_loc > 0) {
+#pragma unroll
+            for (int sp = 0; sp < NP; sp++)
+#pragma unroll
+                for (int k = 0; k < RT_REC; k++)
+                    yc[sp][k] = __ldg(recs + t0 * REC_STRIDE + sp * RT_REC + k);
         }
-        float av[KG];
-        if (!mma_warp) {
+        for (int i = 0; i < n_loc; i++) {
+            const int64_t t = t0 + i;
+            const int abuf = i & 1;
+            float av[KG];
 #pragma unroll
             for (int sp = 0; sp < NP; sp++) {
-                // A of one packed source pair for this point: 10 values per source
+                // A of one packed source pair for this point: 9 values per source
                 const f2_t* yr = yc[sp];
                 const f2_t n0 = yr[3 * RT_NQ], n1 = yr[3 * RT_NQ + 1], n2 = yr[3 * RT_NQ + 2];
                 f2_t T00 = 0ull, T01 = 0ull, T02 = 0ull, T11 = 0ull, T12 = 0ull, T22 = 0ull;
@@ -380,8 +397,7 @@ rt_main(Rule2D<float> rule, const float* __restrict__ pts, const int32_t* __rest
                     T22 = fma2(g2, D2, T22);
                     V[q2] = fma2(g2, n2, fma2(g1, n1, mul2(g0, n0)));
                 }
-                const f2_t S0 = add2(add2(T00, T11), T22);
-                const f2_t Tc[RT_C] = {S0, T00, T01, T02, T11, T12, T22, V[0], V[1], V[2]};
+                const f2_t Tc[RT_C] = {T00, T01, T02, T11, T12, T22, V[0], V[1], V[2]};
 #pragma unroll
                 for (int cc = 0; cc < RT_C; cc++) {
                     float va, vb;
@@ -390,19 +406,17 @@ rt_main(Rule2D<float> rule, const float* __restrict__ pts, const int32_t* __rest
                     av[2 * RT_C * sp + RT_C + cc] = vb;
                 }
             }
-            // the next tile's records: in flight while A is stored and the
-            // CTA waits for the B tile
-            if (t + 1 < t1) {
+            // the next tile's records: in flight while A is stored
+            if (i + 1 < n_loc) {
 #pragma unroll
                 for (int sp = 0; sp < NP; sp++)
 #pragma unroll
                     for (int q = 0; q < RT_REC; q++)
                         yc[sp][q] = __ldg(recs + (t + 1) * REC_STRIDE + sp * RT_REC + q);
             }
-        }
-        // the MMAs of t - 2 read A buffer abuf and B buffer (k + 1) % 3
-        wait_m(abuf, good);
-        if (!mma_warp) {
+            // the MMAs of i - 2 read this A buffer
+            if (i >= 2 && !(good = wait(barm + 8 * abuf, (i - 2) >> 1))) break;
+            __syncwarp();
             // hi / lo parts into A buffer abuf, columns [KG grp, KG (grp + 1));
             // lo is left in FP32: the MMA reads the top 19 bits of a TF32
             // operand, so it is truncated there (|lo| <= 2^-11 |v|, its
@@ -421,70 +435,27 @@ rt_main(Rule2D<float> rule, const float* __restrict__ pts, const int32_t* __rest
                 tmem_st4(ahi + RT_K + 4 * ch, l[0], l[1], l[2], l[3]);
             }
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-        }
-        if (good && t + 1 < t1) issue_b(t + 1, (int)((k + 1) % 3));
-        asm volatile("tcgen05.fence::before_thread_sync;");
-        {
-            bool wb = true;
-            if (mma_warp) {
-                const uint32_t bar = bbuf == 0 ? barb0 : (bbuf == 1 ? barb1 : barb2);
-                const uint32_t ph = bbuf == 0 ? ph_b0 : (bbuf == 1 ? ph_b1 : ph_b2);
-                wb = mbar_wait(bar, ph);
-            }
-            if (bbuf == 0) {
-                ph_b0 ^= 1;
-                pb0 = false;
-            } else if (bbuf == 1) {
-                ph_b1 ^= 1;
-                pb1 = false;
-            } else {
-                ph_b2 ^= 1;
-                pb2 = false;
-            }
-            if (!__syncthreads_and(good && wb)) {
-                ok = false;  // a bounded wait gave up
-                break;
+            asm volatile("tcgen05.fence::before_thread_sync;");
+            __syncwarp();
+            if ((tid & 31) == 0) mbar_arrive(bara + 8 * abuf);
+            if (i > 0 && i % RT_FLUSH == 0) {
+                // a group ended with tile i - 1: D goes into the Kahan pair
+                // before the MMAs of i restart it
+                if (!(good = wait(barm + 8 * (abuf ^ 1), (i - 1) >> 1))) break;
+                __syncwarp();
+                asm volatile("tcgen05.fence::after_thread_sync;");
+                tmem_fold<RT_N>(lane_base, col0, col1, i == RT_FLUSH);
+                asm volatile("tcgen05.fence::before_thread_sync;");
+                __syncwarp();
+                if ((tid & 31) == 0) mbar_arrive(barf);
             }
         }
-        if (mma_lead) {
-            asm volatile("tcgen05.fence::after_thread_sync;");
-            const uint32_t lboB = RT_N / 8 * 128;
-            const uint32_t bH = smem_u32(Bs0) + (uint32_t)bbuf * RT_B_BYTES,
-                           bL = bH + RT_N * RT_K * 4;
-            const uint32_t aH = tmem + RT_COL_A + 2 * RT_K * abuf, aL = aH + RT_K;
-#pragma unroll
-            for (int ks = 0; ks < RT_KSTEPS; ks++) {
-                // D restarts at the first tile of every RT_FLUSH group
-                const uint32_t first = (k % RT_FLUSH == 0 && ks == 0) ? 0u : 1u;
-                const uint64_t dBh = mr_smem_desc(bH + 2 * ks * lboB, lboB, 128);
-                const uint64_t dBl = mr_smem_desc(bL + 2 * ks * lboB, lboB, 128);
-                mma_tf32_ts(tmem, aH + 8 * ks, dBh, idesc, first);
-                mma_tf32_ts(tmem, aH + 8 * ks, dBl, idesc, 1u);
-                mma_tf32_ts(tmem, aL + 8 * ks, dBh, idesc, 1u);
-            }
-            asm volatile(
-                "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                    abuf ? barm1 : barm0)
-                : "memory");
-        }
-        if (abuf) pm1 = true;
-        else pm0 = true;
+        if (good && n_loc > 0) wait(barm + 8 * ((n_loc - 1) & 1), (n_loc - 1) >> 1);
+        __syncwarp();
     }
-    if (ok) {
-        bool good = true;
-        wait_m(0, good);
-        wait_m(1, good);
-        if (!__syncthreads_and(good)) ok = false;
-    }
-    if (!ok) {
-        if (tid == 0) atomicExch(err, 1);
-        // one more bounded wait for whatever is still in flight
-        if (pm0) mbar_wait(barm0, ph_m0);
-        if (pm1) mbar_wait(barm1, ph_m1);
-        if (pb0) mbar_wait(barb0, ph_b0);
-        if (pb1) mbar_wait(barb1, ph_b1);
-        if (pb2) mbar_wait(barb2, ph_b2);
-    }
+    __syncthreads();
+    const bool ok = abort_flag == 0;
+    if (!ok && tid == 0) atomicExch(err, 1);
     asm volatile("tcgen05.fence::after_thread_sync;");
 
     // epilogue: fold the last group, then S - C of this thread's point and

@@ -70,6 +70,29 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t phase) {
     }
 }
 
+// The same, given up as soon as *stop is set as well.
+__device__ __forceinline__ bool mbar_wait_or(uint32_t bar, uint32_t phase, volatile int* stop) {
+    const unsigned long long start = gtimer();
+    for (;;) {
+        uint32_t done;
+        asm volatile(
+            "{\n\t.reg .pred P1;\n\t"
+            "mbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2;\n\t"
+            "selp.b32 %0, 1, 0, P1;\n\t}"
+            : "=r"(done)
+            : "r"(bar), "r"(phase)
+            : "memory");
+        if (done) return true;
+        if (*stop || gtimer() - start > TC_WAIT_NS) return false;
+    }
+}
+__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
+}
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
 __device__ __forceinline__ void mma_tf32(uint32_t d_tmem, uint64_t a, uint64_t b, uint32_t idesc,
                                          uint32_t accumulate) {
     uint32_t mask[4] = {0, 0, 0, 0};
