@@ -435,9 +435,8 @@ int tct_fmm_matvec(int kernel, int prec, int mode, int order, int n_q,
                    void* stream);
 
 /* Work plan of the near leaves (device arrays; the layouts fmm/p2p_plan.py
- * writes): observation chunks of at most `chunk` triangles (64 for
- * elasticRH3 in FP32 with a 3-, 4- or 7-point rule, else 32) against runs of
- * list entries.
+ * writes): observation chunks of at most `chunk` triangles (64 in FP32 with
+ * a 3-, 4- or 7-point rule, else 32) against runs of list entries.
  *   tasks    n_tasks x 4: first obs triangle (tree order), count, first and
  *            end entry (at most 128 entries)
  *   entries  first source triangle, count, first slot or -1 (one-sided)

@@ -244,5 +244,24 @@ __device__ __forceinline__ void vec_totals(const R (&a)[AccVec<K, NQ>::n], const
     }
 }
 
+template <typename R, int K, int NQ>
+__global__ void __launch_bounds__(128)
+far_prep_vec(Consts<R> c, Rule2D<R> rule, const R* __restrict__ pts,
+             const int32_t* __restrict__ src_tris, int64_t n_src, const R* __restrict__ in,
+             const int64_t* __restrict__ orig, R* __restrict__ rec) {
+    using L = RecVec<K, NQ>;
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n_src) return;
+    TriGeom<R> s;
+    load_tri(s, pts, src_tris, i, 0, false, K == kRT);
+    const int64_t ii = orig ? orig[i] : i;  // input row of tree-ordered sources
+    R in9[9], r[L::LEN];
+#pragma unroll
+    for (int k = 0; k < 9; k++) in9[k] = in[ii * 9 + k];
+    vec_record<R, K, NQ>(c, rule, s, in9, r);
+#pragma unroll
+    for (int k = 0; k < L::LEN; k++) rec[i * L::LEN + k] = r[k];
+}
+
 }  // namespace
 }  // namespace tct

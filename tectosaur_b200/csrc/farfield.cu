@@ -226,24 +226,6 @@ far_main_rh2(Consts<float> c, Rule2D<float> rule, const float* __restrict__ pts,
 }
 
 // ---- elasticU3/T3/A3/H3/RT3/RA3, 3-, 4- and 7-point rules (far_vec.cuh) ---------
-template <typename R, int K, int NQ>
-__global__ void __launch_bounds__(128)
-far_prep_vec(Consts<R> c, Rule2D<R> rule, const R* __restrict__ pts,
-             const int32_t* __restrict__ src_tris, int64_t n_src, const R* __restrict__ in,
-             R* __restrict__ rec) {
-    using L = RecVec<K, NQ>;
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n_src) return;
-    TriGeom<R> s;
-    load_tri(s, pts, src_tris, i, 0, false, K == kRT);
-    R in9[9], r[L::LEN];
-#pragma unroll
-    for (int k = 0; k < 9; k++) in9[k] = in[i * 9 + k];
-    vec_record<R, K, NQ>(c, rule, s, in9, r);
-#pragma unroll
-    for (int k = 0; k < L::LEN; k++) rec[i * L::LEN + k] = r[k];
-}
-
 // Sources per staged tile, and shared memory: the tile and, in FP32 with more
 // than four points a lane, the running sums and their compensation (as many
 // registers are not left).
@@ -489,7 +471,7 @@ int run_far_vec(const Consts<typename V::real>& c, const Rule2D<typename V::real
     R* rec = reinterpret_cast<R*>(ws);
     const size_t rec_bytes = align256(sizeof(R) * Rec<K, NQ>::LEN * (size_t)n_src);
     far_prep_vec<R, K, NQ><<<(unsigned)((n_src + 127) / 128), 128, 0, st>>>(c, rule, pts, src_tris,
-                                                                          n_src, in, rec);
+                                                                          n_src, in, nullptr, rec);
     int rc = launch_status("farfield prep");
     if (rc) return rc;
     const int64_t grain = V::H == 2 ? VEC_GRAIN : CHUNK_GRAIN;
@@ -1051,7 +1033,7 @@ int run_t2p_vec(const double* qp, const double* qw, const double* params, void* 
     int rc;
     if (n_src > 0) {
         far_prep_vec<R, K, NQ><<<(unsigned)((n_src + 127) / 128), 128, 0, st>>>(
-            c, rule, (const R*)pts, tris, n_src, (const R*)in, rec);
+            c, rule, (const R*)pts, tris, n_src, (const R*)in, nullptr, rec);
         if ((rc = launch_status("tct_farfield_tris_to_pts prep"))) return rc;
     }
     const int64_t chunks = t2p_chunks(1, sizeof(R) == 4 ? TCT_F32 : TCT_F64, n_obs, n_src, NQ);

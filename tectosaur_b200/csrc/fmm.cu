@@ -1476,7 +1476,7 @@ extern "C" int tct_fmm_matvec_planned(int kernel, int prec, int mode, int order,
                       (plan->n_tasks == 0 || (plan->tasks && plan->entries && plan->chunks)) &&
                       (plan->n_slots == 0 || plan->slots_in),
                   "tct_fmm_matvec_planned: bad plan");
-    TCT_CHECK_ARG(plan->chunk == (prec == TCT_F32 && p2p_is_rh(kernel, n_q) ? 64 : 32),
+    TCT_CHECK_ARG(plan->chunk == (prec == TCT_F32 && n_q != 13 ? 64 : 32),
                   "tct_fmm_matvec_planned: plan chunk %d", plan->chunk);
     TCT_CHECK_ARG(!plan->sym || p2p_is_rh(kernel, n_q),
                   "tct_fmm_matvec_planned: symmetric plan for kernel %d", kernel);

@@ -2,7 +2,7 @@
 //
 // The plan (fmm/p2p_plan.py) cuts the interaction list into tasks of one
 // chunk of an observation leaf (at most 64 triangles for the packed FP32
-// elasticRH3 kernel, 32 otherwise) against about a thousand source triangles
+// kernels, 32 otherwise) against about a thousand source triangles
 // of its list entries, so that blocks do about the same work whatever the
 // leaves' sizes; fmm_p2p (fmm.cu) gives a leaf's whole list to one block.
 // A block's four warps share the chunk and take a quarter of every staged
@@ -19,8 +19,10 @@
 // 32.8 ms with a block per leaf (packed, one-sided), 11.2 ms here; FP64 4-point
 // rule, 72,200 triangles, 7.3e8 pairs: 127 ms (one triangle a lane, records
 // through L1), 18.0 ms.  The whole applies: 37.4 -> 13.6 and 145.7 -> 23.3 ms.
+#include <type_traits>
+
 #include "fmm_p2p.h"
-#include "rh_sym.cuh"
+#include "far_vec.cuh"
 
 namespace tct {
 namespace {
@@ -212,8 +214,111 @@ p2p_rh(P2PArgs a, PairWeights<V, NQ> pw, Rule2D<typename V::real> rule,
     }
 }
 
-// Any other kernel or rule: the direct farfield's one-sided pair loop
-// (far_pair), one observation triangle a lane.
+// elasticU3, elasticRT3, elasticRA3 with the 3-, 4- and 7-point rules: the
+// direct farfield's vec forms (far_vec.cuh), one-sided.
+template <class V, int K, int NQ>
+__global__ void __launch_bounds__(128)
+p2p_vec(P2PArgs a, Consts<typename V::real> c, Rule2D<typename V::real> rule,
+        const typename V::real* __restrict__ opts, const int32_t* __restrict__ otris,
+        const typename V::real* __restrict__ rec, typename V::real* __restrict__ Wp) {
+    using R = typename V::real;
+    using vec = typename V::vec;
+    using L = RecVec<K, NQ>;
+    constexpr int NV = AccVec<K, NQ>::n, NA = NAcc<K, NQ>::n, CH = 32 * V::H;
+    __shared__ P2PTable tab;
+    __shared__ int srcs[P2P_TILE];
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    vec* sm = reinterpret_cast<vec*>(smem_raw);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int64_t o0 = a.tasks[4 * (int64_t)blockIdx.x];
+    const int cnt = a.tasks[4 * (int64_t)blockIdx.x + 1];
+    const int e0 = a.tasks[4 * (int64_t)blockIdx.x + 2];
+    const int ne = a.tasks[4 * (int64_t)blockIdx.x + 3] - e0;
+    load_table(tab, a.entries, e0, ne);
+    const int ns = tab.pos[ne];
+    const bool halves = cnt <= CH / 2;
+    const int li = halves ? lane & 15 : lane, step = halves ? 16 : 32;
+    const bool va = li < cnt, vb = V::H == 2 && li + step < cnt;
+    vec negx[NQ][3], no[3], tot[NV];
+    {
+        TriGeom<R> oa, ob;
+        load_tri(oa, opts, otris, o0 + (va ? li : 0), 0, false, false);
+        load_tri(ob, opts, otris, o0 + (vb ? li + step : 0), 0, false, false);
+#pragma unroll
+        for (int q = 0; q < NQ; q++) {
+            const R ox = rule.x[q], oy = rule.y[q];
+            const R bq[3] = {1 - ox - oy, ox, oy};
+#pragma unroll
+            for (int d = 0; d < 3; d++)
+                negx[q][d] = V::make(-bary_point(oa, bq, d), -bary_point(ob, bq, d));
+        }
+#pragma unroll
+        for (int d = 0; d < 3; d++) no[d] = V::make(oa.n[d], ob.n[d]);
+    }
+#pragma unroll
+    for (int k = 0; k < NV; k++) tot[k] = V::make(0, 0);
+    for (int t0 = 0; t0 < ns; t0 += P2P_TILE) {
+        const int nt = min(P2P_TILE, ns - t0);
+        __syncthreads();
+        if (tid < nt) {
+            const int e = find_entry(tab, ne, t0 + tid);
+            srcs[tid] = tab.src[e] + (t0 + tid - tab.pos[e]);
+        }
+        __syncthreads();
+        for (int k = tid; k < nt * L::LEN; k += 128) {
+            const int j = k / L::LEN;
+            const R v = __ldg(rec + (int64_t)srcs[j] * L::LEN + (k - j * L::LEN));
+            sm[k] = V::make(v, v);
+        }
+        __syncthreads();
+        vec acc[NV];
+#pragma unroll
+        for (int k = 0; k < NV; k++) acc[k] = V::make(0, 0);
+        const int j1 = min(nt, 16 * warp + 16), by = halves ? 2 : 1;
+#pragma unroll 1
+        for (int j = 16 * warp + (halves ? lane >> 4 : 0); j < j1; j += by)
+            vec_pair<V, K, NQ, NQ>(c, rule, sm + j * L::LEN, negx, no, acc);
+#pragma unroll
+        for (int k = 0; k < NV; k++) tot[k] = V::add(tot[k], acc[k]);
+    }
+    // the warps' (half-warps') sums in a fixed order
+    R* red = reinterpret_cast<R*>(smem_raw);  // 4 x CH x NA
+    __syncthreads();
+    const int base = warp * CH + (halves ? (lane >> 4) * (CH / 2) : 0) + li;
+#pragma unroll
+    for (int h = 0; h < V::H; h++) {
+        R s[NV], w[NA], nrm[3];
+#pragma unroll
+        for (int k = 0; k < NV; k++) {
+            R o[V::H];
+            V::split(tot[k], o);
+            s[k] = o[h];
+        }
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            R o[V::H];
+            V::split(no[d], o);
+            nrm[d] = o[h];
+        }
+        vec_totals<R, K, NQ>(s, nrm, w);
+#pragma unroll
+        for (int k = 0; k < NA; k++) red[(base + h * step) * NA + k] = w[k];
+    }
+    __syncthreads();
+    R* wo = Wp + (int64_t)blockIdx.x * CH * NA;
+    for (int e = tid; e < cnt * NA; e += 128) {
+        R s = 0;
+#pragma unroll
+        for (int w = 0; w < 4; w++) {
+            s += red[w * CH * NA + e];
+            if (halves) s += red[(w * CH + CH / 2) * NA + e];
+        }
+        wo[e] = s;
+    }
+}
+
+// The 13-point rule: the direct farfield's one-sided pair loop (far_pair), one
+// observation triangle a lane.
 template <typename R, int K, int NQ>
 __global__ void __launch_bounds__(128)
 p2p_any(P2PArgs a, Consts<R> c, Rule2D<R> rule, const R* __restrict__ opts,
@@ -377,26 +482,51 @@ int run_any(const P2PCall& k, const tct_fmm_p2p_plan& plan, cudaStream_t st) {
     return launch_status("p2p reduce");
 }
 
+template <class V, int K, int NQ>
+int run_vec(const P2PCall& k, const tct_fmm_p2p_plan& plan, cudaStream_t st) {
+    using R = typename V::real;
+    using L = RecVec<K, NQ>;
+    constexpr int NA = NAcc<K, NQ>::n;
+    const Consts<R> c = make_consts<R>(k.params);
+    Rule2D<R> rule;
+    for (int q = 0; q < MAXQ; q++) {
+        rule.x[q] = q < NQ ? (R)k.qp[2 * q] : R(0);
+        rule.y[q] = q < NQ ? (R)k.qp[2 * q + 1] : R(0);
+        rule.w[q] = q < NQ ? (R)k.qw[q] : R(0);
+    }
+    R* rec = reinterpret_cast<R*>(k.ws);
+    R* Wp = reinterpret_cast<R*>(k.ws + al256(sizeof(R) * (size_t)L::LEN * k.n_src));
+    far_prep_vec<R, K, NQ><<<(unsigned)((k.n_src + 127) / 128), 128, 0, st>>>(
+        c, rule, (const R*)k.src_pts, k.src_tris, k.n_src, (const R*)k.in, k.src_orig, rec);
+    int rc = launch_status("p2p prep");
+    if (rc) return rc;
+    const P2PArgs a{plan.tasks, plan.entries};
+    const size_t smem = std::max((size_t)8 * L::LEN * P2P_TILE, sizeof(R) * 4 * 32 * V::H * NA);
+    if ((rc = smem_limit(p2p_vec<V, K, NQ>, smem))) return rc;
+    p2p_vec<V, K, NQ><<<(unsigned)plan.n_tasks, 128, smem, st>>>(
+        a, c, rule, (const R*)k.obs_pts, k.obs_tris, rec, Wp);
+    if ((rc = launch_status("p2p (vec)"))) return rc;
+    p2p_reduce<R><<<(unsigned)plan.n_chunks, 256, 0, st>>>(plan.chunks, plan.slots_in, NA, plan.chunk,
+                                                          Wp, nullptr, (R*)k.W);
+    return launch_status("p2p reduce");
+}
+
 template <typename R>
 int any_dispatch(int kernel, int nq, const P2PCall& k, const tct_fmm_p2p_plan& plan,
                  cudaStream_t st) {
-#define TCT_P2P_NQ(KID, NQV) \
-    if (nq == NQV) return run_any<R, KID, NQV>(k, plan, st);
-#define TCT_P2P_K(KID)      \
-    if (kernel == KID) {    \
-        TCT_P2P_NQ(KID, 3)  \
-        TCT_P2P_NQ(KID, 4)  \
-        TCT_P2P_NQ(KID, 7)  \
-        TCT_P2P_NQ(KID, 13) \
+    using V = std::conditional_t<sizeof(R) == 4, VecF32, VecF64>;
+#define TCT_P2P_K(KID)                                       \
+    if (kernel == KID) {                                     \
+        if (nq == 3) return run_vec<V, KID, 3>(k, plan, st); \
+        if (nq == 4) return run_vec<V, KID, 4>(k, plan, st); \
+        if (nq == 7) return run_vec<V, KID, 7>(k, plan, st); \
+        return run_any<R, KID, 13>(k, plan, st);             \
     }
     TCT_P2P_K(kU)
     TCT_P2P_K(kRT)
     TCT_P2P_K(kRA)
-    if (kernel == kRH) {
-        TCT_P2P_NQ(kRH, 13)
-    }
 #undef TCT_P2P_K
-#undef TCT_P2P_NQ
+    if (kernel == kRH && nq == 13) return run_any<R, kRH, 13>(k, plan, st);
     set_error("p2p: unsupported kernel %d / n_q %d", kernel, nq);
     return TCT_ERR_ARG;
 }
@@ -423,7 +553,9 @@ size_t p2p_workspace_bytes(int kernel, int prec, int nq, int64_t n_src,
         return al256(8 * (size_t)self_rec_len(nq) * n_src) +
                al256(rs * 9 * ((size_t)plan.n_tasks * plan.chunk + (size_t)plan.n_slots));
     const size_t na = kernel == kRH ? 9 : (kernel == kRA ? 3 * nq + 3 : 3 * nq);
-    return al256(rs * na * (size_t)plan.n_tasks * plan.chunk);
+    // records of the vec forms: points, values, a normal, a curl
+    const size_t rec = nq == 13 ? 0 : al256(rs * (6 * nq + 6) * (size_t)n_src);
+    return rec + al256(rs * na * (size_t)plan.n_tasks * plan.chunk);
 }
 
 int p2p_planned(int kernel, int prec, int nq, const P2PCall& k, const tct_fmm_p2p_plan& plan,

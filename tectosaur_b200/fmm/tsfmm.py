@@ -138,7 +138,9 @@ class TSFMM:
         """Cut the near list into the P2P kernels' tasks (p2p_plan.py)."""
         rh = self.K.name == "elasticRH3" and self.nq in (3, 4, 7)
         f32 = self.prec == _lib.TCT_F32
-        plan = p2p_plan.build(self.obs_tree, self.src_tree, near, 64 if rh and f32 else 32, rh,
+        # the FP32 kernels take two triangles a lane (the 13-point rule's one)
+        chunk = 64 if f32 and self.nq != 13 else 32
+        plan = p2p_plan.build(self.obs_tree, self.src_tree, near, chunk, rh,
                               9 * self.float_type.itemsize, keep=self.touch)
         self.p2p_plan = plan
         self.p2p_desc = _lib.FmmList()  # the plan stands for the list
