@@ -231,29 +231,49 @@ far_self_reduce(const R* __restrict__ pts, const int32_t* __restrict__ tris, int
 
 inline size_t al256(size_t b) { return (b + 255) / 256 * 256; }
 
-// The fewest triangles served: below, the general kernel's chunks keep more
-// of the chip busy (FP32, 3-point rule: 722 triangles 0.029 ms general, 0.045
-// here, 1,500 0.047 against 0.045; FP64: 300 triangles 0.044 against 0.041).
-constexpr int64_t SELF_MIN_F32 = 1500, SELF_MIN_F64 = 256;
+// The fewest triangles served: below, the general kernel's chunks are as fast
+// (FP32, 3-point rule: 260 triangles 0.029 ms general, 0.038 here; 500 0.029 both,
+// 722 0.032 against 0.029; 4-point rule: 260 0.037 against 0.029; FP64: 260 0.044
+// against 0.029).
+int64_t self_min(int prec, int nq) { return prec == TCT_F32 && nq == 3 ? 600 : 256; }
 
 // Cut of n triangles: the largest groups and chunks (fewest partial sums) that
 // still give four CTAs for each of two per SM, so that the last wave is a
-// small part; the smallest cut where none does.
+// small part.  Where none does, groups of one strip and the chunk of least
+// cost, CTAs of the busiest SM x (sources + a fixed part of about 8 in FP32,
+// 2 in FP64): 1,000 triangles take 0.045, 0.031, 0.034 ms with chunks of 64,
+// 32, 16 sources (FP32, 3-point rule), 3,042 0.095, 0.086, 0.098.
 SelfCut self_cut(int prec, int64_t n) {
     const int64_t strip = prec == TCT_F32 ? 256 : 128;
-    static const int kStrips[] = {4, 2, 1, 1, 1};
-    static const int kDiv[] = {1, 1, 1, 2, 4};  // chunk = group / div
-    SelfCut c{0, 0, 0, 0, 0};
-    for (int k = 0; k < 5; k++) {
-        c.strips = kStrips[k];
-        const int64_t group = c.strips * strip;
-        c.per_group = kDiv[k];
-        c.chunk = (int)(group / kDiv[k]);
+    auto make = [&](int strips, int div) {
+        SelfCut c;
+        c.strips = strips;
+        const int64_t group = strips * strip;
+        c.per_group = div;
+        c.chunk = (int)(group / div);
         c.groups = (n + group - 1) / group;
         c.chunks = (n + c.chunk - 1) / c.chunk;
-        if (self_tasks_before(c.groups, c.chunks, c.per_group) >= 148 * 2 * 4) return c;
+        return c;
+    };
+    auto tasks = [](const SelfCut& c) {
+        return self_tasks_before(c.groups, c.chunks, c.per_group);
+    };
+    static const int kStrips[] = {4, 2, 1, 1, 1}, kDiv[] = {1, 1, 1, 2, 4};
+    for (int k = 0; k < 5; k++) {
+        const SelfCut c = make(kStrips[k], kDiv[k]);
+        if (tasks(c) >= 148 * 2 * 4) return c;
     }
-    return c;
+    SelfCut best = make(1, 4);
+    int64_t least = 0;
+    for (int div = 4; div <= 16; div *= 2) {
+        const SelfCut c = make(1, div);
+        const int64_t cost = (tasks(c) + 147) / 148 * (c.chunk + (prec == TCT_F32 ? 8 : 2));
+        if (least == 0 || cost < least) {
+            least = cost;
+            best = c;
+        }
+    }
+    return best;
 }
 
 // Bytes of the partials may not exceed this (n = 119,000 in FP32).
@@ -303,7 +323,7 @@ int run_self(const double* params, const double* qp, const double* qw, void* out
 extern "C" size_t tct_farfield_self_workspace_bytes(int kernel, int prec, int64_t n, int n_q) {
     using namespace tct;
     if (kernel != kRH || (prec != TCT_F32 && prec != TCT_F64) || self_rec_len(n_q) == 0 ||
-        n < (prec == TCT_F32 ? SELF_MIN_F32 : SELF_MIN_F64) || n >= (int64_t(1) << 31))
+        n < self_min(prec, n_q) || n >= (int64_t(1) << 31))
         return 0;
     const SelfCut c = self_cut(prec, n);
     const size_t part = self_partials(prec, n, c);

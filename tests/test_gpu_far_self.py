@@ -17,10 +17,11 @@ pytestmark = pytest.mark.gpu
 # double totals: sqrt(128) roundings of the partial sums, times 2 sides
 TOL = {np.float32: 4 * np.sqrt(128) * 6e-8, np.float64: 4 * np.sqrt(128) * 1.2e-16}
 
-# the cuts of self_cut: chunks of 64 (32), 128 (64), 256 (128), groups of 512
-# (256) and 1,024 (512) triangles in FP32 (FP64)
-CASES = [(np.float32, 1, n) for n in (1500, 1537, 2303, 9001, 12545, 24833, 49409)]
-CASES += [(np.float32, 2, 1501), (np.float32, 2, 9217), (np.float32, 3, 2049)]
+# the cuts of self_cut: chunks of 16 (8), 32 (16), 64 (32), 128 (64), 256 (128),
+# groups of 512 (256) and 1,024 (512) triangles in FP32 (FP64)
+CASES = [(np.float32, 1, n) for n in (600, 723, 1001, 1537, 2303, 9001, 12545, 24833, 49409)]
+CASES += [(np.float32, 2, 256), (np.float32, 2, 1501), (np.float32, 2, 9217),
+          (np.float32, 3, 257), (np.float32, 3, 2049)]
 CASES += [(np.float64, 1, n) for n in (256, 257, 700, 1153, 4481, 6401, 12417)]
 CASES += [(np.float64, 2, 511), (np.float64, 2, 4609), (np.float64, 3, 385)]
 
