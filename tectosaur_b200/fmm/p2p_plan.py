@@ -6,9 +6,9 @@ size; a chunk's list entries, in list order, are cut into tasks where the
 sources passed reach a multiple of about a thousand (or 128 entries).  On a
 symmetric list (one tree on both sides, leaves only: the FMM's) an unordered
 leaf pair keeps one entry: the kernel adds both directions, the sources' side
-into the entry's slots, one per source triangle.  Which leaf takes the lanes
-alternates with the parity of the two node indices, so that all leaves keep
-about half of their entries.
+into the entry's slots, one per source triangle.  The leaf that fills its lanes
+better takes them (a chunk of at most half the lanes' triangles doubles them);
+among equals the choice alternates with the parity of the two node indices.
 
 Row shards (`keep`): the tasks are cut on the whole list; a kept node's tasks
 stay whole, of the others the entries whose source is kept stay, so a kept
@@ -63,7 +63,12 @@ def build(obs_tree, src_tree, lst, chunk, want_sym, slot_bytes, keep=None, dev="
             bool((fwd[1:] != fwd[:-1]).all())
     nch = (osize + chunk - 1) // chunk
     if sym:
-        side = t.where((own + src) % 2 == 0, own <= src, own >= src)
+        # lanes a leaf of m triangles occupies, in triangles, and which fills
+        # them better: m_own / lanes_own against m_src / lanes_src
+        lanes = t.where(osize <= chunk // 2, t.full_like(osize, chunk // 2), nch * chunk)
+        a, b = osize[own] * lanes[src], osize[src] * lanes[own]
+        even = t.where((own + src) % 2 == 0, own <= src, own >= src)
+        side = (a > b) | ((a == b) & even)
         slots = int((ssize[src] * nch[own])[side & (own != src)].sum())
         if slots > MAX_SLOTS or slots * slot_bytes > MAX_SLOT_BYTES:
             sym = False
