@@ -153,16 +153,22 @@ class RegularizedNearfieldIntegralOp:
         self.classes = nearfield_pairs(pts, tris, obs_subset, src_subset, near_threshold,
                                        row_range=row_range)
 
-        rows = np.concatenate([self.classes[c][1][:, 0] for c in CLASSES]).astype(np.int64)
-        cols = np.concatenate([self.classes[c][1][:, 1] for c in CLASSES]).astype(np.int64)
-        order = np.lexsort((cols, rows))  # stable: duplicates keep class order
-        slot = np.empty_like(order)
-        slot[order] = np.arange(order.shape[0])
-        n_row_blocks = n_rows
-        indptr = np.zeros(n_row_blocks + 1, dtype=np.int64)
-        np.add.at(indptr, rows + 1, 1)
-        indptr = np.cumsum(indptr)
-        self.bsr = DeviceBSR9(self.shape, indptr, cols[order], float_type, row_align="auto")
+        # block order by (row, column), stable: duplicates keep class order;
+        # sorted on the device (one 64-bit key a block)
+        t = device.torch()
+        rows = np.concatenate([self.classes[c][1][:, 0] for c in CLASSES])
+        cols = np.concatenate([self.classes[c][1][:, 1] for c in CLASSES])
+        cols_dev = device.to_dev(cols, np.int64)
+        key = device.to_dev(rows, np.int64) * max(src_subset.shape[0], 1) + cols_dev
+        _, order = t.sort(key, stable=True)
+        slot_dev = t.empty_like(order)
+        slot_dev[order] = t.arange(order.shape[0], device="cuda")
+        slot = slot_dev.cpu().numpy()
+        indptr = np.zeros(n_rows + 1, dtype=np.int64)
+        np.cumsum(np.bincount(rows, minlength=n_rows), out=indptr[1:])
+        self.bsr = DeviceBSR9(self.shape, indptr, cols_dev[order].cpu().numpy(), float_type,
+                              row_align="auto")
+        del cols_dev, key, order, slot_dev
         self.class_slots = {}  # CSR positions of each class's blocks
         start = 0
         for c in CLASSES:
@@ -231,11 +237,8 @@ class RegularizedNearfieldIntegralOp:
             if n == 0:
                 continue
             (qp, qw), adj, check0 = host_rules[c]
-            base = np.zeros((n, 5), dtype=np.int64)
-            base[:, :2] = recs[:, :2]
-            r5 = recs[:, :5] if adj else base
-            groups.append((r5, (qp, qw, adj, check0)))
-            corr_groups.append((base, (far_q[0], far_q[1], False, c == "co")))
+            groups.append((recs[:, :5] if adj else recs[:, :2], (qp, qw, adj, check0)))
+            corr_groups.append((recs[:, :2], (far_q[0], far_q[1], False, c == "co")))
             slots.append(self.bsr.slots(self.class_slots[c]))
         if not groups:
             return

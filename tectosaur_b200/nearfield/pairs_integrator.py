@@ -143,44 +143,50 @@ class PairsIntegrator:
 
     def class_plan(self, classes, small=768):
         """Work plan for groups of pairs that share a rule (the nearfield
-        operator's classes), no pair split: classes = [(records (n, 5), rule
-        (pts, wts, adjacent, check0))].  Pairs of rules above `small` points
+        operator's classes), no pair split: classes = [(records (n, 5) or, without
+        rotations, (n, 2), rule (pts, wts, adjacent, check0))].  Pairs of rules above `small` points
         are warp items (the 32 lanes stride over the rule), the others thread
         items; both queues run the larger rules first and keep each class
         contiguous, so no sort of the (possibly 10^8) pairs is needed.
         Deterministic: every block is summed in a fixed order by one warp or
         one thread.  Pair p of the plan is the p-th record in class order."""
-        groups = [(np.asarray(r).reshape(-1, 5), q) for r, q in classes]
+        # records and items are laid out on the device: the host only narrows
+        # the pairs to int32
+        t = device.torch()
+        groups = [(np.asarray(r), q) for r, q in classes]
+        groups = [(r if r.ndim == 2 and r.shape[1] in (2, 5) else r.reshape(-1, 5), q)
+                  for r, q in groups]
         rules = [q for _, q in groups]
         sizes = np.array([q[0].shape[0] for q in rules], dtype=np.int64)
         rule_off = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
         rule_flags = np.array([(1 if q[2] else 0) | (2 if q[3] else 0) for q in rules], np.int32)
         pts_all = np.concatenate([np.asarray(q[0], np.float64).reshape(-1, 4) for q in rules])
         wts_all = np.concatenate([np.asarray(q[1], np.float64).reshape(-1) for q in rules])
-        n = int(sum(r.shape[0] for r, _ in groups))
-        rec7 = np.empty((n, 7), dtype=np.int32)
-        starts = np.concatenate([[0], np.cumsum([r.shape[0] for r, _ in groups])]).astype(np.int64)
+        counts = np.array([r.shape[0] for r, _ in groups], dtype=np.int64)
+        starts = np.concatenate([[0], np.cumsum(counts)]).astype(np.int64)
+        n = int(starts[-1])
+        rec7 = t.zeros((n, 7), dtype=t.int32, device="cuda")
         for g, (r, _) in enumerate(groups):
-            rec7[starts[g]:starts[g + 1], :5] = r
-            rec7[starts[g]:starts[g + 1], 5] = g
-        rec7[:, 6] = 0
-        witems, titems = [], []
+            rows = rec7[starts[g]:starts[g + 1]]
+            if rows.shape[0]:
+                rows[:, :r.shape[1]] = device.to_dev(r, np.int32)
+            rows[:, 5] = g
+        items = t.zeros((max(n, 1), 4), dtype=t.int32, device="cuda")
+        pos = n_warp = 0
         for g in np.argsort(-sizes, kind="stable"):
-            k = np.arange(starts[g], starts[g + 1], dtype=np.int64)
-            it = np.stack([k, np.zeros_like(k), np.full_like(k, sizes[g]), np.zeros_like(k)],
-                          axis=1)
-            (witems if sizes[g] > small else titems).append(it)
-        witems = np.concatenate(witems) if witems else np.zeros((0, 4), np.int64)
-        titems = np.concatenate(titems) if titems else np.zeros((0, 4), np.int64)
-        items = np.ascontiguousarray(np.concatenate([witems, titems]).astype(np.int32))
+            it = items[pos:pos + counts[g]]
+            it[:, 0] = t.arange(int(starts[g]), int(starts[g + 1]), dtype=t.int32, device="cuda")
+            it[:, 2] = int(sizes[g])
+            pos += int(counts[g])
+            if sizes[g] > small:
+                n_warp = pos
         ft = self.float_type
-        return dict(n=n, n_warp=witems.shape[0], n_thread=titems.shape[0],
-                    param_sets=self.params.reshape(1, 2), n_points=int(sizes[rec7[:, 5]].sum()),
+        return dict(n=n, n_warp=n_warp, n_thread=n - n_warp,
+                    param_sets=self.params.reshape(1, 2), n_points=int((sizes * counts).sum()),
                     ws=device.workspace(2048),
-                    dev=[device.to_dev(rec7), device.to_dev(rule_off),
+                    dev=[rec7, device.to_dev(rule_off),
                          device.to_dev(rule_flags), device.to_dev(pts_all, ft),
-                         device.to_dev(wts_all, ft),
-                         device.to_dev(items if items.size else np.zeros((1, 4), np.int32))])
+                         device.to_dev(wts_all, ft), items])
 
     def batched_run_slots(self, plan, out, slot_dev, slot_stride, sign=1.0, add=False,
                           stream=None):
