@@ -730,6 +730,15 @@ int tct_csr_matvec_panel(int prec, int64_t n_rows, const int64_t* indptr, const 
                          const double* data, const void* x, int64_t x_stride, void* y,
                          int64_t y_stride, int n_vec, int accumulate, void* stream);
 
+/* One Arnoldi step on the device: w is orthogonalised against the basis V_0 ..
+ * V_(rows-1) (rows of n doubles) by classical Gram-Schmidt applied twice,
+ * col[0 .. rows-1] receives the coefficients, col[rows] the norm of what is
+ * left, and V_rows that vector over its norm (untouched when the norm is not
+ * positive); w is not changed.  For the sizes of tct_arnoldi_step_fits (1 =
+ * fits: bound by launches rather than bytes). */
+int tct_arnoldi_step_fits(int64_t n, int rows);
+int tct_arnoldi_step(double* V, int64_t n, int rows, const double* w, double* col, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -202,6 +202,8 @@ EXPORTED = sorted(set(EXPORTED) | set(_FMM_SIGS))
 
 _SOLVE_SIGS = {
     "tct_csr_matvec": ([c_i, c_i64, c_p, c_p, c_p, c_p, c_p, c_i, c_p], c_i),
+    "tct_arnoldi_step_fits": ([c_i64, c_i], c_i),
+    "tct_arnoldi_step": ([c_p, c_i64, c_i, c_p, c_p, c_p], c_i),
     "tct_csr_matvec_panel": ([c_i, c_i64, c_p, c_p, c_p, c_p, c_i64, c_p, c_i64, c_i, c_i, c_p],
                              c_i),
     "tct_fp64_fma_probe": ([c_p, c_i64, c_i, c_p], c_i),

@@ -43,6 +43,8 @@ def gmres(A, b, tol=1e-8, restart=200, maxiter=None, x0=None, M=None, callback=N
     maxiter = 10 * n if maxiter is None else maxiter
     m = max(1, min(restart, n))
     V = t.empty((m + 1, n), dtype=b.dtype, device=b.device)
+    on_gpu = V.is_cuda and V.dtype == t.float64
+    col_dev = t.empty(m + 1, dtype=b.dtype, device=b.device) if on_gpu else None
     total = 0
     first = x0 is None
     while True:
@@ -61,17 +63,26 @@ def gmres(A, b, tol=1e-8, restart=200, maxiter=None, x0=None, M=None, callback=N
         j_end = m
         for j in range(m):
             w = A(V[j] if M is None else M(V[j]))
-            Vj = V[: j + 1]
-            h = Vj @ w
-            w = w - h @ Vj
-            h2 = Vj @ w
-            w = w - h2 @ Vj
-            h = h + h2
-            hn = t.linalg.norm(w)
-            col = t.cat([h, hn.reshape(1)]).cpu().numpy()  # the one sync of a step
-            H[: j + 2, j] = col
-            if col[-1] > 0.0:
-                V[j + 1] = w / hn
+            if on_gpu and _lib.lib.tct_arnoldi_step_fits(n, j + 1):
+                # launch-bound sizes: the whole orthogonalisation in one launch
+                w = w.contiguous()
+                _lib.check(_lib.lib.tct_arnoldi_step(
+                    _lib.tptr(V), n, j + 1, _lib.tptr(w), _lib.tptr(col_dev),
+                    _lib.stream_ptr()), "tct_arnoldi_step")
+                col = col_dev[: j + 2].cpu().numpy()  # the one sync of a step
+                H[: j + 2, j] = col
+            else:
+                Vj = V[: j + 1]
+                h = Vj @ w
+                w = w - h @ Vj
+                h2 = Vj @ w
+                w = w - h2 @ Vj
+                h = h + h2
+                hn = t.linalg.norm(w)
+                col = t.cat([h, hn.reshape(1)]).cpu().numpy()  # the one sync of a step
+                H[: j + 2, j] = col
+                if col[-1] > 0.0:
+                    V[j + 1] = w / hn
             for i in range(j):
                 a, c = H[i, j], H[i + 1, j]
                 H[i, j] = cs[i] * a + sn[i] * c
@@ -178,11 +189,13 @@ class ConstrainedOperator:
     def __call__(self, v):
         t = device.torch()
         self.n_matvecs += 1
-        if self.cm is not None:
+        if self.cm is None:
+            self.x_full.copy_(v)
+        elif self.ft == t.float64:
+            self.cm.dot_device(v, self.x_full)
+        else:
             self.cm.dot_device(v, self._tmp)
             self.x_full.copy_(self._tmp)
-        else:
-            self.x_full.copy_(v)
         self.iop.dot_device(self.x_full, self.y_full)
         yd = self.y_full.to(t.float64)
         if self.cmT is None:

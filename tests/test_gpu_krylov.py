@@ -1,0 +1,58 @@
+"""The one-launch Arnoldi step (csrc/krylov.cu) against the same steps as
+matrix-vector products: slices of one unknown and less, rows at the warp count
+and above, the largest it takes, a vector already in the span's zero."""
+import pytest
+
+from tectosaur_b200 import _lib
+
+pytestmark = pytest.mark.gpu
+
+
+def _step(t, V, j, w):
+    col = t.empty(j + 2, dtype=t.float64, device="cuda")
+    _lib.check(_lib.lib.tct_arnoldi_step(_lib.tptr(V), V.shape[1], j + 1, _lib.tptr(w),
+                                         _lib.tptr(col), _lib.stream_ptr()), "tct_arnoldi_step")
+    return col
+
+
+@pytest.mark.parametrize("n,rows", [(1, 1), (7, 2), (8, 8), (9, 3), (65, 16), (2907, 17), (2907, 60),
+                                    (4097, 33), (32768, 45), (1400, 1024)])
+def test_arnoldi_step(cuda, n, rows):
+    t = cuda
+    g = t.Generator(device="cuda").manual_seed(n + rows)
+    V = t.zeros((rows + 1, n), dtype=t.float64, device="cuda")
+    k = min(rows, n)
+    q, _ = t.linalg.qr(t.randn((n, k), generator=g, dtype=t.float64, device="cuda"))
+    V[:k] = q.T
+    w = t.randn(n, generator=g, dtype=t.float64, device="cuda")
+    w0 = w.clone()
+    V0 = V.clone()
+    col = _step(t, V, rows - 1, w)
+    Vj = V0[:rows]
+    h = Vj @ w
+    r = w - h @ Vj
+    h2 = Vj @ r
+    r = r - h2 @ Vj
+    assert t.equal(w, w0) and t.equal(V[:rows], V0[:rows])
+    # sums of n products of unit vectors' entries and w: n^(1/2) roundings
+    tol = 8 * 1.2e-16 * n ** 0.5 * float(w.norm())
+    assert float((col[:rows] - (h + h2)).abs().max()) <= tol
+    assert abs(float(col[rows]) - float(r.norm())) <= tol
+    if k < n:
+        assert float((V[rows] * col[rows] - r).norm()) <= tol * rows ** 0.5
+        assert float((Vj @ V[rows]).abs().max()) < 1e-13
+    again = V.clone()
+    assert t.equal(_step(t, V, rows - 1, w), col) and t.equal(V, again)
+
+
+def test_arnoldi_step_zero_and_sizes(cuda):
+    t = cuda
+    V = t.full((3, 100), 0.1, dtype=t.float64, device="cuda")
+    V[2] = 7.0
+    col = _step(t, V, 1, t.zeros(100, dtype=t.float64, device="cuda"))
+    assert float(col.abs().max()) == 0.0 and bool((V[2] == 7.0).all())
+    fits = _lib.lib.tct_arnoldi_step_fits
+    assert fits(32768, 45) and not fits(32769, 1) and not fits(10, 1025) and not fits(30000, 51)
+    assert not fits(0, 1) and not fits(10, 0)
+    assert _lib.lib.tct_arnoldi_step(_lib.tptr(V), 40000, 1, _lib.tptr(V), _lib.tptr(col),
+                                     _lib.stream_ptr()) == _lib.TCT_ERR_ARG
