@@ -40,10 +40,13 @@ K_NAME = "elasticRH3"
 # kernel (FMA = 2): D 3, r^2 5, rsqrt 1, weights 4, S0 1, g*D 3, T 12 = 29,
 # plus the per-triangle-pair W update 63 flops / 9 point pairs = 7.
 FLOPS_PER_POINT_PAIR_RH = 36.0
-# DRAM bytes of one far_main_rh2 launch on the 59,858-triangle surface (ncu
+# The self farfield forms a pair's geometry once for both directions: 29 / 2 of
+# it per ordered point pair, the update in full.
+FLOPS_PER_POINT_PAIR_RH_SELF = 21.5
+# DRAM bytes of one far_self_main launch on the 59,858-triangle surface (ncu
 # dram__bytes_read.sum + dram__bytes_write.sum, one full-size capture): the
-# kernel reads its source records through L2 and is compute-bound
-FAR_TRAFFIC_BYTES = 14.856e6
+# partial sums of both directions; the kernel is compute-bound
+FAR_TRAFFIC_BYTES = None
 # DRAM bytes of one bsr9_kernel launch on the same surface's nearfield matrix
 # (5,477,848 blocks, rows aligned to 32 slots; one full-size capture):
 # 1.05x the algorithmic 1.801e9 bytes
@@ -332,8 +335,8 @@ FMM_CFG = dict(mac=3.0, pts_per_cell=128, order=8, mode="fmm")
 
 def fmm_algorithmic_flops(fmm, n_q):
     """FP32 flops of one FMM apply counted from the interaction lists: P2P
-    point pairs x 36 (the hoisted elasticRH3 pair loop) + M2L pairs x
-    C(p+6, 6) (a, b) products x 21 channels x 2."""
+    point pairs x 21.5 (both directions of a pair from one geometry) + M2L
+    pairs x the harmonic (a, b) products of |a| + |b| <= p x 12 channels x 2."""
     st, ot = fmm.src_tree, fmm.obs_tree
     l = fmm.p2p
     n_o = (ot.end - ot.start)[l.obs_n_idxs]
@@ -342,9 +345,9 @@ def fmm_algorithmic_flops(fmm, n_q):
     src_per_obs = np.add.reduceat(n_s, l.obs_src_starts[:-1]) if lens.size else np.zeros(0)
     p2p_pairs = float(np.sum(n_o * src_per_obs)) * n_q * n_q
     p = fmm.order
-    ab = (p + 1) * (p + 2) * (p + 3) * (p + 4) * (p + 5) * (p + 6) / 720.0
-    m2l = float(fmm.m2l.src_n_idxs.shape[0]) * ab * 21 * 2
-    return p2p_pairs * FLOPS_PER_POINT_PAIR_RH + m2l, p2p_pairs, m2l
+    ab = sum((2 * k + 1) * (p + 1 - k) ** 2 for k in range(p + 1))
+    m2l = float(fmm.m2l.src_n_idxs.shape[0]) * ab * 12 * 2
+    return p2p_pairs * FLOPS_PER_POINT_PAIR_RH_SELF + m2l, p2p_pairs, m2l
 
 
 def cpu_direct_far_baseline(pts, tris, target_s=10.0, K=None):
@@ -446,6 +449,7 @@ def run_fmm_workload(args, rank, world, torch, dist):
     peak_ffma, peak_ffma2 = fp32_peak_tflops(torch, _lib.lib)
     peak = max(peak_ffma, peak_ffma2)
     achieved = flops / (ms * 1e-3) / 1e12
+    # two preps, P2P and its reduction, P2M, M2L, L2P, finish; M2M and L2L per level
     n_launch = 8 + op.fmm.src_desc.n_levels + op.fmm.obs_desc.n_levels
     line = {
         "metric": "BEM farfield matvecs/s (FMM)", "value": world * args.steps / (total_ms * 1e-3),
@@ -469,7 +473,7 @@ def run_fmm_workload(args, rank, world, torch, dist):
                      "frac": achieved / peak, "traffic": None,
                      "peak_source": "measured live: best FP32 FMA probe (scalar %.1f, packed "
                                     "%.1f TFLOP/s)" % (peak_ffma, peak_ffma2),
-                     "algorithmic": "%.3e flops per apply: %.3e P2P point pairs x 36 + M2L "
+                     "algorithmic": "%.3e flops per apply: %.3e P2P point pairs x 21.5 + M2L "
                                     "%.3e" % (flops, p2p_pairs, m2l_flops)},
         "e2e": {"value": world * args.steps / t_e2e, "unit": "matvecs/s",
                 "h2d_bytes_per_step": int(xh.nbytes), "d2h_bytes_per_step": int(yh.nbytes),
@@ -2272,14 +2276,12 @@ def main():
     if rank == 0:
         peak_ffma, peak_ffma2 = fp32_peak_tflops(torch, _lib.lib)
         peak = max(peak_ffma, peak_ffma2)
-        flops = float(n) * n * 9 * FLOPS_PER_POINT_PAIR_RH
+        flops = float(n) * n * 9 * FLOPS_PER_POINT_PAIR_RH_SELF
         achieved = flops / (far_ms * 1e-3) / 1e12
         near_ms = ms_per_step - far_ms
         near_bytes = nnzb * (81 * 4 + 4) + (n + 1) * 4 + 2 * 9 * n * 4
         mp = measured_peaks()
         hbm = mp.get("hbm_gbs") if mp else 6650.0
-        obs_blocks = (n + 127) // 128
-        chunks = max(1, min(-(-1184 // obs_blocks), max(1, n // 128), 32))
         line = {
             "metric": "BEM matvecs/s", "value": value, "unit": "matvecs/s", "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms_per_step,
@@ -2287,17 +2289,17 @@ def main():
             "data": "synthetic (seeded mesh and inputs)",
             "config": config_block(n, nnzb),
             "roofline": {
-                "kernel": "far_main_rh2<3, uniform> (packed f32x2 elasticRH3 tri-to-tri "
-                          "farfield)",
+                "kernel": "far_self_main<3, uniform> (packed f32x2 elasticRH3 tri-to-tri "
+                          "farfield of a set on itself)",
                 "bound": "fp32", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                 "frac": achieved / peak, "traffic": FAR_TRAFFIC_BYTES,
                 "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one "
-                                  "full-size launch (profiles/far_main_rh2_c2_full.md)",
+                                  "full-size launch (profiles/far_self_main.md)",
                 "peak_source": "measured live: best of the FP32 FMA probes (scalar FFMA "
                                "%.1f, packed fma.rn.f32x2 %.1f TFLOP/s); MEASURED_PEAKS.json "
                                "has no FP32 figure" % (peak_ffma, peak_ffma2),
                 "algorithmic": "%.3e flops per apply = %d^2 tri pairs x 9 point pairs x %g"
-                               % (flops, n, FLOPS_PER_POINT_PAIR_RH),
+                               % (flops, n, FLOPS_PER_POINT_PAIR_RH_SELF),
                 "far_ms": far_ms,
             },
             "nearfield": {"ms": near_ms, "bytes": near_bytes,
@@ -2315,7 +2317,8 @@ def main():
                                             "of one full-size launch "
                                             "(profiles/bsr9_fp32_c2.md)"},
             "e2e": e2e,
-            "gpu_launches": args.steps * (2 + (1 if chunks > 1 else 0) + (1 if nnzb else 0)),
+            # prep, main, reduce; the nearfield
+            "gpu_launches": args.steps * (3 + (1 if nnzb else 0)),
             "clocks": clocks,
             "setup_s": t_build,
             "autotune": dict(shapes, seconds=t_tune),

@@ -587,9 +587,10 @@ def _op_bytes(op):
     n = near.bsr.nbytes
     if getattr(near, "correction", None) is not None:
         n += near.correction.numel() * near.correction.element_size()
-    ws = getattr(op.farfield, "workspace", None)
-    if ws is not None:
-        n += ws.numel() * ws.element_size()
+    for name in ("workspace", "self_workspace"):
+        ws = getattr(op.farfield, name, None)
+        if ws is not None:
+            n += ws.numel() * ws.element_size()
     return int(n)
 
 
