@@ -43,9 +43,8 @@ FLOPS_PER_POINT_PAIR_RH = 36.0
 # The self farfield forms a pair's geometry once for both directions: 29 / 2 of
 # it per ordered point pair, the update in full.
 FLOPS_PER_POINT_PAIR_RH_SELF = 21.5
-# DRAM bytes of one far_self_main launch on the 59,858-triangle surface (ncu
-# dram__bytes_read.sum + dram__bytes_write.sum, one full-size capture): the
-# partial sums of both directions; the kernel is compute-bound
+# DRAM bytes of one far_self_main launch: not captured at full size (the partial
+# sums of both directions, 0.25 GB a launch; the kernel is compute-bound)
 FAR_TRAFFIC_BYTES = None
 # DRAM bytes of one bsr9_kernel launch on the same surface's nearfield matrix
 # (5,477,848 blocks, rows aligned to 32 slots; one full-size capture):
@@ -2293,8 +2292,8 @@ def main():
                           "farfield of a set on itself)",
                 "bound": "fp32", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
                 "frac": achieved / peak, "traffic": FAR_TRAFFIC_BYTES,
-                "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one "
-                                  "full-size launch (profiles/far_self_main.md)",
+                "traffic_source": "not captured (pipes and stalls of a 20,001-triangle launch: "
+                                  "profiles/far_self_main.md)",
                 "peak_source": "measured live: best of the FP32 FMA probes (scalar FFMA "
                                "%.1f, packed fma.rn.f32x2 %.1f TFLOP/s); MEASURED_PEAKS.json "
                                "has no FP32 figure" % (peak_ffma, peak_ffma2),
